@@ -19,6 +19,11 @@ struct sqd_paulis_s {
   sqd::DevBuf<uint64_t> term_z;       // [M]
   sqd::DevBuf<double> term_c;         // [2M] interleaved (re, im)
   sqd::DevBuf<int32_t> term_group;    // [M]
+  // The same table packed for the kernels that compose elements: one 8-byte load gives a
+  // group's terms, one 16-byte load a term's mask and real coefficient.
+  sqd::DevBuf<uint2> group_span;      // [J] (first term, group_eff)
+  sqd::DevBuf<ulonglong2> term_rec;   // [M] (z, bits of Re c)
+  uint64_t version = 0;               // bumped by sqd_paulis_set_coeffs
   sqd::DevBuf<int32_t> raw_to_term;   // [num_raw]
   // term -> raw terms merged into it, in input order (for coefficient updates)
   int64_t num_kept = 0;
@@ -99,6 +104,27 @@ struct ProductLayout {
   sqd::DevBuf<uint32_t> slist;       // [soff[nh]] ascending source slabs
 };
 
+// Connectivity of a product subspace by half strings (connect.cu): rows r = h * nl + l.  Four
+// lists of (key, partner) entries, each string's entries in ascending mask order:
+//   H: X masks on the high half only,  key = group, partner h' (H[h'] = H[h] ^ x);
+//   L: X masks on the low half only,   key = group, partner l';
+//   A: distinct high parts of the two-half masks, key = index a, partner h';
+//   B: distinct low parts of the two-half masks,  key = index b, partner l'.
+// A two-half group connects (h, l) for every (a in A(h), b in B(l)) whose group exists.  The
+// lists take a few hundred entries per string, so an operator without cached sources keeps
+// them too.
+struct ProductPlan {
+  int64_t nh = 0, nl = 0;
+  int d = 0;                          // the diagonal group exists
+  int64_t th = 0, tl = 0, ta = 0, tb = 0;   // entries per list
+  sqd::DevBuf<int64_t> offs;          // [2 nh + 2 nl + 1]: H, L, A, B offsets into key / part
+  sqd::DevBuf<uint32_t> key, part;
+  int64_t na = 0, nb = 0, nm = 0;
+  sqd::DevBuf<int32_t> mtable;        // [na * nb] group of (a, b) or -1 (dense form)
+  sqd::DevBuf<uint64_t> xa, xb, xm;   // distinct parts; two-half masks, ascending (sparse form)
+  sqd::DevBuf<int32_t> gm;            // [nm] groups of xm
+};
+
 // Solver objects an operator keeps between LOCG solves (locg.cu): work vectors and the
 // instantiated CUDA graphs of the iteration, rebuilt when the matvec schedule changes.
 struct LocgCacheBase {
@@ -123,6 +149,8 @@ struct sqd_op_s {
   int64_t n_gpre = 0;
   int64_t n_gpre_cls[3] = {0, 0, 0};  // gpre entries per class (H, L, M), in that order
   int product_built = 0;          // connectivity assembled from the two halves' lists
+  std::unique_ptr<ProductPlan> plan;  // product subspaces: the halves' lists
+  uint64_t values_version = 0;    // p->version that the cached elements were computed from
   sqd::DevBuf<int> status;        // device status word
   int layout[2] = {0, 0};         // SQD_LAYOUT_* per precision
   ProductLayout prod;
@@ -133,6 +161,86 @@ struct sqd_op_s {
 };
 
 namespace sqd {
+
+// The packed Pauli table as the kernels read it.
+struct TermTable {
+  const uint2* span;
+  const ulonglong2* rec;
+  const double* c;
+};
+inline TermTable term_table(const sqd_paulis_s* p) {
+  return TermTable{p->group_span.ptr, p->term_rec.ptr, p->term_c.ptr};
+}
+
+// Composed diagonal of a group (its span) at state s, term by term in the reference's order
+// (get_diagonal, sqd.py:603-628): sums of c or -c by the parity of s & z.
+template <int NCA>
+__device__ __forceinline__ Cx<double> compose(const TermTable& T, uint2 sp, uint64_t s) {
+  double dr = 0.0, di = 0.0;
+#pragma unroll 4
+  for (uint32_t t = sp.x; t < sp.x + sp.y; ++t) {
+    const ulonglong2 r = __ldg(T.rec + t);
+    const uint64_t v = s & r.x;
+    const uint64_t flip =
+        static_cast<uint64_t>(__popc(static_cast<unsigned>(v) ^ static_cast<unsigned>(v >> 32)))
+        << 63;
+    dr += __longlong_as_double(static_cast<long long>(r.y ^ flip));
+    if constexpr (NCA == 2)
+      di += __longlong_as_double(__double_as_longlong(__ldg(T.c + 2 * int64_t(t) + 1)) ^
+                                 static_cast<long long>(flip));
+  }
+  return cx_make<double>(dr, di);
+}
+
+// Device view of a ProductPlan.
+struct PlanView {
+  int64_t nh, nl;
+  int d;
+  const int64_t *hoff, *loff, *aoff, *boff;   // [nh + 1], [nl + 1], [nh + 1], [nl + 1]
+  const uint32_t *key, *part;
+  const int32_t* table;
+  int64_t nb;
+  const uint64_t *xa, *xb, *xm;
+  const int32_t* gm;
+  int64_t nm;
+};
+inline PlanView plan_view(const ProductPlan& q) {
+  PlanView v{};
+  v.nh = q.nh;
+  v.nl = q.nl;
+  v.d = q.d;
+  v.hoff = q.offs.ptr;
+  v.loff = v.hoff + q.nh;
+  v.aoff = v.loff + q.nl;
+  v.boff = v.aoff + q.nh;
+  v.key = q.key.ptr;
+  v.part = q.part.ptr;
+  v.table = q.mtable.ptr;
+  v.nb = q.nb;
+  v.xa = q.xa.ptr;
+  v.xb = q.xb.ptr;
+  v.xm = q.xm.ptr;
+  v.gm = q.gm.ptr;
+  v.nm = q.nm;
+  return v;
+}
+
+__device__ __forceinline__ int64_t sorted_find(const uint64_t* __restrict__ a, int64_t n,
+                                               uint64_t key) {
+  int64_t lo = 0, hi = n;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (__ldg(a + mid) < key) lo = mid + 1; else hi = mid;
+  }
+  return (lo < n && __ldg(a + lo) == key) ? lo : -1;
+}
+
+// Group of the two-half mask with parts a and b, or -1.
+__device__ __forceinline__ int32_t plan_group(const PlanView& c, uint32_t a, uint32_t b) {
+  if (c.table) return __ldg(c.table + int64_t(a) * c.nb + b);
+  const int64_t i = sorted_find(c.xm, c.nm, __ldg(c.xa + a) | __ldg(c.xb + b));
+  return i >= 0 ? __ldg(c.gm + i) : -1;
+}
 
 // Lookup of key in the space: index or -1.
 __device__ __forceinline__ int64_t hash_lookup(const uint64_t* __restrict__ keys,
@@ -163,18 +271,36 @@ __device__ __forceinline__ uint32_t sector_bitmap_index(uint64_t proj, int shift
   return static_cast<uint32_t>(v & ((1ull << kBitmapLog2) - 1));
 }
 
-// Build helpers implemented in matvec.cu / connect.cu.
+// Build helpers implemented in operator.cu and matvec.cu.
 void op_build(sqd_op_s* op, cudaStream_t st);
 void op_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st);
 void op_ensure_values32(sqd_op_s* op, cudaStream_t st);
 // Product layout (product.cu).
 bool op_product_detect(sqd_op_s* op, cudaStream_t st, int64_t* nh, int64_t* nl);
 void op_product_build(sqd_op_s* op, cudaStream_t st);
-void op_product_values(sqd_op_s* op, cudaStream_t st);
+void op_product_refresh(sqd_op_s* op, cudaStream_t st);
 void op_product_values32(sqd_op_s* op, cudaStream_t st);
 void op_product_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st);
-// Connectivity (row_ptr, cols, grps, nnz) of a product subspace from per-half partner lists;
-// false when the subspace is not such a product.
+// Product subspaces (connect.cu): builds op->plan unless it exists (false when the subspace is
+// not such a product), and the connectivity (row_ptr, cols, grps, nnz) from it.
+bool op_plan(sqd_op_s* op, cudaStream_t st);
 bool op_connect_product(sqd_op_s* op, cudaStream_t st);
+// Where the elements of the stored pairs go (elements.cu): the pair list (values: NCA doubles per
+// pair, or complex128 with out_complex) and, for the H and L pairs of a product subspace, the
+// slabs and their FP32 copies (NULL = not wanted).
+struct ElementOut {
+  double* values;
+  int out_complex;
+  double *vh, *vl;
+  float *vh32, *vl32;
+  int wide32;
+};
+void op_pair_elements(sqd_op_s* op, const ElementOut& out, cudaStream_t st);
+// Slabs from the elements in the pair list (op->plan exists).
+void op_slab_elements(sqd_op_s* op, const ElementOut& out, cudaStream_t st);
+// The slab buffers of op->prod that a refresh has to fill.
+void op_product_targets(sqd_op_s* op, ElementOut* out);
+// Copies the packed Pauli table from the current coefficients (paulis.cu).
+void paulis_pack(sqd_paulis_s* p, cudaStream_t st);
 
 }  // namespace sqd

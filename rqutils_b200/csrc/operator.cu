@@ -5,8 +5,7 @@
 // (run_sqd, sqd.py:343-351): instead of a dense J x N int32 array with -1 for missing sources,
 // only the pairs whose source exists are stored, row by row, in group order:
 //   row_ptr[states_size + 1], cols[nnz] (source index), grps[nnz] (group index).
-// Matrix elements (z = 2) are the composed diagonals C^(j)_i of the stored pairs
-// (sqd.py:95-98), summed term by term in the reference's order (get_diagonal, sqd.py:603-628).
+// Matrix elements (z = 2): elements.cu.  Product subspaces' connectivity: connect.cu.
 #include "internal.cuh"
 #include "dispatch.cuh"
 #include "sweep.cuh"
@@ -101,34 +100,6 @@ __device__ __forceinline__ Cx<double> diag_seq(const int64_t* gs, const int32_t*
   return cx_make<double>(dr, di);
 }
 
-// One warp per row, lanes over the row's stored pairs: matrix element per pair.
-// out_mode 0: values as NCA doubles per pair; 1: complex128 per pair (CSR export).
-template <int NCA>
-__global__ void k_values(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ grps,
-                         const uint64_t* __restrict__ states, int64_t n_unique,
-                         uint64_t fill_state, int64_t size, const int64_t* gs, const int32_t* ge,
-                         const uint64_t* tz, const double* tc, double* out, int out_complex) {
-  const int lane = threadIdx.x & 31;
-  const int64_t w0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t r = w0; r < size; r += nw) {
-    const uint64_t s = r < n_unique ? __ldg(states + r) : fill_state;
-    const int64_t b = row_ptr[r], e = row_ptr[r + 1];
-    for (int64_t i = b + lane; i < e; i += 32) {
-      const Cx<double> d = diag_seq<NCA>(gs, ge, tz, tc, grps[i], s);
-      if (out_complex) {
-        out[2 * i] = d.re;
-        out[2 * i + 1] = d.im;
-      } else if constexpr (NCA == 2) {
-        out[2 * i] = d.re;
-        out[2 * i + 1] = d.im;
-      } else {
-        out[i] = d.re;
-      }
-    }
-  }
-}
-
 __global__ void k_to_float(const double* in, float* out, int64_t n) {
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x)
@@ -161,16 +132,21 @@ __device__ __forceinline__ unsigned long long order_key(double v) {
   return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
 
-// Argmin of Re diag_0 over real rows; ties -> smallest index (jnp.argmin).
-__global__ void k_argmin_partial(const uint64_t* states, int64_t n_unique, const int64_t* gs,
-                                 const int32_t* ge, const uint64_t* tz, const double* tc,
+// Argmin of Re diag_0 over real rows; ties -> smallest index (jnp.argmin).  CACHED: the diagonal is
+// read back from the cached elements (the first pair of every row, the same sums), 8 bytes a row
+// instead of the group's hundreds of terms (48 qubits, 1.15 M rows: 726 us when composed).
+template <bool CACHED>
+__global__ void k_argmin_partial(const uint64_t* states, int64_t n_unique, TermTable T,
+                                 const int64_t* row_ptr, const double* values, int stride,
                                  unsigned long long* best_key, long long* best_idx) {
   unsigned long long bk = ~0ull;
   long long bi = 0x7fffffffffffffffll;
+  const uint2 sp = __ldg(T.span);
   for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n_unique;
        r += int64_t(gridDim.x) * blockDim.x) {
-    const Cx<double> d = diag_seq<1>(gs, ge, tz, tc, 0, states[r]);
-    const unsigned long long k = order_key(d.re);
+    const double v = CACHED ? __ldg(values + stride * __ldg(row_ptr + r))
+                            : compose<1>(T, sp, states[r]).re;
+    const unsigned long long k = order_key(v);
     if (k < bk || (k == bk && r < bi)) {
       bk = k;
       bi = r;
@@ -456,16 +432,10 @@ void op_values_and_lanes(sqd_op_s* op, cudaStream_t st) {
   if (op->z_cache == 2) {
     const int nca = op->value_complex ? 2 : 1;
     op->values.alloc(static_cast<size_t>(op->nnz > 0 ? op->nnz : 1) * nca, st);
-    const unsigned G = grid_for(size * 32, 256, 16384);
-    if (nca == 2)
-      k_values<2><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->grps.ptr, sp->states.ptr, nu,
-                                     sp->fill_state, size, p->group_start.ptr, p->group_eff.ptr,
-                                     p->term_z.ptr, p->term_c.ptr, op->values.ptr, 0);
-    else
-      k_values<1><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->grps.ptr, sp->states.ptr, nu,
-                                     sp->fill_state, size, p->group_start.ptr, p->group_eff.ptr,
-                                     p->term_z.ptr, p->term_c.ptr, op->values.ptr, 0);
-    SQD_CHECK_LAUNCH();
+    ElementOut out{};
+    out.values = op->values.ptr;
+    op_pair_elements(op, out, st);
+    op->values_version = p->version;
   }
   // Lanes per row from the mean row length.
   const double avg = nu > 0 ? static_cast<double>(op->nnz) / static_cast<double>(nu) : 0.0;
@@ -589,9 +559,15 @@ extern "C" int sqd_vinit(sqd_op_t op, int64_t* index_host, void* stream) {
     keys.alloc(nw, st);
     idx.alloc(nw, st);
     res.alloc(1, st);
-    k_argmin_partial<<<G, 256, 0, st>>>(sp->states.ptr, sp->n_unique, p->group_start.ptr,
-                                        p->group_eff.ptr, p->term_z.ptr, p->term_c.ptr,
-                                        keys.ptr, idx.ptr);
+    // Elements older than the coefficients (set_coeffs without a refresh) do not count.
+    const bool cached = op->z_cache == 2 && op->values.ptr && op->values_version == p->version;
+    if (cached)
+      k_argmin_partial<true><<<G, 256, 0, st>>>(sp->states.ptr, sp->n_unique, term_table(p),
+                                                op->row_ptr.ptr, op->values.ptr,
+                                                op->value_complex ? 2 : 1, keys.ptr, idx.ptr);
+    else
+      k_argmin_partial<false><<<G, 256, 0, st>>>(sp->states.ptr, sp->n_unique, term_table(p),
+                                                 nullptr, nullptr, 0, keys.ptr, idx.ptr);
     SQD_CHECK_LAUNCH();
     k_argmin_final<<<1, 1024, 0, st>>>(keys.ptr, idx.ptr, nw, res.ptr);
     SQD_CHECK_LAUNCH();
@@ -608,10 +584,8 @@ extern "C" int sqd_op_csr(sqd_op_t op, int64_t* indptr, int32_t* indices, double
     SQD_REQUIRE(op->x_cache == 1, "CSR export needs cache_strategy x = 1");
     SQD_REQUIRE(op->nnz == 0 || op->grps.ptr != nullptr,
                 "the operator released its group indices; create a new operator");
-    sqd_paulis_s* p = op->p;
-    sqd_space_s* sp = op->s;
     cudaStream_t st = as_stream(stream);
-    const int64_t size = sp->states_size;
+    const int64_t size = op->s->states_size;
     if (indptr)
       SQD_CUDA(cudaMemcpyAsync(indptr, op->row_ptr.ptr, (size + 1) * sizeof(int64_t),
                                cudaMemcpyDeviceToDevice, st));
@@ -621,16 +595,10 @@ extern "C" int sqd_op_csr(sqd_op_t op, int64_t* indptr, int32_t* indices, double
       SQD_CHECK_LAUNCH();
     }
     if (data && op->nnz > 0) {
-      const unsigned G = grid_for(size * 32, 256, 16384);
-      if (p->is_complex)
-        k_values<2><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->grps.ptr, sp->states.ptr,
-                                       sp->n_unique, sp->fill_state, size, p->group_start.ptr,
-                                       p->group_eff.ptr, p->term_z.ptr, p->term_c.ptr, data, 1);
-      else
-        k_values<1><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->grps.ptr, sp->states.ptr,
-                                       sp->n_unique, sp->fill_state, size, p->group_start.ptr,
-                                       p->group_eff.ptr, p->term_z.ptr, p->term_c.ptr, data, 1);
-      SQD_CHECK_LAUNCH();
+      ElementOut out{};
+      out.values = data;
+      out.out_complex = 1;
+      op_pair_elements(op, out, st);
     }
   });
 }
@@ -667,30 +635,21 @@ extern "C" int sqd_op_refresh(sqd_op_t op, void* stream) {
     SQD_REQUIRE(op->z_cache != 2 || op->nnz == 0 || op->grps.ptr != nullptr,
                 "the operator released its group indices; create a new operator");
     sqd_paulis_s* p = op->p;
-    sqd_space_s* sp = op->s;
     SQD_REQUIRE(p->is_complex == op->value_complex,
                 "the Pauli sum changed between real and complex; create a new operator");
     if (op->z_cache != 2 || op->nnz == 0) return;
     cudaStream_t st = as_stream(stream);
-    const int64_t size = sp->states_size;
-    const unsigned G = grid_for(size * 32, 256, 16384);
-    if (op->value_complex)
-      k_values<2><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->grps.ptr, sp->states.ptr,
-                                     sp->n_unique, sp->fill_state, size, p->group_start.ptr,
-                                     p->group_eff.ptr, p->term_z.ptr, p->term_c.ptr,
-                                     op->values.ptr, 0);
-    else
-      k_values<1><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->grps.ptr, sp->states.ptr,
-                                     sp->n_unique, sp->fill_state, size, p->group_start.ptr,
-                                     p->group_eff.ptr, p->term_z.ptr, p->term_c.ptr,
-                                     op->values.ptr, 0);
-    SQD_CHECK_LAUNCH();
+    ElementOut out{};
+    out.values = op->values.ptr;
+    op_product_targets(op, &out);
+    op_pair_elements(op, out, st);
+    op->values_version = p->version;
     if (op->values32.ptr) {
       const size_t n = static_cast<size_t>(op->nnz) * (op->value_complex ? 2 : 1);
       k_to_float<<<grid_for(n, 256, 16384), 256, 0, st>>>(op->values.ptr, op->values32.ptr, n);
       SQD_CHECK_LAUNCH();
     }
-    op_product_values(op, st);
+    op_product_refresh(op, st);
     ++op->schedule_version;
   });
 }

@@ -2,7 +2,7 @@
 //
 // SQD subspaces are usually the Cartesian product of strings on the high half of the qubits
 // (beta) and strings on the low half (alpha).  Sorted, row r = h * nl + l holds H[h] | L[l].
-// The stored pairs of a row come in three classes (k_gpre_flags, operator.cu):
+// The stored pairs of a row come in three classes (k_gpre_flags, operator.cu; lists of the halves' partners: connect.cu):
 //   H: x on the high half only, source (h', l) with H[h'] = H[h] ^ x.  Every row of slab h has
 //      the same H sources in the same order;
 //   L: the diagonal group and x on the low half only, source (h, l') with L[l'] = L[l] ^ x.
@@ -36,9 +36,6 @@
 // FP32 vectors keep the compensated accumulation in every part and pass partials in FP64, so
 // the result is rounded once.  The elements are the same numbers as in the CSR arrays; only
 // the summation order of a row changes (L and M pairs before H pairs).
-//
-// The file also builds the connectivity itself for such subspaces (op_connect_product): the
-// partners of every string of each half, then each row's pairs assembled from them.
 #include <cstdlib>
 #include <algorithm>
 #include <climits>
@@ -52,173 +49,29 @@
 namespace sqd {
 namespace {
 
-__device__ __forceinline__ void warp_count_add(unsigned long long c, unsigned long long* dst) {
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFullMask, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(dst, c);
-}
-
-// Number of distinct high strings (rows whose high half differs from the previous row's).
-__global__ void k_count_slabs(const uint64_t* __restrict__ s, int64_t n, uint64_t mhi,
-                              unsigned long long* cnt) {
-  unsigned long long c = 0;
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
-       r += int64_t(gridDim.x) * blockDim.x)
-    if (r == 0 || ((s[r] ^ s[r - 1]) & mhi) != 0) ++c;
-  warp_count_add(c, cnt);
-}
-
-// Rows that are not H[r / nl] | L[r % nl].
-__global__ void k_check_product(const uint64_t* __restrict__ s, int64_t n, int64_t nl,
-                                uint64_t mlo, uint64_t mhi, unsigned long long* bad) {
-  unsigned long long c = 0;
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
-       r += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t l = r % nl;
-    const uint64_t v = s[r];
-    if (((v ^ s[l]) & mlo) != 0 || ((v ^ s[r - l]) & mhi) != 0) ++c;
+// Source offsets of the slabs from the halves' partner lists: hsrc[k] = h' * nl over the H lists,
+// lsrc[e] = l' * nh over the L lists, each low string's diagonal entry (d) first; lo with those
+// diagonal entries counted.
+__global__ void k_slab_sources(PlanView c, int64_t th, uint32_t* hsrc, int64_t* lo,
+                               uint32_t* lsrc) {
+  const int64_t t0 = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  const int64_t step = int64_t(gridDim.x) * blockDim.x;
+  for (int64_t k = t0; k < th; k += step) hsrc[k] = static_cast<uint32_t>(c.part[k] * c.nl);
+  const int64_t l0 = c.loff[0];
+  for (int64_t l = t0; l <= c.nl; l += step) {
+    int64_t e = c.loff[l] - l0 + c.d * l;
+    lo[l] = e;
+    if (l == c.nl) continue;
+    if (c.d) lsrc[e++] = static_cast<uint32_t>(l * c.nh);
+    for (int64_t i = c.loff[l]; i < c.loff[l + 1]; ++i)
+      lsrc[e++] = static_cast<uint32_t>(c.part[i] * c.nh);
   }
-  warp_count_add(c, bad);
-}
-
-// Per row: the H pairs that follow the diagonal entry and the L pairs after them; a pair of
-// another class before the M pairs end counts as an error.
-__global__ void k_row_kinds(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ grps,
-                            const uint64_t* __restrict__ group_x, int64_t n, int d, uint64_t mlo,
-                            uint64_t mhi, int32_t* rkh, int32_t* rkl, unsigned long long* bad) {
-  unsigned long long c = 0;
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
-       r += int64_t(gridDim.x) * blockDim.x) {
-    int64_t i = row_ptr[r];
-    const int64_t e = row_ptr[r + 1];
-    bool ok = true;
-    if (d) {
-      ok = i < e && grps[i] == 0;
-      ++i;
-    }
-    const int64_t b = i;
-    while (i < e && (__ldg(group_x + grps[i]) & mlo) == 0) ++i;
-    const int64_t b2 = i;
-    while (i < e && (__ldg(group_x + grps[i]) & mhi) == 0) ++i;
-    const int64_t b3 = i;
-    for (; i < e; ++i) {
-      const uint64_t x = __ldg(group_x + grps[i]);
-      if ((x & mlo) == 0 || (x & mhi) == 0) ok = false;
-    }
-    rkh[r] = static_cast<int32_t>(b2 - b);
-    rkl[r] = static_cast<int32_t>(b3 - b2);
-    if (!ok) ++c;
-  }
-  warp_count_add(c, bad);
-}
-
-// Entries per slab (from the slab's first row) and per low string (from slab 0, diagonal
-// included); every row must agree with both.
-__global__ void k_slab_meta(const int32_t* __restrict__ rkh, const int32_t* __restrict__ rkl,
-                            int64_t n, int64_t nl, int d, int64_t* kh, int64_t* kl,
-                            unsigned long long* bad) {
-  unsigned long long c = 0;
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
-       r += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t h = r / nl, l = r - h * nl;
-    if (l == 0) kh[h] = rkh[r];
-    if (h == 0) kl[l] = d + rkl[r];
-    if (rkh[r] != rkh[h * nl] || rkl[r] != rkl[l]) ++c;
-  }
-  warp_count_add(c, bad);
-}
-
-// H sources as offsets h' * nl: the sources of row (h, 0) itself.
-__global__ void k_hsrc(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ cols,
-                       int64_t nh, int64_t nl, int d, const int64_t* __restrict__ ho,
-                       uint32_t* hsrc) {
-  for (int64_t h = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; h < nh;
-       h += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t b = row_ptr[h * nl] + d;
-    for (int64_t k = 0; k < ho[h + 1] - ho[h]; ++k) hsrc[ho[h] + k] = cols[b + k];
-  }
-}
-
-// L sources as offsets l' * nh (into the transposed vector), from row (0, l).
-__global__ void k_lsrc(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ cols,
-                       int64_t nh, int64_t nl, int d, const int64_t* __restrict__ ho,
-                       const int64_t* __restrict__ lo, uint32_t* lsrc) {
-  const int64_t kh0 = ho[1] - ho[0];
-  for (int64_t l = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; l < nl;
-       l += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t b = row_ptr[l];
-    for (int64_t e = 0; e < lo[l + 1] - lo[l]; ++e) {
-      const int64_t lp = (d && e == 0) ? l : int64_t(cols[b + kh0 + e]);
-      lsrc[lo[l] + e] = static_cast<uint32_t>(lp * nh);
-    }
-  }
-}
-
-// Panel-major slab index of entry k at contiguous position b.
-__device__ __forceinline__ int64_t panel_index(int64_t k, int64_t b, int64_t total_k) {
-  return ((b >> 5) * total_k + k) * 32 + (b & 31);
-}
-
-// Copies every H and L element into its slab and checks that its stored source is the one the
-// slab position implies.
-template <int NCA>
-__global__ void k_prod_extract(const int64_t* __restrict__ row_ptr,
-                               const uint32_t* __restrict__ cols, const double* __restrict__ vals,
-                               int64_t n, int64_t nh, int64_t nl, int d,
-                               const int64_t* __restrict__ ho, const int64_t* __restrict__ lo,
-                               const uint32_t* __restrict__ hsrc,
-                               const uint32_t* __restrict__ lsrc, double* vh, double* vl,
-                               int check, unsigned long long* bad) {
-  const int64_t th = ho[nh], tl = lo[nl];
-  unsigned long long c = 0;
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
-       r += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t h = r / nl, l = r - h * nl;
-    const int64_t b = row_ptr[r];
-    const int64_t h0 = ho[h], nkh = ho[h + 1] - h0, l0 = lo[l], nkl = lo[l + 1] - l0;
-    if (check && row_ptr[r + 1] < b + nkh + nkl) {
-      ++c;
-      continue;
-    }
-    for (int64_t k = 0; k < nkh; ++k) {
-      const int64_t p = b + d + k;
-      if (check && int64_t(cols[p]) != int64_t(hsrc[h0 + k]) + l) ++c;
-      const int64_t q = panel_index(h0 + k, l, th);
-#pragma unroll
-      for (int t = 0; t < NCA; ++t) vh[NCA * q + t] = vals[NCA * p + t];
-    }
-    for (int64_t e = 0; e < nkl; ++e) {
-      const int64_t p = (d && e == 0) ? b : b + nkh + e;
-      if (check && int64_t(cols[p]) != h * nl + int64_t(lsrc[l0 + e]) / nh) ++c;
-      const int64_t q = panel_index(l0 + e, h, tl);
-#pragma unroll
-      for (int t = 0; t < NCA; ++t) vl[NCA * q + t] = vals[NCA * p + t];
-    }
-  }
-  warp_count_add(c, bad);
 }
 
 __global__ void k_to_float32(const double* __restrict__ in, float* __restrict__ out, int64_t n) {
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x)
     out[i] = static_cast<float>(in[i]);
-}
-
-// FP32 copy of a slab in 64-wide panels: out[((b / 64) * total_k + k) * 64 + b % 64] =
-// in[panel_index(k, b, total_k)] for b < B, zero in the padding of the last panel.
-template <int NCA>
-__global__ void k_float_panels64(const double* __restrict__ in, int64_t total_k, int64_t B,
-                                 float* __restrict__ out) {
-  const int64_t n = ((B + 63) / 64) * total_k * 64;
-  for (int64_t q = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; q < n;
-       q += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t rest = q >> 6, pos = q & 63;   // rest = panel * total_k + k
-    const int64_t p = rest / total_k, k = rest - p * total_k;
-    const int64_t b = p * 64 + pos;
-    const int64_t src = b < B ? panel_index(k, b, total_k) : 0;
-#pragma unroll
-    for (int t = 0; t < NCA; ++t)
-      out[NCA * q + t] = b < B ? static_cast<float>(in[NCA * src + t]) : 0.0f;
-  }
 }
 
 // out[c][r] = in[r][c] for an rows x cols matrix of elements E (32 x 32 tiles, 256 threads).
@@ -694,21 +547,6 @@ unsigned mixed_grid(int64_t rows, int lpr) {
   return static_cast<unsigned>(std::max<int64_t>(1, std::min(blocks, cap)));
 }
 
-void extract(sqd_op_s* op, cudaStream_t st, int check, unsigned long long* bad) {
-  ProductLayout& L = op->prod;
-  const int64_t n = L.nh * L.nl;
-  const unsigned G = grid_for(n, 256, 16384);
-  if (op->value_complex)
-    k_prod_extract<2><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->values.ptr, n, L.nh,
-                                         L.nl, op->has_diag_group, L.ho.ptr, L.lo.ptr,
-                                         L.hsrc.ptr, L.lsrc.ptr, L.vh.ptr, L.vl.ptr, check, bad);
-  else
-    k_prod_extract<1><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->values.ptr, n, L.nh,
-                                         L.nl, op->has_diag_group, L.ho.ptr, L.lo.ptr,
-                                         L.hsrc.ptr, L.lsrc.ptr, L.vh.ptr, L.vl.ptr, check, bad);
-  SQD_CHECK_LAUNCH();
-}
-
 void to_float(const DevBuf<double>& in, DevBuf<float>& out, cudaStream_t st) {
   out.alloc(in.count, st);
   k_to_float32<<<grid_for(static_cast<int64_t>(in.count), 256, 16384), 256, 0, st>>>(
@@ -716,27 +554,29 @@ void to_float(const DevBuf<double>& in, DevBuf<float>& out, cudaStream_t st) {
   SQD_CHECK_LAUNCH();
 }
 
-// FP32 copies of both slab sets: 64-wide panels when wide32, else the FP64 layout.
-void slabs_to_float(sqd_op_s* op, cudaStream_t st) {
+// Slabs (f64) and their FP32 copies (f32) from the elements in the pair list.
+void fill_slabs(sqd_op_s* op, bool f64, bool f32, cudaStream_t st) {
   ProductLayout& L = op->prod;
-  if (!L.wide32) {
-    to_float(L.vh, L.vh32, st);
-    to_float(L.vl, L.vl32, st);
-    return;
+  ElementOut out{};
+  out.values = op->values.ptr;
+  if (f64) {
+    out.vh = L.vh.ptr;
+    out.vl = L.vl.ptr;
   }
+  if (f32) {
+    out.vh32 = L.vh32.ptr;
+    out.vl32 = L.vl32.ptr;
+  }
+  out.wide32 = L.wide32;
+  op_slab_elements(op, out, st);
+}
+
+void alloc_slabs32(sqd_op_s* op, cudaStream_t st) {
+  ProductLayout& L = op->prod;
   const int nca = op->value_complex ? 2 : 1;
-  auto conv = [&](const DevBuf<double>& in, int64_t total_k, int64_t B, DevBuf<float>& out) {
-    const int64_t n = ((B + 63) / 64) * total_k * 64;
-    out.alloc(static_cast<size_t>(std::max<int64_t>(n, 1)) * nca, st);
-    const unsigned G = grid_for(std::max<int64_t>(n, 1), 256, 16384);
-    if (nca == 2)
-      k_float_panels64<2><<<G, 256, 0, st>>>(in.ptr, total_k, B, out.ptr);
-    else
-      k_float_panels64<1><<<G, 256, 0, st>>>(in.ptr, total_k, B, out.ptr);
-    SQD_CHECK_LAUNCH();
-  };
-  conv(L.vh, L.th, L.nl, L.vh32);
-  conv(L.vl, L.tl, L.nh, L.vl32);
+  const int64_t w = L.wide32 ? 64 : 32;
+  L.vh32.alloc(static_cast<size_t>(std::max<int64_t>((L.nl + w - 1) / w * L.th * w, 1)) * nca, st);
+  L.vl32.alloc(static_cast<size_t>(std::max<int64_t>((L.nh + w - 1) / w * L.tl * w, 1)) * nca, st);
 }
 
 // A row tail read in place is a short segment of the row's long pair list (C3-like subspaces:
@@ -886,285 +726,7 @@ bool launch_tail_smem(sqd_op_s* op, int prec, const R* vin, cudaStream_t st) {
   return true;
 }
 
-// ---- connectivity of a product subspace -------------------------------------------------
-// The (row, group) sweep tests every group against every row.  In a product subspace a group
-// acting on one half connects a row iff the row's string of that half has a partner, so the
-// partners are searched once per string of the half, and a two-half group connects (h, l) iff
-// both halves have partners.  The pairs are then assembled per row in the sweep's order:
-// diagonal, H groups, L groups, M groups, each class in ascending group index (= ascending x:
-// for M groups, ascending high part, then low part).
-
-__device__ __forceinline__ int64_t sorted_find(const uint64_t* __restrict__ a, int64_t n,
-                                               uint64_t key) {
-  int64_t lo = 0, hi = n;
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (__ldg(a + mid) < key) lo = mid + 1; else hi = mid;
-  }
-  return (lo < n && __ldg(a + lo) == key) ? lo : -1;
-}
-
-// Partners of every string s of one half under the masks xs[k]: entries (k, partner) with
-// strs[partner] == strs[s] ^ xs[k], in k order.  One warp per string, lanes over k, ballots
-// keep the order.  COUNT: count[s]; FILL: writes at off[s].
-template <bool FILL>
-__global__ void k_half_partners(const uint64_t* __restrict__ strs, int64_t nstr,
-                                const uint64_t* __restrict__ xs, int64_t nx,
-                                const int64_t* __restrict__ off, int64_t* count,
-                                uint32_t* out_k, uint32_t* out_p) {
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  const int64_t w0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t s = w0; s < nstr; s += nw) {
-    const uint64_t base = __ldg(strs + s);
-    int64_t pos = FILL ? off[s] : 0;
-    for (int64_t k0 = 0; k0 < nx; k0 += 32) {
-      const int64_t k = k0 + lane;
-      int64_t found = -1;
-      if (k < nx) found = sorted_find(strs, nstr, base ^ __ldg(xs + k));
-      const unsigned b = __ballot_sync(kFullMask, found >= 0);
-      if (FILL && found >= 0) {
-        const int64_t idx = pos + __popc(b & lt);
-        out_k[idx] = static_cast<uint32_t>(k);
-        out_p[idx] = static_cast<uint32_t>(found);
-      }
-      pos += __popc(b);
-    }
-    if (!FILL && lane == 0) count[s] = pos;
-  }
-}
-
-struct ProdConnect {
-  int64_t nh, nl;
-  int d;
-  const int64_t *hoff, *loff, *aoff, *boff;          // H, L, M-high, M-low lists per string
-  const uint32_t *hk, *hp, *lk, *lp, *ak, *ap, *bk, *bp;
-  const int32_t *gh, *gl;                            // group index of H / L list entry k
-  const int32_t* table;                              // [na * nb] M group or -1 (dense form)
-  int64_t na, nb;
-  const uint64_t *xa, *xb, *xm;                      // sparse form: M masks, sorted
-  const int32_t* gm;
-  int64_t nm;
-};
-
-__device__ __forceinline__ int32_t m_group(const ProdConnect& c, uint32_t a, uint32_t b) {
-  if (c.table) return __ldg(c.table + int64_t(a) * c.nb + b);
-  const int64_t i = sorted_find(c.xm, c.nm, __ldg(c.xa + a) | __ldg(c.xb + b));
-  return i >= 0 ? __ldg(c.gm + i) : -1;
-}
-
-template <bool FILL>
-__global__ void k_prod_rows(ProdConnect c, int64_t* counts, const int64_t* __restrict__ row_ptr,
-                            uint32_t* cols, uint32_t* grps) {
-  const int64_t n = c.nh * c.nl;
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
-       r += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t h = r / c.nl, l = r - h * c.nl;
-    const int64_t h0 = c.hoff[h], h1 = c.hoff[h + 1], l0 = c.loff[l], l1 = c.loff[l + 1];
-    const int64_t a0 = c.aoff[h], a1 = c.aoff[h + 1], b0 = c.boff[l], b1 = c.boff[l + 1];
-    if (!FILL) {
-      int64_t m = 0;
-      for (int64_t i = a0; i < a1; ++i)
-        for (int64_t j = b0; j < b1; ++j) m += m_group(c, c.ak[i], c.bk[j]) >= 0;
-      counts[r] = c.d + (h1 - h0) + (l1 - l0) + m;
-      continue;
-    }
-    int64_t p = row_ptr[r];
-    if (c.d) {
-      cols[p] = static_cast<uint32_t>(r);
-      grps[p] = 0;
-      ++p;
-    }
-    for (int64_t i = h0; i < h1; ++i, ++p) {
-      cols[p] = static_cast<uint32_t>(int64_t(c.hp[i]) * c.nl + l);
-      grps[p] = static_cast<uint32_t>(c.gh[c.hk[i]]);
-    }
-    for (int64_t i = l0; i < l1; ++i, ++p) {
-      cols[p] = static_cast<uint32_t>(h * c.nl + c.lp[i]);
-      grps[p] = static_cast<uint32_t>(c.gl[c.lk[i]]);
-    }
-    for (int64_t i = a0; i < a1; ++i) {
-      const int64_t src_h = int64_t(c.ap[i]) * c.nl;
-      for (int64_t j = b0; j < b1; ++j) {
-        const int32_t g = m_group(c, c.ak[i], c.bk[j]);
-        if (g < 0) continue;
-        cols[p] = static_cast<uint32_t>(src_h + c.bp[j]);
-        grps[p] = static_cast<uint32_t>(g);
-        ++p;
-      }
-    }
-  }
-}
-
-__global__ void k_half_strings(const uint64_t* __restrict__ s, int64_t count, int64_t stride,
-                               uint64_t mask, uint64_t* out) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < count;
-       i += int64_t(gridDim.x) * blockDim.x)
-    out[i] = s[i * stride] & mask;
-}
-
-// Device copy of a host vector.
-template <typename T>
-void upload(DevBuf<T>& d, const std::vector<T>& h, cudaStream_t st) {
-  d.alloc(std::max<size_t>(h.size(), 1), st);
-  if (!h.empty())
-    SQD_CUDA(cudaMemcpyAsync(d.ptr, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-}
-
-// Partner lists of one half: counts, offsets, (k, partner) entries.
-struct HalfLists {
-  DevBuf<int64_t> off;
-  DevBuf<uint32_t> k, p;
-};
-
-void half_lists(const DevBuf<uint64_t>& strs, int64_t nstr, const DevBuf<uint64_t>& xs,
-                int64_t nx, HalfLists& out, cudaStream_t st) {
-  DevBuf<int64_t> cnt;
-  cnt.alloc(std::max<int64_t>(nstr, 1), st);
-  const unsigned G = grid_for(nstr * 32, 256, 8192);
-  k_half_partners<false><<<G, 256, 0, st>>>(strs.ptr, nstr, xs.ptr, nx, nullptr, cnt.ptr,
-                                             nullptr, nullptr);
-  SQD_CHECK_LAUNCH();
-  out.off.alloc(nstr + 1, st);
-  exclusive_scan_i64(cnt.ptr, out.off.ptr, nstr, true, st);
-  int64_t total = 0;
-  copy_to_host(&total, out.off.ptr + nstr, 1, st);
-  out.k.alloc(std::max<int64_t>(total, 1), st);
-  out.p.alloc(std::max<int64_t>(total, 1), st);
-  k_half_partners<true><<<G, 256, 0, st>>>(strs.ptr, nstr, xs.ptr, nx, out.off.ptr, nullptr,
-                                            out.k.ptr, out.p.ptr);
-  SQD_CHECK_LAUNCH();
-}
-
 }  // namespace
-
-bool op_product_detect(sqd_op_s* op, cudaStream_t st, int64_t* nh_out, int64_t* nl_out) {
-  sqd_space_s* sp = op->s;
-  const int64_t n = sp->n_unique;
-  *nh_out = *nl_out = 0;
-  if (n == 0 || sp->states_size != n || sp->num_qubits < 2) return false;
-  const uint64_t mlo = half_mask_low(sp->num_qubits), mhi = sp->fill_state & ~mlo;
-  DevBuf<unsigned long long> cnt;
-  cnt.alloc(2, st);
-  SQD_CUDA(cudaMemsetAsync(cnt.ptr, 0, 2 * sizeof(unsigned long long), st));
-  const unsigned G = grid_for(n, 256, 4096);
-  k_count_slabs<<<G, 256, 0, st>>>(sp->states.ptr, n, mhi, cnt.ptr);
-  SQD_CHECK_LAUNCH();
-  unsigned long long nh = 0;
-  copy_to_host(&nh, cnt.ptr, 1, st);
-  if (nh == 0 || n % static_cast<int64_t>(nh) != 0) return false;
-  const int64_t nl = n / static_cast<int64_t>(nh);
-  k_check_product<<<G, 256, 0, st>>>(sp->states.ptr, n, nl, mlo, mhi, cnt.ptr + 1);
-  SQD_CHECK_LAUNCH();
-  unsigned long long bad = 0;
-  copy_to_host(&bad, cnt.ptr + 1, 1, st);
-  if (bad) return false;
-  *nh_out = static_cast<int64_t>(nh);
-  *nl_out = nl;
-  return true;
-}
-
-bool op_connect_product(sqd_op_s* op, cudaStream_t st) {
-  int64_t nh = 0, nl = 0;
-  if (!op_product_detect(op, st, &nh, &nl)) return false;
-  sqd_space_s* sp = op->s;
-  const int64_t n = nh * nl;
-  if (n > (int64_t(1) << 32)) return false;
-  const uint64_t mlo = half_mask_low(sp->num_qubits), mhi = sp->fill_state & ~mlo;
-  // Group lists per class from the preprocessed groups (class order, ascending group index).
-  std::vector<GroupPre> gp(static_cast<size_t>(op->n_gpre));
-  copy_to_host(gp.data(), op->gpre.ptr, gp.size(), st);
-  const int64_t n0 = op->n_gpre_cls[0], n1 = op->n_gpre_cls[1];
-  std::vector<uint64_t> xh, xl, xm;
-  std::vector<int32_t> gh, gl, gm;
-  for (int64_t i = 0; i < op->n_gpre; ++i) {
-    const GroupPre& g = gp[static_cast<size_t>(i)];
-    if (i < n0) { xh.push_back(g.x); gh.push_back(g.group); }
-    else if (i < n0 + n1) { xl.push_back(g.x); gl.push_back(g.group); }
-    else { xm.push_back(g.x); gm.push_back(g.group); }
-  }
-  // Distinct high and low parts of the M masks (ascending), and the M group lookup.
-  std::vector<uint64_t> xa, xb;
-  for (uint64_t x : xm) { xa.push_back(x & mhi); xb.push_back(x & mlo); }
-  std::sort(xa.begin(), xa.end());
-  xa.erase(std::unique(xa.begin(), xa.end()), xa.end());
-  std::sort(xb.begin(), xb.end());
-  xb.erase(std::unique(xb.begin(), xb.end()), xb.end());
-  const bool dense = !xm.empty() && double(xa.size()) * double(xb.size()) <= double(1 << 24);
-  std::vector<int32_t> table;
-  if (dense) {
-    table.assign(xa.size() * xb.size(), -1);
-    for (size_t i = 0; i < xm.size(); ++i) {
-      const size_t a = std::lower_bound(xa.begin(), xa.end(), xm[i] & mhi) - xa.begin();
-      const size_t b = std::lower_bound(xb.begin(), xb.end(), xm[i] & mlo) - xb.begin();
-      table[a * xb.size() + b] = gm[i];
-    }
-  }
-  DevBuf<uint64_t> hstr, lstr, dxh, dxl, dxa, dxb, dxm;
-  DevBuf<int32_t> dgh, dgl, dgm, dtable;
-  hstr.alloc(nh, st);
-  lstr.alloc(nl, st);
-  k_half_strings<<<grid_for(nh, 256, 4096), 256, 0, st>>>(sp->states.ptr, nh, nl, mhi, hstr.ptr);
-  k_half_strings<<<grid_for(nl, 256, 4096), 256, 0, st>>>(sp->states.ptr, nl, 1, mlo, lstr.ptr);
-  SQD_CHECK_LAUNCH();
-  upload(dxh, xh, st);
-  upload(dxl, xl, st);
-  upload(dxa, xa, st);
-  upload(dxb, xb, st);
-  upload(dxm, xm, st);
-  upload(dgh, gh, st);
-  upload(dgl, gl, st);
-  upload(dgm, gm, st);
-  if (dense) upload(dtable, table, st);
-  HalfLists H, Lh, A, Bl;
-  half_lists(hstr, nh, dxh, static_cast<int64_t>(xh.size()), H, st);
-  half_lists(lstr, nl, dxl, static_cast<int64_t>(xl.size()), Lh, st);
-  half_lists(hstr, nh, dxa, static_cast<int64_t>(xa.size()), A, st);
-  half_lists(lstr, nl, dxb, static_cast<int64_t>(xb.size()), Bl, st);
-  ProdConnect c{};
-  c.nh = nh;
-  c.nl = nl;
-  c.d = op->has_diag_group;
-  c.hoff = H.off.ptr;
-  c.loff = Lh.off.ptr;
-  c.aoff = A.off.ptr;
-  c.boff = Bl.off.ptr;
-  c.hk = H.k.ptr;
-  c.hp = H.p.ptr;
-  c.lk = Lh.k.ptr;
-  c.lp = Lh.p.ptr;
-  c.ak = A.k.ptr;
-  c.ap = A.p.ptr;
-  c.bk = Bl.k.ptr;
-  c.bp = Bl.p.ptr;
-  c.gh = dgh.ptr;
-  c.gl = dgl.ptr;
-  c.table = dense ? dtable.ptr : nullptr;
-  c.na = static_cast<int64_t>(xa.size());
-  c.nb = static_cast<int64_t>(xb.size());
-  c.xa = dxa.ptr;
-  c.xb = dxb.ptr;
-  c.xm = dxm.ptr;
-  c.gm = dgm.ptr;
-  c.nm = static_cast<int64_t>(xm.size());
-  DevBuf<int64_t> counts;
-  counts.alloc(n, st);
-  const unsigned G = grid_for(n, 256, 16384);
-  k_prod_rows<false><<<G, 256, 0, st>>>(c, counts.ptr, nullptr, nullptr, nullptr);
-  SQD_CHECK_LAUNCH();
-  op->row_ptr.alloc(n + 1, st);
-  exclusive_scan_i64(counts.ptr, op->row_ptr.ptr, n, true, st);
-  copy_to_host(&op->nnz, op->row_ptr.ptr + n, 1, st);
-  counts.release();
-  op->cols.alloc(op->nnz > 0 ? op->nnz : 1, st);
-  op->grps.alloc(op->nnz > 0 ? op->nnz : 1, st);
-  k_prod_rows<true><<<G, 256, 0, st>>>(c, nullptr, op->row_ptr.ptr, op->cols.ptr, op->grps.ptr);
-  SQD_CHECK_LAUNCH();
-  SQD_CUDA(cudaStreamSynchronize(st));  // the host vectors above go out of scope
-  op->product_built = 1;
-  return true;
-}
 
 void op_product_build(sqd_op_s* op, cudaStream_t st) {
   if (op->prod.built) return;
@@ -1172,104 +734,76 @@ void op_product_build(sqd_op_s* op, cudaStream_t st) {
               "the product layout needs cache_strategy (1, 2)");
   SQD_REQUIRE(op->nnz == 0 || op->grps.ptr != nullptr,
               "the operator released its group indices; create a new operator");
-  int64_t nh = 0, nl = 0;
-  if (!op_product_detect(op, st, &nh, &nl))
+  if (!op_plan(op, st))
     throw Error(SQD_ERR_UNSUPPORTED,
                 "the subspace is not a product of high-half and low-half strings without "
                 "fill-in slots; the product layout does not apply");
-  sqd_space_s* sp = op->s;
-  const uint64_t mlo = half_mask_low(sp->num_qubits), mhi = sp->fill_state & ~mlo;
-  const int d = op->has_diag_group;
-  const int64_t n = nh * nl;
+  const ProductPlan& q = *op->plan;
+  const int64_t nh = q.nh, nl = q.nl, n = nh * nl;
   ProductLayout L;
   L.nh = nh;
   L.nl = nl;
   L.wide32 = (nh % 2 == 0 && nl % 2 == 0) ? 1 : 0;
-  DevBuf<unsigned long long> bad;
-  bad.alloc(1, st);
-  SQD_CUDA(cudaMemsetAsync(bad.ptr, 0, sizeof(unsigned long long), st));
-  {
-    DevBuf<int32_t> rkh, rkl;
-    rkh.alloc(n, st);
-    rkl.alloc(n, st);
-    DevBuf<int64_t> kh, kl;
-    kh.alloc(nh, st);
-    kl.alloc(nl, st);
-    const unsigned G = grid_for(n, 256, 16384);
-    k_row_kinds<<<G, 256, 0, st>>>(op->row_ptr.ptr, op->grps.ptr, op->p->group_x.ptr, n, d, mlo,
-                                   mhi, rkh.ptr, rkl.ptr, bad.ptr);
-    SQD_CHECK_LAUNCH();
-    k_slab_meta<<<G, 256, 0, st>>>(rkh.ptr, rkl.ptr, n, nl, d, kh.ptr, kl.ptr, bad.ptr);
-    SQD_CHECK_LAUNCH();
-    unsigned long long hbad = 0;
-    copy_to_host(&hbad, bad.ptr, 1, st);
-    if (hbad)
-      throw Error(SQD_ERR_DEVICE, "stored pairs do not follow the product structure (" +
-                                      std::to_string(hbad) + " rows)");
-    L.ho.alloc(nh + 1, st);
-    L.lo.alloc(nl + 1, st);
-    exclusive_scan_i64(kh.ptr, L.ho.ptr, nh, true, st);
-    exclusive_scan_i64(kl.ptr, L.lo.ptr, nl, true, st);
-  }
-  int64_t th = 0, tl = 0;
-  copy_to_host(&th, L.ho.ptr + nh, 1, st);
-  copy_to_host(&tl, L.lo.ptr + nl, 1, st);
-  L.th = th;
-  L.tl = tl;
-  L.hsrc.alloc(std::max<int64_t>(th, 1), st);
-  L.lsrc.alloc(std::max<int64_t>(tl, 1), st);
-  k_hsrc<<<grid_for(nh, 256, 4096), 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, nh, nl, d,
-                                                   L.ho.ptr, L.hsrc.ptr);
-  SQD_CHECK_LAUNCH();
-  k_lsrc<<<grid_for(nl, 256, 4096), 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, nh, nl, d,
-                                                   L.ho.ptr, L.lo.ptr, L.lsrc.ptr);
-  SQD_CHECK_LAUNCH();
-  L.pairs_h = th * nl;
-  L.pairs_l = tl * nh;
+  L.th = q.th;
+  L.tl = q.tl + q.d * nl;
+  L.pairs_h = L.th * nl;
+  L.pairs_l = L.tl * nh;
   L.pairs_m = op->nnz - L.pairs_h - L.pairs_l;
+  if (L.pairs_m < 0)
+    throw Error(SQD_ERR_DEVICE, "stored pairs do not follow the product structure");
+  L.ho.alloc(nh + 1, st);
+  L.lo.alloc(nl + 1, st);
+  L.hsrc.alloc(std::max<int64_t>(L.th, 1), st);
+  L.lsrc.alloc(std::max<int64_t>(L.tl, 1), st);
+  SQD_CUDA(cudaMemcpyAsync(L.ho.ptr, q.offs.ptr, (nh + 1) * sizeof(int64_t),
+                           cudaMemcpyDeviceToDevice, st));
+  k_slab_sources<<<grid_for(std::max(L.th, nl + 1), 256, 4096), 256, 0, st>>>(
+      plan_view(q), L.th, L.hsrc.ptr, L.lo.ptr, L.lsrc.ptr);
+  SQD_CHECK_LAUNCH();
   const int nca = op->value_complex ? 2 : 1;
   // Panel-major slabs, each panel padded to 32 positions (the padding is never read).
-  const size_t nvh = static_cast<size_t>(std::max<int64_t>(th * ((nl + 31) / 32) * 32, 1)) * nca;
-  const size_t nvl = static_cast<size_t>(std::max<int64_t>(tl * ((nh + 31) / 32) * 32, 1)) * nca;
-  L.vh.alloc(nvh, st);
-  L.vl.alloc(nvl, st);
-  SQD_CUDA(cudaMemsetAsync(L.vh.ptr, 0, nvh * sizeof(double), st));
-  SQD_CUDA(cudaMemsetAsync(L.vl.ptr, 0, nvl * sizeof(double), st));
+  L.vh.alloc(static_cast<size_t>(std::max<int64_t>(L.th * ((nl + 31) / 32) * 32, 1)) * nca, st);
+  L.vl.alloc(static_cast<size_t>(std::max<int64_t>(L.tl * ((nh + 31) / 32) * 32, 1)) * nca, st);
   L.vt.alloc(static_cast<size_t>(n) * 2, st);
   L.tt.alloc(static_cast<size_t>(n) * 2, st);
   L.t.alloc(L.pairs_m > 0 ? static_cast<size_t>(n) * 2 : 1, st);
   op->prod = std::move(L);
-  extract(op, st, 1, bad.ptr);
-  unsigned long long hbad = 0;
-  copy_to_host(&hbad, bad.ptr, 1, st);
-  if (hbad) {
+  try {
+    const bool f32 = op->values32.ptr && op->layout[1] != SQD_LAYOUT_CSR;
+    if (f32) alloc_slabs32(op, st);
+    fill_slabs(op, true, f32, st);
+    build_tail(op, st);
+    if (f32 && op->prod.mval.ptr) to_float(op->prod.mval, op->prod.mval32, st);
+    SQD_CUDA(cudaStreamSynchronize(st));
+  } catch (...) {
     op->prod = ProductLayout();
-    throw Error(SQD_ERR_DEVICE, "stored sources do not follow the product structure (" +
-                                    std::to_string(hbad) + " pairs)");
-  }
-  build_tail(op, st);
-  if (op->values32.ptr && op->layout[1] != SQD_LAYOUT_CSR) {
-    slabs_to_float(op, st);
-    if (op->prod.mval.ptr) to_float(op->prod.mval, op->prod.mval32, st);
+    throw;
   }
   op->prod.built = 1;
-  SQD_CUDA(cudaStreamSynchronize(st));
 }
 
-// Elements again after a coefficient update (sources unchanged).
-void op_product_values(sqd_op_s* op, cudaStream_t st) {
+// A coefficient update (sources unchanged): the slabs are filled beside the pair list, the tails
+// from it.
+void op_product_targets(sqd_op_s* op, ElementOut* out) {
+  ProductLayout& L = op->prod;
+  if (!L.built) return;
+  out->vh = L.vh.ptr;
+  out->vl = L.vl.ptr;
+  out->vh32 = L.vh32.ptr;
+  out->vl32 = L.vl32.ptr;
+  out->wide32 = L.wide32;
+}
+
+void op_product_refresh(sqd_op_s* op, cudaStream_t st) {
   if (!op->prod.built) return;
-  extract(op, st, 0, nullptr);
   refill_tail(op, st);
-  if (op->prod.vh32.ptr) {
-    slabs_to_float(op, st);
-    if (op->prod.mval.ptr) to_float(op->prod.mval, op->prod.mval32, st);
-  }
+  if (op->prod.vh32.ptr && op->prod.mval.ptr) to_float(op->prod.mval, op->prod.mval32, st);
 }
 
 void op_product_values32(sqd_op_s* op, cudaStream_t st) {
   if (!op->prod.built || op->prod.vh32.ptr) return;
-  slabs_to_float(op, st);
+  alloc_slabs32(op, st);
+  fill_slabs(op, false, true, st);
   if (op->prod.mval.ptr) to_float(op->prod.mval, op->prod.mval32, st);
 }
 
