@@ -173,12 +173,14 @@ inline TermTable term_table(const sqd_paulis_s* p) {
 }
 
 // Composed diagonal of a group (its span) at state s, term by term in the reference's order
-// (get_diagonal, sqd.py:603-628): sums of c or -c by the parity of s & z.
-template <int NCA>
-__device__ __forceinline__ Cx<double> compose(const TermTable& T, uint2 sp, uint64_t s) {
+// (get_diagonal, sqd.py:603-628): sums of c or -c by the parity of s & z.  STEP > 1: every
+// STEP-th term from `first` on, one lane's share of the sum.
+template <int NCA, int STEP = 1>
+__device__ __forceinline__ Cx<double> compose(const TermTable& T, uint2 sp, uint64_t s,
+                                              int first = 0) {
   double dr = 0.0, di = 0.0;
 #pragma unroll 4
-  for (uint32_t t = sp.x; t < sp.x + sp.y; ++t) {
+  for (uint32_t t = sp.x + first; t < sp.x + sp.y; t += STEP) {
     const ulonglong2 r = __ldg(T.rec + t);
     const uint64_t v = s & r.x;
     const uint64_t flip =

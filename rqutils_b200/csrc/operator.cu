@@ -343,7 +343,20 @@ void op_build(sqd_op_s* op, cudaStream_t st) {
                                   sp->sector_mask[1], op->gpre.ptr);
     SQD_CHECK_LAUNCH();
   }
-  if (op->x_cache == 0) return;
+  if (op->x_cache == 0) {
+    // Nothing is kept per row; on a product subspace the halves' partner lists (a few hundred
+    // entries per string) let the matvec enumerate its pairs (k_mv_plan).
+    if (op->lookup == SQD_LOOKUP_AUTO || op->lookup == SQD_LOOKUP_PRODUCT) {
+      try {
+        op_plan(op, st);
+      } catch (const Error& e) {   // no memory for the lists: every matvec searches
+        if (e.status != SQD_ERR_MEMORY) throw;
+        (void)cudaGetLastError();
+      }
+      SQD_CUDA(cudaStreamSynchronize(st));
+    }
+    return;
+  }
 
   bool connected = false;
   if (op->lookup == SQD_LOOKUP_AUTO || op->lookup == SQD_LOOKUP_PRODUCT) {

@@ -48,10 +48,7 @@ struct SweepParams {
   uint32_t* grps;
   int diag_first;
   // APPLY
-  const int64_t* group_start;
-  const int32_t* group_eff;
-  const uint64_t* term_z;
-  const double* term_c;
+  TermTable terms;
   const void* vin;
   void* vout;
   int has_diag;
@@ -65,16 +62,8 @@ struct QEntry {
 
 template <typename R, int NCA>
 __device__ __forceinline__ Cx<R> group_diag(const SweepParams& P, int64_t j, uint64_t s) {
-  const int64_t b = P.group_start[j];
-  const int32_t k = P.group_eff[j];
-  R dr = 0, di = 0;
-  for (int32_t t = 0; t < k; ++t) {
-    const uint64_t z = __ldg(P.term_z + b + t);
-    const R sg = parity64(s & z) ? R(-1) : R(1);
-    dr += R(__ldg(P.term_c + 2 * (b + t))) * sg;
-    if constexpr (NCA == 2) di += R(__ldg(P.term_c + 2 * (b + t) + 1)) * sg;
-  }
-  return cx_make<R>(dr, di);
+  const Cx<double> d = compose<NCA>(P.terms, __ldg(P.terms.span + j), s);
+  return cx_make<R>(R(d.re), R(d.im));
 }
 
 template <int MODE, typename R, int NCV, int NCA>
