@@ -48,12 +48,14 @@ struct sqd_space_s {
   int num_sectors = 0;
   uint64_t sector_mask[2] = {0, 0};
   int sector_weight[2] = {0, 0};
-  // Per-sector membership bitmaps over the sector projection (exact when the sector is at most
-  // kBitmapBits wide, hashed otherwise).  Used as a no-false-negative prefilter.
-  sqd::DevBuf<uint32_t> bitmap;       // [num_sectors << kBitmapLog2 / 32]
+  // Membership filter of the sweep: 2^filter_log2 bits, bit filter_bit(s) set for every state s,
+  // at least eight bits per state up to kFilterMax.
+  sqd::DevBuf<uint32_t> filter;
+  int filter_log2 = 0;
 };
 
-constexpr int kBitmapLog2 = 17;
+constexpr int kFilterMin = 10, kFilterMax = 28;
+constexpr int kFilterShared = 20;     // largest filter that the sweep keeps in shared memory
 
 namespace sqd {
 // Low half of the qubits (bits 0 .. n/2 - 1): the low sector of the conserved-weight sectors and
@@ -268,9 +270,13 @@ __device__ __forceinline__ int64_t bsearch_lookup(const uint64_t* __restrict__ s
   return (lo < n && __ldg(states + lo) == key) ? lo : -1;
 }
 
-__device__ __forceinline__ uint32_t sector_bitmap_index(uint64_t proj, int shift, bool exact) {
-  const uint64_t v = exact ? (proj >> shift) : mix64(proj);
-  return static_cast<uint32_t>(v & ((1ull << kBitmapLog2) - 1));
+// Multiplicative hashing of both halves (the 32-bit primes of xxHash, Y. Collet), one mixing
+// step, top bits.
+__device__ __forceinline__ uint32_t filter_bit(uint64_t key, int log2) {
+  uint32_t h = static_cast<uint32_t>(key) * 0x9E3779B1u +
+               static_cast<uint32_t>(key >> 32) * 0x85EBCA77u;
+  h ^= h >> 15;
+  return (h * 0xC2B2AE3Du) >> (32 - log2);
 }
 
 // Build helpers implemented in operator.cu and matvec.cu.

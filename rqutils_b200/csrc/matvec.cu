@@ -265,33 +265,17 @@ void op_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t s
       return;
     }
     // Uncached: sources searched in the matvec.
-    SweepParams P{};
-    P.states = sp->states.ptr;
-    P.n_unique = sp->n_unique;
-    P.gpre = op->gpre.ptr;
-    P.n_gpre = op->n_gpre;
-    P.hkeys = sp->hkeys.ptr;
-    P.hvals = sp->hvals.ptr;
-    P.hmask = sp->hmask;
-    P.lookup = op->lookup == SQD_LOOKUP_BSEARCH ? SQD_LOOKUP_BSEARCH : SQD_LOOKUP_HASH;
-    P.nsec = sp->num_sectors;
-    P.m0 = sp->sector_mask[0];
-    P.m1 = sp->sector_mask[1];
-    P.sh0 = sp->num_sectors > 0 ? __builtin_ctzll(sp->sector_mask[0]) : 0;
-    P.sh1 = sp->num_sectors > 1 ? __builtin_ctzll(sp->sector_mask[1]) : 0;
-    P.ex0 = sp->num_sectors > 0 && __builtin_popcountll(sp->sector_mask[0]) <= kBitmapLog2;
-    P.ex1 = sp->num_sectors > 1 && __builtin_popcountll(sp->sector_mask[1]) <= kBitmapLog2;
-    P.bitmap = sp->bitmap.ptr;
-    P.terms = term_table(p);
+    SweepParams P = sweep_params(op);
     P.vin = v;
     P.vout = out;
     P.has_diag = op->has_diag_group;
-    const size_t dyn = P.bitmap ? (static_cast<size_t>(sp->num_sectors) << kBitmapLog2) / 8 : 0;
-    auto kern = k_sweep<SWEEP_APPLY, R, NCV, NCA>;
+    constexpr int kRows = 512;
+    const size_t dyn = sweep_shared(P);
+    auto kern = k_sweep<SWEEP_APPLY, R, NCV, NCA, kRows, 1>;
     SQD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(dyn)));
     if (sp->n_unique > 0) {
-      kern<<<grid_for(sp->n_unique, SW_TILE), SW_THREADS, dyn, st>>>(P);
+      kern<<<grid_for(sp->n_unique, kRows), kRows, dyn, st>>>(P);
       SQD_CHECK_LAUNCH();
     }
     if (size > sp->n_unique) {

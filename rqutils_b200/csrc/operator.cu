@@ -54,16 +54,34 @@ __global__ void k_gpre_fill(const uint64_t* group_x, int64_t J, const int64_t* f
   }
 }
 
-__global__ void k_fill_counts(int64_t n_unique, int64_t size, int has_diag, int64_t* counts) {
-  for (int64_t r = n_unique + blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < size;
-       r += int64_t(gridDim.x) * blockDim.x)
-    counts[r] = (has_diag && r == size - 1) ? 1 : 0;
+// Fill-in slots: only the last one has an entry (the diagonal group).
+__global__ void k_fill_counts(int64_t n_unique, int64_t size, int chunks, int has_diag,
+                              int64_t* counts) {
+  for (int64_t i = n_unique * chunks + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+       i < size * chunks; i += int64_t(gridDim.x) * blockDim.x)
+    counts[i] = (has_diag && i == (size - 1) * chunks) ? 1 : 0;
 }
 
-__global__ void k_add_const(int64_t* counts, int64_t n, int64_t c) {
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
+__global__ void k_row_starts(const int64_t* __restrict__ place, int64_t size, int chunks,
+                             int64_t* row_ptr) {
+  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r <= size;
        r += int64_t(gridDim.x) * blockDim.x)
-    counts[r] += c;
+    row_ptr[r] = place[r * chunks];
+}
+
+// The pairs that the counting sweep kept, to their rows' slots.
+__global__ void k_scatter_hits(const SweepHit* __restrict__ hits, int64_t n,
+                               const int64_t* __restrict__ place, int chunks, int diag_first,
+                               uint32_t* __restrict__ cols, uint32_t* __restrict__ grps) {
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const uint4 h = __ldg(reinterpret_cast<const uint4*>(hits) + i);
+    const uint32_t chunk = h.w >> 25, rank = h.w & ((1u << 25) - 1u);
+    const int64_t slot = __ldg(place + int64_t(h.x) * chunks + chunk) +
+                         (chunk == 0 ? diag_first : 0) + rank;
+    cols[slot] = h.y;
+    grps[slot] = h.z;
+  }
 }
 
 // Diagonal-group entries: real row r -> (r, 0); last fill-in slot -> (n_unique, 0).
@@ -370,51 +388,65 @@ void op_build(sqd_op_s* op, cudaStream_t st) {
   op_values_and_lanes(op, st);
 }
 
-// Connectivity by the (row, group) sweep: any subspace, fill-in slots included.
+// Connectivity by the (row, group) sweep: any subspace, fill-in slots included.  One sweep finds
+// the pairs, whose order in the buffer is that of the blocks; their places follow from the counts
+// per (row, group chunk).  Subspaces with more pairs than the buffer holds are swept again.
 void op_connect_sweep(sqd_op_s* op, cudaStream_t st) {
+  constexpr int kThreads = 1024, kRpt = 2, kTile = kThreads * kRpt;
+  constexpr int64_t kHitsPerRow = 256, kHitsMax = int64_t(1) << 26;
   sqd_space_s* sp = op->s;
   const int64_t size = sp->states_size;
   const int64_t nu = sp->n_unique;
-  SweepParams P{};
-  P.states = sp->states.ptr;
-  P.n_unique = nu;
-  P.gpre = op->gpre.ptr;
-  P.n_gpre = op->n_gpre;
-  P.hkeys = sp->hkeys.ptr;
-  P.hvals = sp->hvals.ptr;
-  P.hmask = sp->hmask;
-  P.lookup = op->lookup == SQD_LOOKUP_BSEARCH ? SQD_LOOKUP_BSEARCH : SQD_LOOKUP_HASH;
-  P.nsec = sp->num_sectors;
-  P.m0 = sp->sector_mask[0];
-  P.m1 = sp->sector_mask[1];
-  P.sh0 = sp->num_sectors > 0 ? __builtin_ctzll(sp->sector_mask[0]) : 0;
-  P.sh1 = sp->num_sectors > 1 ? __builtin_ctzll(sp->sector_mask[1]) : 0;
-  P.ex0 = sp->num_sectors > 0 && __builtin_popcountll(sp->sector_mask[0]) <= kBitmapLog2;
-  P.ex1 = sp->num_sectors > 1 && __builtin_popcountll(sp->sector_mask[1]) <= kBitmapLog2;
-  P.bitmap = sp->bitmap.ptr;
-  const size_t dyn = P.bitmap ? (static_cast<size_t>(sp->num_sectors) << kBitmapLog2) / 8 : 0;
-  const unsigned tiles = grid_for(nu, SW_TILE);
+  SweepParams P = sweep_params(op);
+  P.diag_first = op->has_diag_group;
+  // Group chunks: about four blocks per SM over all row tiles (one block is resident at a time
+  // with a full filter), at least 32 groups each.
+  const int64_t tiles = (nu + kTile - 1) / kTile;
+  int64_t chunks = std::min<int64_t>(4 * num_sms() / std::max<int64_t>(tiles, 1),
+                                     (op->n_gpre + 31) / 32);
+  chunks = std::max<int64_t>(1, std::min<int64_t>(chunks, kSweepMaxChunks));
+  P.chunk_groups = (op->n_gpre + chunks - 1) / chunks;
+  P.chunks = static_cast<int>(chunks);
+  const size_t dyn = sweep_shared(P);
+  const unsigned blocks = static_cast<unsigned>(tiles * chunks);
 
-  DevBuf<int64_t> counts;
-  counts.alloc(size, st);
-  P.counts = counts.ptr;
+  DevBuf<int64_t> place;
+  place.alloc(size * chunks + 1, st);
+  P.counts = place.ptr;
+  DevBuf<unsigned long long> n_hits;
+  n_hits.alloc(1, st);
+  SQD_CUDA(cudaMemsetAsync(n_hits.ptr, 0, sizeof(unsigned long long), st));
+  P.n_hits = n_hits.ptr;
+  DevBuf<SweepHit> hits;
+  try {
+    const int64_t room = std::min(std::min(nu * kHitsPerRow, kHitsMax), nu * op->n_gpre);
+    hits.alloc(static_cast<size_t>(std::max<int64_t>(room, 1)), st);
+    P.max_hits = static_cast<unsigned long long>(room);
+  } catch (const Error& e) {   // no room for the buffer: two sweeps
+    if (e.status != SQD_ERR_MEMORY) throw;
+    (void)cudaGetLastError();
+  }
+  P.hits = hits.ptr;
   {
-    auto kern = k_sweep<SWEEP_COUNT, double, 1, 1>;
+    auto kern = k_sweep<SWEEP_COUNT, double, 1, 1, kThreads, kRpt>;
     SQD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(dyn)));
-    kern<<<tiles, SW_THREADS, dyn, st>>>(P);
+    kern<<<blocks, kThreads, dyn, st>>>(P);
     SQD_CHECK_LAUNCH();
   }
-  if (op->has_diag_group)
-    k_add_const<<<grid_for(nu, 256, 8192), 256, 0, st>>>(counts.ptr, nu, 1);
-  if (size > nu)
-    k_fill_counts<<<grid_for(size - nu, 256, 1024), 256, 0, st>>>(nu, size, op->has_diag_group,
-                                                                  counts.ptr);
-  SQD_CHECK_LAUNCH();
+  if (size > nu) {
+    k_fill_counts<<<grid_for((size - nu) * chunks, 256, 1024), 256, 0, st>>>(
+        nu, size, P.chunks, op->has_diag_group, place.ptr);
+    SQD_CHECK_LAUNCH();
+  }
+  exclusive_scan_i64(place.ptr, place.ptr, size * chunks, true, st);
   op->row_ptr.alloc(size + 1, st);
-  exclusive_scan_i64(counts.ptr, op->row_ptr.ptr, size, true, st);
+  k_row_starts<<<grid_for(size + 1, 256, 8192), 256, 0, st>>>(place.ptr, size, P.chunks,
+                                                              op->row_ptr.ptr);
+  SQD_CHECK_LAUNCH();
+  unsigned long long found = 0;
+  SQD_CUDA(cudaMemcpyAsync(&found, n_hits.ptr, sizeof(found), cudaMemcpyDeviceToHost, st));
   copy_to_host(&op->nnz, op->row_ptr.ptr + size, 1, st);
-  counts.release();
 
   op->cols.alloc(op->nnz > 0 ? op->nnz : 1, st);
   op->grps.alloc(op->nnz > 0 ? op->nnz : 1, st);
@@ -423,17 +455,23 @@ void op_connect_sweep(sqd_op_s* op, cudaStream_t st) {
                                                              op->cols.ptr, op->grps.ptr);
     SQD_CHECK_LAUNCH();
   }
-  P.row_ptr = op->row_ptr.ptr;
+  if (found <= P.max_hits) {
+    if (found > 0) {
+      k_scatter_hits<<<grid_for(static_cast<int64_t>(found), 256, 16384), 256, 0, st>>>(
+          hits.ptr, static_cast<int64_t>(found), place.ptr, P.chunks, op->has_diag_group,
+          op->cols.ptr, op->grps.ptr);
+      SQD_CHECK_LAUNCH();
+    }
+    return;
+  }
+  P.place = place.ptr;
   P.cols = op->cols.ptr;
   P.grps = op->grps.ptr;
-  P.diag_first = op->has_diag_group;
-  {
-    auto kern = k_sweep<SWEEP_FILL, double, 1, 1>;
-    SQD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(dyn)));
-    kern<<<tiles, SW_THREADS, dyn, st>>>(P);
-    SQD_CHECK_LAUNCH();
-  }
+  auto kern = k_sweep<SWEEP_FILL, double, 1, 1, kThreads, kRpt>;
+  SQD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(dyn)));
+  kern<<<blocks, kThreads, dyn, st>>>(P);
+  SQD_CHECK_LAUNCH();
 }
 
 // Matrix elements of the stored pairs (z = 2) and the initial lanes-per-row choice.

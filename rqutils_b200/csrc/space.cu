@@ -5,7 +5,7 @@
 //    byte rows, because the pad bit is 0 for every real state.
 //  * sqd_space_create: uniquify_states (sqd.py:445-482) — radix sort + unique; the fill-in
 //    slots are kept implicit (states_size > n_unique), then lookup structures are built:
-//    an open-addressing hash table, conserved-weight sectors and sector bitmaps.
+//    an open-addressing hash table, conserved-weight sectors and a membership filter.
 //  * sqd_xsource: get_xsource (sqd.py:485-548) for one X mask, bit-exact including the values
 //    the reference's sort-based algorithm produces for fill-in slots.
 //  * sqd_space_lookup: sorted index of arbitrary keys, for the unsorted-input branch of
@@ -83,29 +83,13 @@ __global__ void k_sector_stats(const uint64_t* __restrict__ s, int64_t n, uint64
   }
 }
 
-__global__ void k_bitmap_build(const uint64_t* __restrict__ s, int64_t n, int nsec, uint64_t m0,
-                               uint64_t m1, int sh0, int sh1, int ex0, int ex1,
-                               uint32_t* bitmap) {
-  constexpr uint32_t words = (1u << kBitmapLog2) / 32;
+__global__ void k_filter_build(const uint64_t* __restrict__ s, int64_t n, int log2,
+                               uint32_t* filter) {
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x) {
-    const uint64_t v = s[i];
-    uint32_t b = sector_bitmap_index(v & m0, sh0, ex0);
-    atomicOr(bitmap + (b >> 5), 1u << (b & 31));
-    if (nsec > 1) {
-      b = sector_bitmap_index(v & m1, sh1, ex1);
-      atomicOr(bitmap + words + (b >> 5), 1u << (b & 31));
-    }
+    const uint32_t b = filter_bit(s[i], log2);
+    atomicOr(filter + (b >> 5), 1u << (b & 31));
   }
-}
-
-__global__ void k_popc_sum(const uint32_t* w, int64_t n, unsigned long long* out) {
-  unsigned long long acc = 0;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * blockDim.x)
-    acc += __popc(w[i]);
-  acc = warp_sum(acc);
-  if ((threadIdx.x & 31) == 0) atomicAdd(out, acc);
 }
 
 // get_xsource for one x.  Real rows: index of s^x or -1.  Fill-in slots f_1..f_m (all equal
@@ -259,29 +243,14 @@ extern "C" int sqd_space_create(const uint64_t* states, int64_t n_in, int num_qu
       sp->sector_mask[0] = m_all;
       sp->sector_weight[0] = hs[0];
     }
-    // Sector bitmaps (kept only if at most half full).
-    if (sp->num_sectors > 0) {
-      const size_t words = (static_cast<size_t>(sp->num_sectors) << kBitmapLog2) / 32;
-      sp->bitmap.alloc(words, st);
-      SQD_CUDA(cudaMemsetAsync(sp->bitmap.ptr, 0, words * sizeof(uint32_t), st));
-      const int sh0 = __builtin_ctzll(sp->sector_mask[0]);
-      const int sh1 = sp->num_sectors > 1 ? __builtin_ctzll(sp->sector_mask[1]) : 0;
-      const int ex0 = __builtin_popcountll(sp->sector_mask[0]) <= kBitmapLog2;
-      const int ex1 = sp->num_sectors > 1 && __builtin_popcountll(sp->sector_mask[1]) <= kBitmapLog2;
-      k_bitmap_build<<<grid_for(nu, 256, 4096), 256, 0, st>>>(
-          sp->states.ptr, nu, sp->num_sectors, sp->sector_mask[0], sp->sector_mask[1], sh0, sh1,
-          ex0, ex1, sp->bitmap.ptr);
-      SQD_CHECK_LAUNCH();
-      DevBuf<unsigned long long> cnt;
-      cnt.alloc(1, st);
-      SQD_CUDA(cudaMemsetAsync(cnt.ptr, 0, sizeof(unsigned long long), st));
-      k_popc_sum<<<64, 256, 0, st>>>(sp->bitmap.ptr, static_cast<int64_t>(words), cnt.ptr);
-      SQD_CHECK_LAUNCH();
-      unsigned long long set = 0;
-      copy_to_host(&set, cnt.ptr, 1, st);
-      if (set > static_cast<unsigned long long>(sp->num_sectors) << (kBitmapLog2 - 1))
-        sp->bitmap.release();
-    }
+    sp->filter_log2 = kFilterMin;
+    while (sp->filter_log2 < kFilterMax && (int64_t(1) << sp->filter_log2) < 8 * nu)
+      ++sp->filter_log2;
+    sp->filter.alloc((size_t(1) << sp->filter_log2) / 32, st);
+    SQD_CUDA(cudaMemsetAsync(sp->filter.ptr, 0, sp->filter.bytes(), st));
+    k_filter_build<<<grid_for(nu, 256, 4096), 256, 0, st>>>(sp->states.ptr, nu, sp->filter_log2,
+                                                            sp->filter.ptr);
+    SQD_CHECK_LAUNCH();
     SQD_CUDA(cudaStreamSynchronize(st));
     *out = sp.release();
   });
