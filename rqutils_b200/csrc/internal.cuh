@@ -90,20 +90,29 @@ struct ProductLayout {
   sqd::DevBuf<float> vh32, vl32;     // FP32 copies (64-wide panels when wide32)
   int wide32 = 0;                    // both halves even: FP32 slabs read two positions per lane
   sqd::DevBuf<double> vt, tt, t;     // per-matvec scratch: transposed input, L and M partials
-  // Compact copies of the row tails (the M pairs of each row, contiguous: mptr, mval) with the
-  // sources in one or both of two forms.  Shared memory (tail_slots > 0), when every slab's M
-  // source slabs fit there together: indices into the block's staged slabs (msidx = slot * nl +
-  // l'), and each slab's source slabs are listed (slist).  Short tails (compact_tail): rows
-  // (mcol), read by the CSR tail kernel.
-  int tail_slots = 0;                // largest number of M source slabs of one slab
-  int compact_tail = 0;
+  // Two-half (M) pairs.  Panel form (SQD_LAYOUT_PRODUCT, product.cu k_tail_panels): the low
+  // strings sorted by the length of their B list (perm, 0xffffffff in the padding) in panels of
+  // 32, panel p with panel_at[p + 1] - panel_at[p] steps; element of A entry k, step t, lane at
+  // ((k * steps + panel_at[p] + t) * 32 + lane); source l' of a step at
+  // panel_src[(panel_at[p] + t) * 32 + lane], nl in the padding.  horder: high strings by the
+  // length of their A list, longest first.  panel_full: every combination's group exists;
+  // otherwise absent elements are marked (kAbsent*).
+  int panel_state = 0;               // 0 not tried, 1 built, -1 does not apply
+  int64_t panels = 0, steps = 0;
+  sqd::DevBuf<int32_t> panel_at;     // [panels + 1]
+  sqd::DevBuf<uint32_t> perm;        // [panels * 32]
+  sqd::DevBuf<uint16_t> panel_src;   // [steps * 32]
+  sqd::DevBuf<uint32_t> horder;      // [nh]
+  int panel_full = 0;
+  sqd::DevBuf<double> vm;            // [ta * steps * 32] (x2 interleaved when complex)
+  sqd::DevBuf<float> vm32;
+  // Otherwise the CSR kernel runs over the row tails: in place, or over a contiguous copy when
+  // they are short (row offsets, elements, source rows).
+  int tail_state = 0;                // 0 not tried, 1 copied, -1 read in place
   sqd::DevBuf<int64_t> mptr;         // [n + 1]
-  sqd::DevBuf<uint16_t> msidx;       // [pairs_m] (shared-memory form)
-  sqd::DevBuf<uint32_t> mcol;        // [pairs_m] (short-tail form)
+  sqd::DevBuf<uint32_t> mcol;        // [pairs_m]
   sqd::DevBuf<double> mval;          // [pairs_m] (x2 interleaved when complex)
   sqd::DevBuf<float> mval32;
-  sqd::DevBuf<int64_t> soff;         // [nh + 1]
-  sqd::DevBuf<uint32_t> slist;       // [soff[nh]] ascending source slabs
 };
 
 // Connectivity of a product subspace by half strings (connect.cu): rows r = h * nl + l.  Four
@@ -141,6 +150,7 @@ struct sqd_op_s {
   int value_complex = 0;
   int64_t nnz = 0;
   int lanes_per_row[2] = {32, 32};  // [0]: FP64 vectors, [1]: FP32 vectors
+  int lanes_chosen[2] = {0, 0};     // set by the caller: also for the tails' CSR kernel
   int64_t chunk_rows[2] = {0, 0};   // rows a block owns at a time (0 = interleaved rows)
   sqd::DevBuf<int64_t> row_ptr;   // [states_size + 1]
   sqd::DevBuf<uint32_t> cols;     // [nnz] source index of each stored pair
@@ -163,6 +173,11 @@ struct sqd_op_s {
 };
 
 namespace sqd {
+
+// Lanes that share a row of the CSR kernels, from the mean number of pairs per row.
+inline int lanes_for(double avg) {
+  return avg >= 96 ? 32 : avg >= 40 ? 16 : avg >= 16 ? 8 : avg >= 6 ? 4 : 2;
+}
 
 // The packed Pauli table as the kernels read it.
 struct TermTable {
@@ -285,7 +300,7 @@ void op_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t s
 void op_ensure_values32(sqd_op_s* op, cudaStream_t st);
 // Product layout (product.cu).
 bool op_product_detect(sqd_op_s* op, cudaStream_t st, int64_t* nh, int64_t* nl);
-void op_product_build(sqd_op_s* op, cudaStream_t st);
+void op_product_build(sqd_op_s* op, int layout, cudaStream_t st);
 void op_product_refresh(sqd_op_s* op, cudaStream_t st);
 void op_product_values32(sqd_op_s* op, cudaStream_t st);
 void op_product_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st);

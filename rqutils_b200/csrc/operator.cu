@@ -490,8 +490,8 @@ void op_values_and_lanes(sqd_op_s* op, cudaStream_t st) {
   }
   // Lanes per row from the mean row length.
   const double avg = nu > 0 ? static_cast<double>(op->nnz) / static_cast<double>(nu) : 0.0;
-  const int lpr = avg >= 96 ? 32 : avg >= 40 ? 16 : avg >= 16 ? 8 : avg >= 6 ? 4 : 2;
-  op->lanes_per_row[0] = op->lanes_per_row[1] = lpr;
+  op->lanes_per_row[0] = op->lanes_per_row[1] = lanes_for(avg);
+  op->lanes_chosen[0] = op->lanes_chosen[1] = 0;
   SQD_CUDA(cudaStreamSynchronize(st));
 }
 
@@ -548,6 +548,7 @@ extern "C" int sqd_op_set_lanes(sqd_op_t op, int precision, int lanes_per_row) {
     SQD_REQUIRE(precision == 0 || precision == 1, "precision must be 0 (FP64) or 1 (FP32)");
     dispatch_lpr(lanes_per_row, [](auto) {});
     op->lanes_per_row[precision] = lanes_per_row;
+    op->lanes_chosen[precision] = 1;
     ++op->schedule_version;
   });
 }

@@ -27,12 +27,11 @@
 // at ~5 TB/s while L2 serves one amplitude per entry (~19 TB/s).  The FP32 copies of the slabs
 // of even-sized halves use 64-wide panels, read by k_slab2 with two adjacent positions per
 // lane (paired 16-byte amplitude loads).
-// Step 4: when all M source slabs of every slab fit in shared memory together (small slabs,
-// e.g. 512 strings per half), k_tail_smem stages them per block and gathers from shared
-// memory through 16-bit indices of a compact copy of the row tails; otherwise (and under
-// SQD_LAYOUT_PRODUCT_CSR) the CSR kernel runs over the row tails, gathering from global
-// memory: from a contiguous copy of the tails (row offsets, elements, source rows) when they
-// average at most kCompactTailMax pairs per row, else inside the rows' pair lists.
+// Step 4: SQD_LAYOUT_PRODUCT reads the M pairs in panels (k_tail_panels: no source per pair, the
+// gathered row of v in shared memory) when most combinations of the halves' partners exist;
+// otherwise, and under SQD_LAYOUT_PRODUCT_CSR, the CSR kernel runs over the row tails, gathering
+// from global memory: from a contiguous copy of the tails (row offsets, elements, source rows)
+// when they average at most kCompactTailMax pairs per row, else inside the rows' pair lists.
 // FP32 vectors keep the compensated accumulation in every part and pass partials in FP64, so
 // the result is rounded once.  The elements are the same numbers as in the CSR arrays; only
 // the summation order of a row changes (L and M pairs before H pairs).
@@ -321,9 +320,28 @@ k_mv_mixed(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ col
   }
 }
 
-// ---- M pairs through shared memory ----------------------------------------------------
-constexpr int kTailThreads = 512;
-constexpr size_t kTailSmemMax = 200 * 1024;
+// ---- M pairs in panels -------------------------------------------------------------------
+// A row's two-half sources are A(h) x B(l) (connect.cu): h' from the high string alone, l' from
+// the low string alone.  So no source is stored per pair: for a fixed A entry (h, h') the sources
+// lie in one row of v, nl amplitudes that a block stages in shared memory, at positions that are
+// the same for every A entry (panel_src, kept in L1).  A lane owns one low string and keeps its
+// sum over all A entries, and the elements of 32 low strings are one 256-byte line per step.
+// Low strings are sorted by the length of their lists, so the lanes of a panel end together; high
+// strings run longest A list first, so that the last blocks are short.
+// Bound by the element stream (DRAM) and the shared-memory gathers, about 10 wavefronts per 32
+// complex128 amplitudes.  32 qubits, 512 x 512 strings, 49.6 M pairs: 117 us complex128, 79 us
+// complex64 (285 us with all source slabs of a high string in shared memory and 32 lanes per row,
+// about 170 us at its best with 16 lanes from the pair list); 48 qubits, 3072 x 2816, 48 M
+// pairs, complex64: 0.20 ms (1.87 ms with 32 lanes per row).
+constexpr unsigned kAbsent64 = 0x7ff8deadu;   // high word of an absent element (a NaN)
+constexpr unsigned kAbsent32 = 0x7fc0deadu;
+constexpr int kPanelMaxWarps = 32, kPanelMaxPerWarp = 4;
+constexpr size_t kPanelSmem = 200 * 1024;
+
+__device__ __forceinline__ bool is_absent(double re) {
+  return static_cast<unsigned>(__double2hiint(re)) == kAbsent64;
+}
+__device__ __forceinline__ bool is_absent(float re) { return __float_as_uint(re) == kAbsent32; }
 
 __device__ __forceinline__ int64_t tail_begin(const int64_t* row_ptr, const int64_t* ho,
                                               const int64_t* lo, int64_t r, int64_t nl) {
@@ -331,78 +349,82 @@ __device__ __forceinline__ int64_t tail_begin(const int64_t* row_ptr, const int6
   return row_ptr[r] + (ho[h + 1] - ho[h]) + (lo[l + 1] - lo[l]);
 }
 
-// Per-row tail lengths and, when bits is given, bits[h][h' / 32] |= 1 << (h' % 32) for every M
-// source slab h' of slab h.
-__global__ void k_tail_mark(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ cols,
-                            const int64_t* __restrict__ ho, const int64_t* __restrict__ lo,
-                            int64_t n, int64_t nl, int64_t words, uint32_t* bits, int64_t* len) {
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
-       r += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t h = r / nl;
-    const int64_t b = tail_begin(row_ptr, ho, lo, r, nl), e = row_ptr[r + 1];
-    len[r] = e - b;
-    if (bits == nullptr) continue;
-    for (int64_t i = b; i < e; ++i) {
-      const uint32_t hs = static_cast<uint32_t>(cols[i] / nl);
-      atomicOr(bits + h * words + (hs >> 5), 1u << (hs & 31));
-    }
+// Source positions of the panels' steps (B entry t of the lane's low string, nl in the padding).
+__global__ void k_panel_src(PlanView c, const int32_t* __restrict__ at,
+                            const uint32_t* __restrict__ perm, int64_t panels, uint16_t* src) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t p = w0; p < panels; p += nw) {
+    const uint32_t l = perm[p * 32 + lane];
+    const int64_t b0 = l < c.nl ? c.boff[l] : 0, b1 = l < c.nl ? c.boff[l + 1] : 0;
+    for (int32_t t = 0; t < at[p + 1] - at[p]; ++t)
+      src[(int64_t(at[p]) + t) * 32 + lane] =
+          static_cast<uint16_t>(b0 + t < b1 ? c.part[b0 + t] : static_cast<uint32_t>(c.nl));
   }
 }
 
-__global__ void k_tail_counts(const uint32_t* __restrict__ bits, int64_t nh, int64_t words,
-                              int64_t* counts, unsigned* max_count) {
-  for (int64_t h = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; h < nh;
-       h += int64_t(gridDim.x) * blockDim.x) {
-    int64_t c = 0;
-    for (int64_t w = 0; w < words; ++w) c += __popc(bits[h * words + w]);
-    counts[h] = c;
-    atomicMax(max_count, static_cast<unsigned>(c));
-  }
-}
-
-__global__ void k_tail_slist(const uint32_t* __restrict__ bits, int64_t nh, int64_t words,
-                             const int64_t* __restrict__ soff, uint32_t* slist) {
-  for (int64_t h = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; h < nh;
-       h += int64_t(gridDim.x) * blockDim.x) {
-    int64_t k = soff[h];
-    for (int64_t w = 0; w < words; ++w) {
-      uint32_t m = bits[h * words + w];
-      while (m) {
-        const int bit = __ffs(m) - 1;
-        m &= m - 1;
-        slist[k++] = static_cast<uint32_t>(w * 32 + bit);
+// Elements from the pair list: a warp is one high string and one panel; every lane walks its
+// row's tail, whose order is A(h) x B(l) without the absent groups.
+template <int NCA>
+__global__ void __launch_bounds__(256)
+k_panel_fill(PlanView c, const int64_t* __restrict__ row_ptr, const double* __restrict__ vals,
+             const int64_t* __restrict__ ho, const int64_t* __restrict__ lo,
+             const int32_t* __restrict__ at, const uint32_t* __restrict__ perm, int64_t panels,
+             int64_t steps, int full, double* vm, float* vm32) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  const int64_t a_first = c.aoff[0];
+  const double gone = __hiloint2double(static_cast<int>(kAbsent64), 0);
+  for (int64_t w = w0; w < c.nh * panels; w += nw) {
+    const int64_t h = w / panels, p = w - h * panels;
+    const uint32_t l = perm[p * 32 + lane];
+    const bool live = l < c.nl;
+    const int64_t b0 = live ? c.boff[l] : 0, b1 = live ? c.boff[l + 1] : 0;
+    int64_t i = live ? tail_begin(row_ptr, ho, lo, h * c.nl + l, c.nl) : 0;
+    const int32_t t0 = at[p], len = at[p + 1] - t0;
+    for (int64_t k = c.aoff[h]; k < c.aoff[h + 1]; ++k) {
+      const uint32_t a = __ldg(c.key + k);
+      for (int32_t t = 0; t < len; ++t) {
+        const bool there = b0 + t < b1 && plan_group(c, a, __ldg(c.key + b0 + t)) >= 0;
+        const int64_t q = ((k - a_first) * steps + t0 + t) * 32 + lane;
+        double re = full ? 0.0 : gone, im = 0.0;   // full: only the padding, a zero
+        if (there) {
+          const Cx<double> el = ld_elem<double, NCA>(vals, i++);
+          re = el.re;
+          im = el.im;
+        }
+        if (vm) {
+          if constexpr (NCA == 2) reinterpret_cast<double2*>(vm)[q] = make_double2(re, im);
+          else vm[q] = re;
+        }
+        if (vm32) {
+          const float fr = there || full ? static_cast<float>(re) : __uint_as_float(kAbsent32);
+          if constexpr (NCA == 2)
+            reinterpret_cast<float2*>(vm32)[q] = make_float2(fr, static_cast<float>(im));
+          else
+            vm32[q] = fr;
+        }
       }
     }
   }
 }
 
-// Compact tail copy: the element, and the source row (mcol, when given) or the shared-memory
-// index (slot of h' among h's sources; with_index).
-template <int NCA>
-__global__ void k_tail_fill(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ cols,
-                            const double* __restrict__ vals, const int64_t* __restrict__ ho,
-                            const int64_t* __restrict__ lo, const uint32_t* __restrict__ bits,
-                            int64_t n, int64_t nl, int64_t words,
-                            const int64_t* __restrict__ mptr, uint16_t* msidx, double* mval,
-                            int with_index, uint32_t* mcol) {
-  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
-       r += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t h = r / nl;
-    const int64_t b = tail_begin(row_ptr, ho, lo, r, nl), e = row_ptr[r + 1];
-    int64_t j = mptr[r];
-    for (int64_t i = b; i < e; ++i, ++j) {
-#pragma unroll
-      for (int t = 0; t < NCA; ++t) mval[NCA * j + t] = vals[NCA * i + t];
-      if (mcol != nullptr) mcol[j] = cols[i];
-      if (!with_index) continue;
-      const int64_t c = cols[i];
-      const int64_t hs = c / nl;
-      int64_t slot = 0;
-      for (int64_t w = 0; w < (hs >> 5); ++w) slot += __popc(bits[h * words + w]);
-      slot += __popc(bits[h * words + (hs >> 5)] & ((1u << (hs & 31)) - 1u));
-      msidx[j] = static_cast<uint16_t>(slot * nl + (c - hs * nl));
-    }
-  }
+// Bytes of a staged row of nl elements and the zero behind it.
+__host__ __device__ __forceinline__ int64_t panel_row(int64_t nl, int element_bytes) {
+  return ((nl + 1) * element_bytes + 15) / 16 * 16;
+}
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* smem, const void* global) {
+  const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(global));
+  else if constexpr (BYTES == 8)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(global));
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(global));
 }
 
 template <typename R, int NC>
@@ -420,82 +442,141 @@ __device__ __forceinline__ Cx<R> sm_elem(const R* p, int64_t i) {
   }
 }
 
-// M pairs of the rows of slab h (split in `chunks` row ranges, one block each): the block
-// copies all M source slabs of h into shared memory once, then LPR lanes per row stream the
-// compact tail (element + 16-bit shared-memory index) and gather from shared memory.
-template <typename R, int NCV, int NCA, int LPR>
-__global__ void __launch_bounds__(kTailThreads)
-k_tail_smem(const int64_t* __restrict__ mptr, const uint16_t* __restrict__ msidx,
-            const R* __restrict__ mval, const R* __restrict__ v, const int64_t* __restrict__ soff,
-            const uint32_t* __restrict__ slist, int64_t nh, int64_t nl, int64_t chunks,
-            double* __restrict__ part) {
-  extern __shared__ __align__(16) unsigned char tail_raw[];
-  using E = std::conditional_t<NCV == 2, std::conditional_t<sizeof(R) == 8, double2, float2>, R>;
-  E* vse = reinterpret_cast<E*>(tail_raw);
-  const R* vs = reinterpret_cast<const R*>(tail_raw);
-  const E* ve = reinterpret_cast<const E*>(v);
-  constexpr int RPW = 32 / LPR;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sub = lane % LPR, slot = lane / LPR;
-  const int nwarps = blockDim.x >> 5;
-  const int64_t per_chunk = (nl + chunks - 1) / chunks;
-  for (int64_t blk = blockIdx.x; blk < nh * chunks; blk += gridDim.x) {
-    const int64_t h = blk / chunks, c = blk - h * chunks;
-    const int64_t s0 = __ldg(soff + h), s1 = __ldg(soff + h + 1);
-    __syncthreads();  // the previous block's slabs are consumed
-    for (int64_t s = s0; s < s1; ++s) {
-      const int64_t base = int64_t(__ldg(slist + s)) * nl;
-      E* dst = vse + (s - s0) * nl;
-      for (int64_t i = threadIdx.x; i < nl; i += blockDim.x) dst[i] = ve[base + i];
-    }
-    __syncthreads();
-    const int64_t l0 = c * per_chunk, l1 = min(nl, l0 + per_chunk);
-    for (int64_t lb = l0 + int64_t(warp) * RPW; lb < l1; lb += int64_t(nwarps) * RPW) {
-      const int64_t l = lb + slot;
-      CAcc<R, NCV, NCA> acc;
-      if (l < l1) {
-        const int64_t r = h * nl + l;
-        const int64_t e = __ldg(mptr + r + 1);
-        int64_t i = __ldg(mptr + r) + sub;
-        for (; i + 3 * LPR < e; i += 4 * LPR) {
-          uint16_t si[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) si[u] = __ldg(msidx + i + u * LPR);
-          Cx<R> a[4], x[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            a[u] = ld_elem<R, NCA>(mval, i + u * LPR);
-            x[u] = sm_elem<R, NCV>(vs, si[u]);
-          }
-          acc.add4(a, x);
-        }
-        for (; i < e; i += LPR) acc.add(ld_elem<R, NCA>(mval, i), sm_elem<R, NCV>(vs, __ldg(msidx + i)));
+// M pairs of one high string, chunk `blockIdx % chunks` of its panels: FP64 partials.  Up to four
+// A entries at a time: their rows of v are staged together (STAGED; rows too long for shared
+// memory are gathered from global memory), then every step of a panel loads its source position
+// once and one element per A entry, four independent 256-byte lines, and one barrier pair serves
+// four entries (one entry at a time spent a third of its time at barriers and in the chain
+// position -> amplitude: 202 us at 512 x 512 strings, 32 qubits, complex128).  Each step's lines
+// are prefetched into L2 six steps ahead (900 x 800 strings: 890 -> 739 us).  Six blocks per SM for
+// the narrow forms cap the registers at 42.
+constexpr int kPanelGroup = 4;
+constexpr int kPanelAhead = 6;
+
+template <typename R, int NCV, int NCA, int P, bool STAGED, bool FULL>
+__global__ void __launch_bounds__(P < kPanelMaxPerWarp ? 256 : 1024, P < kPanelMaxPerWarp ? 6 : 1)
+k_tail_panels(PlanView c, const int32_t* __restrict__ at, const uint32_t* __restrict__ perm,
+              const uint16_t* __restrict__ src, const uint32_t* __restrict__ horder, int panels,
+              int steps, int chunks, int group, const R* __restrict__ vm, const R* __restrict__ v, double* __restrict__ part) {
+  extern __shared__ __align__(16) unsigned char panel_raw[];
+  constexpr int EB = static_cast<int>(sizeof(R)) * NCV;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int at_h = blockIdx.x / chunks, chunk = blockIdx.x - at_h * chunks;
+  const int h = __ldg(horder + at_h);
+  const int nl = static_cast<int>(c.nl);
+  const int64_t a_first = __ldg(c.aoff);
+  const int64_t k0 = __ldg(c.aoff + h);
+  const int nk = static_cast<int>(__ldg(c.aoff + h + 1) - k0);
+  const uint32_t* part_h = c.part + k0;
+  const int row = panel_row(nl, EB) / static_cast<int>(sizeof(R));          // staged row, in R
+  R* rows = reinterpret_cast<R*>(panel_raw);
+  const int64_t stride = int64_t(steps) * 32 * NCA;                         // one A entry of vm
+  CAcc<R, NCV, NCA> acc[P];
+  for (int kb = 0; kb < nk; kb += group) {
+    const int kn = min(group, nk - kb);
+    if constexpr (STAGED) {
+      if (kb) __syncthreads();   // the previous rows are consumed
+      for (int u = 0; u < kn; ++u) {
+        const char* from = reinterpret_cast<const char*>(v) +
+                           int64_t(__ldg(part_h + kb + u)) * c.nl * EB;
+        char* to = reinterpret_cast<char*>(rows + u * row);
+        for (int i = threadIdx.x; i < nl; i += blockDim.x)
+          copy_async<EB>(to + i * EB, from + int64_t(i) * EB);
+        if (threadIdx.x < NCV) rows[u * row + nl * NCV + threadIdx.x] = R(0);   // padding's source
       }
-      acc.merge(LPR);
-      if (sub == 0 && l < l1) acc.store_partial(part, h * nl + l);
+      asm volatile("cp.async.commit_group;");
+      asm volatile("cp.async.wait_group 0;");
+      __syncthreads();
     }
+    const R* x[kPanelGroup];
+#pragma unroll
+    for (int u = 0; u < kPanelGroup; ++u) {
+      if constexpr (STAGED) x[u] = rows + u * row;
+      else x[u] = v + (u < kn ? int64_t(__ldg(part_h + kb + u)) * c.nl * NCV : 0);
+    }
+    const R* vk = vm + (k0 - a_first + kb) * stride;
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      // the panels of a chunk in zigzag order over the warps (their lengths descend)
+      const int p = (i * W + (i & 1 ? W - 1 - warp : warp)) * chunks + chunk;
+      if (p >= panels) continue;
+      const int t0 = __ldg(at + p), len = __ldg(at + p + 1) - t0;
+      const R* vp = vk + (int64_t(t0) * 32 + lane) * NCA;
+      const uint16_t* sp = src + int64_t(t0) * 32 + lane;
+      // KN entries, no branches inside.  FULL: padding multiplies zero by the zero behind the
+      // staged row.  Otherwise absent elements and their amplitudes are replaced by zeros (a
+      // product with an amplitude that does not belong there could be a NaN).
+      auto steps_of = [&](auto kn_t) {
+        constexpr int KN = decltype(kn_t)::value;
+        // a step's lines of one entry, and the entry whose line this lane prefetches
+        constexpr int kLines = 32 * NCA * static_cast<int>(sizeof(R)) / 128;
+        const R* ahead = vp - lane * NCA + (lane / kLines) * stride +
+                         (lane % kLines) * (128 / static_cast<int>(sizeof(R)));
+#pragma unroll 2
+        for (int t = 0; t < len; ++t) {
+          if (lane < KN * kLines && t + kPanelAhead < len)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(ahead + (t + kPanelAhead) * 32 * NCA));
+          int s = __ldg(sp + t * 32);
+          if constexpr (!STAGED) s = min(s, nl - 1);
+          Cx<R> el[kPanelGroup], xv[kPanelGroup];
+#pragma unroll
+          for (int u = 0; u < KN; ++u) el[u] = ld_elem<R, NCA>(vp + u * stride, t * 32);
+#pragma unroll
+          for (int u = 0; u < KN; ++u)
+            xv[u] = STAGED ? sm_elem<R, NCV>(x[u], s) : ld_elem<R, NCV>(x[u], s);
+#pragma unroll
+          for (int u = 0; u < KN; ++u) {
+            if constexpr (FULL) break;
+            const bool gone = is_absent(el[u].re);
+            el[u].re = gone ? R(0) : el[u].re;
+            xv[u].re = gone ? R(0) : xv[u].re;
+            if constexpr (NCV == 2) xv[u].im = gone ? R(0) : xv[u].im;
+          }
+#pragma unroll
+          for (int u = KN; u < kPanelGroup; ++u) el[u] = xv[u] = cx_make<R>(R(0), R(0));
+          acc[i].add4(el, xv);
+        }
+      };
+      if (kn == 4) steps_of(IntTag<4>{});
+      else if (kn == 3) steps_of(IntTag<3>{});
+      else if (kn == 2) steps_of(IntTag<2>{});
+      else steps_of(IntTag<1>{});
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const int p = (i * W + (i & 1 ? W - 1 - warp : warp)) * chunks + chunk;
+    if (p >= panels) continue;
+    const uint32_t l = __ldg(perm + p * 32 + lane);
+    if (l < c.nl) acc[i].store_partial(part, h * c.nl + l);
   }
 }
 
-template <typename R, int NCV, int NCA>
-void allow_tail_smem() {
-  const int bytes = static_cast<int>(kTailSmemMax);
-  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  SQD_CUDA(cudaFuncSetAttribute(k_tail_smem<R, NCV, NCA, 1>, attr, bytes));
-  SQD_CUDA(cudaFuncSetAttribute(k_tail_smem<R, NCV, NCA, 2>, attr, bytes));
-  SQD_CUDA(cudaFuncSetAttribute(k_tail_smem<R, NCV, NCA, 4>, attr, bytes));
-  SQD_CUDA(cudaFuncSetAttribute(k_tail_smem<R, NCV, NCA, 8>, attr, bytes));
-  SQD_CUDA(cudaFuncSetAttribute(k_tail_smem<R, NCV, NCA, 16>, attr, bytes));
-  SQD_CUDA(cudaFuncSetAttribute(k_tail_smem<R, NCV, NCA, 32>, attr, bytes));
+// ---- short row tails ----------------------------------------------------------------------
+__global__ void k_tail_lengths(const int64_t* __restrict__ row_ptr, const int64_t* __restrict__ ho,
+                               const int64_t* __restrict__ lo, int64_t n, int64_t nl,
+                               int64_t* len) {
+  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
+       r += int64_t(gridDim.x) * blockDim.x)
+    len[r] = row_ptr[r + 1] - tail_begin(row_ptr, ho, lo, r, nl);
 }
 
-void allow_tail_smem_all() {
-  allow_tail_smem<double, 1, 1>();
-  allow_tail_smem<double, 2, 1>();
-  allow_tail_smem<double, 2, 2>();
-  allow_tail_smem<float, 1, 1>();
-  allow_tail_smem<float, 2, 1>();
-  allow_tail_smem<float, 2, 2>();
+// Contiguous copy of the row tails: elements and (mcol, when given) source rows.
+template <int NCA>
+__global__ void k_tail_fill(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ cols,
+                            const double* __restrict__ vals, const int64_t* __restrict__ ho,
+                            const int64_t* __restrict__ lo, int64_t n, int64_t nl,
+                            const int64_t* __restrict__ mptr, double* mval, uint32_t* mcol) {
+  for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n;
+       r += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t b = tail_begin(row_ptr, ho, lo, r, nl), e = row_ptr[r + 1];
+    int64_t j = mptr[r];
+    for (int64_t i = b; i < e; ++i, ++j) {
+#pragma unroll
+      for (int t = 0; t < NCA; ++t) mval[NCA * j + t] = vals[NCA * i + t];
+      if (mcol != nullptr) mcol[j] = cols[i];
+    }
+  }
 }
 
 unsigned capped_grid(int64_t blocks) {
@@ -579,157 +660,224 @@ void alloc_slabs32(sqd_op_s* op, cudaStream_t st) {
   L.vl32.alloc(static_cast<size_t>(std::max<int64_t>((L.nh + w - 1) / w * L.tl * w, 1)) * nca, st);
 }
 
-// A row tail read in place is a short segment of the row's long pair list (C3-like subspaces:
+// A row tail read in place is a short segment of the row's long pair list (48-qubit subspaces:
 // ~11 M pairs among ~160), so its element and source loads use few bytes of the sectors they
 // fetch.  Tails up to this many pairs per row on average are also copied contiguously.
 constexpr int64_t kCompactTailMax = 32;
 
-// Shared-memory form of the M pairs, when every slab's M source slabs fit in kTailSmemMax
-// together (at 8 bytes per amplitude) and 16-bit indices reach them.  Fills len (per-row tail
-// lengths) either way; returns whether the form was built.
-bool build_tail_smem(sqd_op_s* op, DevBuf<int64_t>& len, cudaStream_t st) {
+void fill_panels(sqd_op_s* op, bool f64, bool f32, cudaStream_t st) {
   ProductLayout& L = op->prod;
-  const int64_t nh = L.nh, nl = L.nl, n = nh * nl;
-  const unsigned G = grid_for(n, 256, 16384);
-  if (nh > 65536) {
-    k_tail_mark<<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, L.ho.ptr, L.lo.ptr, n, nl, 0,
-                                   nullptr, len.ptr);
+  const unsigned G = grid_for(L.nh * L.panels * 32, 256, num_sms() * 64);
+  auto run = [&](auto nca) {
+    k_panel_fill<decltype(nca)::value><<<G, 256, 0, st>>>(
+        plan_view(*op->plan), op->row_ptr.ptr, op->values.ptr, L.ho.ptr, L.lo.ptr, L.panel_at.ptr,
+        L.perm.ptr, L.panels, L.steps, L.panel_full, f64 ? L.vm.ptr : nullptr,
+        f32 ? L.vm32.ptr : nullptr);
     SQD_CHECK_LAUNCH();
-    return false;
-  }
-  const int64_t words = (nh + 31) / 32;
-  DevBuf<uint32_t> bits;
-  bits.alloc(static_cast<size_t>(nh * words), st);
-  SQD_CUDA(cudaMemsetAsync(bits.ptr, 0, sizeof(uint32_t) * nh * words, st));
-  DevBuf<int64_t> counts;
-  counts.alloc(nh, st);
-  DevBuf<unsigned> maxc;
-  maxc.alloc(1, st);
-  SQD_CUDA(cudaMemsetAsync(maxc.ptr, 0, sizeof(unsigned), st));
-  k_tail_mark<<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, L.ho.ptr, L.lo.ptr, n, nl, words,
-                                 bits.ptr, len.ptr);
-  SQD_CHECK_LAUNCH();
-  k_tail_counts<<<grid_for(nh, 256, 4096), 256, 0, st>>>(bits.ptr, nh, words, counts.ptr,
-                                                          maxc.ptr);
-  SQD_CHECK_LAUNCH();
-  unsigned slots = 0;
-  copy_to_host(&slots, maxc.ptr, 1, st);
-  const int64_t span = static_cast<int64_t>(slots) * nl;
-  if (slots == 0 || span > 65535 || static_cast<size_t>(span) * 8 > kTailSmemMax) return false;
-  L.soff.alloc(nh + 1, st);
-  exclusive_scan_i64(counts.ptr, L.soff.ptr, nh, true, st);
-  int64_t total = 0;
-  copy_to_host(&total, L.soff.ptr + nh, 1, st);
-  L.slist.alloc(std::max<int64_t>(total, 1), st);
-  k_tail_slist<<<grid_for(nh, 256, 4096), 256, 0, st>>>(bits.ptr, nh, words, L.soff.ptr,
-                                                         L.slist.ptr);
-  SQD_CHECK_LAUNCH();
-  L.mptr.alloc(n + 1, st);
-  exclusive_scan_i64(len.ptr, L.mptr.ptr, n, true, st);
-  const int nca = op->value_complex ? 2 : 1;
-  L.msidx.alloc(static_cast<size_t>(L.pairs_m), st);
-  L.mval.alloc(static_cast<size_t>(L.pairs_m) * nca, st);
-  if (nca == 2)
-    k_tail_fill<2><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->values.ptr, L.ho.ptr,
-                                      L.lo.ptr, bits.ptr, n, nl, words, L.mptr.ptr, L.msidx.ptr,
-                                      L.mval.ptr, 1, nullptr);
-  else
-    k_tail_fill<1><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->values.ptr, L.ho.ptr,
-                                      L.lo.ptr, bits.ptr, n, nl, words, L.mptr.ptr, L.msidx.ptr,
-                                      L.mval.ptr, 1, nullptr);
-  SQD_CHECK_LAUNCH();
-  allow_tail_smem_all();
-  SQD_CUDA(cudaStreamSynchronize(st));
-  L.tail_slots = static_cast<int>(slots);
-  return true;
+  };
+  if (op->value_complex) run(IntTag<2>{});
+  else run(IntTag<1>{});
 }
 
-// Compact forms of the M pairs: the shared-memory form where it applies, and the short-tail
-// form (source rows beside the same contiguous elements, for the CSR tail kernel) when the
-// tails average at most kCompactTailMax pairs per row.  Longer tails are read in place.
+// Panel form of the M pairs.  It applies when most of A(h) x B(l) exists (the panels hold every
+// combination; up to 1.6 elements per stored pair, where the stream still costs less than
+// sources and scattered gathers) and 16 bits reach a row of v.
+void build_panels(sqd_op_s* op, cudaStream_t st) {
+  ProductLayout& L = op->prod;
+  const ProductPlan& q = *op->plan;
+  L.panel_state = -1;
+  if (L.pairs_m <= 0 || q.ta == 0 || q.tb == 0 || L.nl > 65535) return;
+  std::vector<int64_t> boff(static_cast<size_t>(L.nl) + 1);
+  copy_to_host(boff.data(), plan_view(q).boff, boff.size(), st);
+  std::vector<uint32_t> perm(static_cast<size_t>((L.nl + 31) / 32 * 32), 0xffffffffu);
+  for (int64_t l = 0; l < L.nl; ++l) perm[static_cast<size_t>(l)] = static_cast<uint32_t>(l);
+  auto len = [&](uint32_t l) { return boff[l + 1] - boff[l]; };
+  std::stable_sort(perm.begin(), perm.begin() + L.nl,
+                   [&](uint32_t a, uint32_t b) { return len(a) > len(b); });
+  std::vector<int64_t> aoff(static_cast<size_t>(L.nh) + 1);
+  copy_to_host(aoff.data(), plan_view(q).aoff, aoff.size(), st);
+  std::vector<uint32_t> horder(static_cast<size_t>(L.nh));
+  for (int64_t h = 0; h < L.nh; ++h) horder[static_cast<size_t>(h)] = static_cast<uint32_t>(h);
+  std::stable_sort(horder.begin(), horder.end(), [&](uint32_t a, uint32_t b) {
+    return aoff[a + 1] - aoff[a] > aoff[b + 1] - aoff[b];
+  });
+  // Rows too long to stage have no zero behind them for the padding.
+  L.panel_full = L.pairs_m == q.ta * q.tb &&
+                 panel_row(L.nl, 16) <= static_cast<int64_t>(kPanelSmem);
+  const int64_t panels = (L.nl + 31) / 32;
+  std::vector<int32_t> at(static_cast<size_t>(panels) + 1, 0);
+  int64_t steps = 0;
+  for (int64_t p = 0; p < panels; ++p) {
+    at[static_cast<size_t>(p)] = static_cast<int32_t>(steps);
+    steps += len(perm[static_cast<size_t>(p * 32)]);
+  }
+  at[static_cast<size_t>(panels)] = static_cast<int32_t>(steps);
+  const double total = double(q.ta) * double(steps) * 32.0;
+  if (steps > INT_MAX / 64 || total > 1.6 * double(L.pairs_m)) return;
+  const int nca = op->value_complex ? 2 : 1;
+  try {
+    L.panel_at.alloc(at.size(), st);
+    L.perm.alloc(perm.size(), st);
+    L.horder.alloc(horder.size(), st);
+    L.panel_src.alloc(static_cast<size_t>(steps) * 32, st);
+    L.vm.alloc(static_cast<size_t>(q.ta * steps * 32) * nca, st);
+  } catch (const Error& e) {   // no memory: the tails are read as CSR rows
+    if (e.status != SQD_ERR_MEMORY) throw;
+    (void)cudaGetLastError();
+    L.panel_at = DevBuf<int32_t>();
+    L.perm = DevBuf<uint32_t>();
+    L.horder = DevBuf<uint32_t>();
+    L.panel_src = DevBuf<uint16_t>();
+    L.vm = DevBuf<double>();
+    return;
+  }
+  SQD_CUDA(cudaMemcpyAsync(L.panel_at.ptr, at.data(), L.panel_at.bytes(), cudaMemcpyHostToDevice,
+                           st));
+  SQD_CUDA(cudaMemcpyAsync(L.perm.ptr, perm.data(), L.perm.bytes(), cudaMemcpyHostToDevice, st));
+  SQD_CUDA(cudaMemcpyAsync(L.horder.ptr, horder.data(), L.horder.bytes(), cudaMemcpyHostToDevice,
+                           st));
+  L.panels = panels;
+  L.steps = steps;
+  k_panel_src<<<grid_for(panels * 32, 256, 4096), 256, 0, st>>>(
+      plan_view(q), L.panel_at.ptr, L.perm.ptr, panels, L.panel_src.ptr);
+  SQD_CHECK_LAUNCH();
+  fill_panels(op, true, false, st);
+  SQD_CUDA(cudaStreamSynchronize(st));   // the host vectors above go out of scope
+  L.panel_state = 1;
+}
+
+void fill_tail(sqd_op_s* op, bool sources, cudaStream_t st) {
+  ProductLayout& L = op->prod;
+  const int64_t n = L.nh * L.nl;
+  const unsigned G = grid_for(n, 256, 16384);
+  auto run = [&](auto nca) {
+    k_tail_fill<decltype(nca)::value><<<G, 256, 0, st>>>(
+        op->row_ptr.ptr, op->cols.ptr, op->values.ptr, L.ho.ptr, L.lo.ptr, n, L.nl, L.mptr.ptr,
+        L.mval.ptr, sources ? L.mcol.ptr : nullptr);
+    SQD_CHECK_LAUNCH();
+  };
+  if (op->value_complex) run(IntTag<2>{});
+  else run(IntTag<1>{});
+}
+
+// Contiguous copy of short row tails; longer ones, or without memory for it, are read in place.
 void build_tail(sqd_op_s* op, cudaStream_t st) {
   ProductLayout& L = op->prod;
   const int64_t n = L.nh * L.nl;
-  if (L.pairs_m <= 0) return;
+  L.tail_state = -1;
+  if (L.pairs_m <= 0 || L.pairs_m > kCompactTailMax * n) return;
   DevBuf<int64_t> len;
-  len.alloc(n, st);
-  const bool smem = build_tail_smem(op, len, st);
-  if (L.pairs_m > kCompactTailMax * n) return;
   const int nca = op->value_complex ? 2 : 1;
-  // The copy is optional: without device memory for it the tails are read in place.
   try {
-    if (!smem) {
-      L.mptr.alloc(n + 1, st);
-      L.mval.alloc(static_cast<size_t>(L.pairs_m) * nca, st);
-    }
+    len.alloc(n, st);
+    L.mptr.alloc(n + 1, st);
+    L.mval.alloc(static_cast<size_t>(L.pairs_m) * nca, st);
     L.mcol.alloc(static_cast<size_t>(L.pairs_m), st);
   } catch (const Error& e) {
     if (e.status != SQD_ERR_MEMORY) throw;
     (void)cudaGetLastError();  // the failed pool allocation
-    if (!smem) {
-      L.mptr = DevBuf<int64_t>();
-      L.mval = DevBuf<double>();
-    }
+    L.mptr = DevBuf<int64_t>();
+    L.mval = DevBuf<double>();
     L.mcol = DevBuf<uint32_t>();
     return;
   }
-  if (!smem) exclusive_scan_i64(len.ptr, L.mptr.ptr, n, true, st);
-  const unsigned G = grid_for(n, 256, 16384);
-  if (nca == 2)
-    k_tail_fill<2><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->values.ptr, L.ho.ptr,
-                                      L.lo.ptr, nullptr, n, L.nl, 0, L.mptr.ptr, nullptr,
-                                      L.mval.ptr, 0, L.mcol.ptr);
-  else
-    k_tail_fill<1><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->values.ptr, L.ho.ptr,
-                                      L.lo.ptr, nullptr, n, L.nl, 0, L.mptr.ptr, nullptr,
-                                      L.mval.ptr, 0, L.mcol.ptr);
+  k_tail_lengths<<<grid_for(n, 256, 16384), 256, 0, st>>>(op->row_ptr.ptr, L.ho.ptr, L.lo.ptr, n,
+                                                          L.nl, len.ptr);
   SQD_CHECK_LAUNCH();
-  SQD_CUDA(cudaStreamSynchronize(st));
-  L.compact_tail = 1;
+  exclusive_scan_i64(len.ptr, L.mptr.ptr, n, true, st);
+  fill_tail(op, true, st);
+  L.tail_state = 1;
 }
 
-// Tail elements again after a coefficient update (sources unchanged).
-void refill_tail(sqd_op_s* op, cudaStream_t st) {
+// The form of the M pairs that a layout reads, on its first use.
+void build_mixed(sqd_op_s* op, int layout, cudaStream_t st) {
   ProductLayout& L = op->prod;
-  if (L.mval.ptr == nullptr) return;
-  const int64_t n = L.nh * L.nl;
-  const unsigned G = grid_for(n, 256, 16384);
-  if (op->value_complex)
-    k_tail_fill<2><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->values.ptr, L.ho.ptr,
-                                      L.lo.ptr, nullptr, n, L.nl, 0, L.mptr.ptr, nullptr,
-                                      L.mval.ptr, 0, nullptr);
-  else
-    k_tail_fill<1><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->values.ptr, L.ho.ptr,
-                                      L.lo.ptr, nullptr, n, L.nl, 0, L.mptr.ptr, nullptr,
-                                      L.mval.ptr, 0, nullptr);
-  SQD_CHECK_LAUNCH();
+  if (layout == SQD_LAYOUT_PRODUCT && L.panel_state == 0) build_panels(op, st);
+  if ((layout == SQD_LAYOUT_PRODUCT_CSR || L.panel_state < 0) && L.tail_state == 0)
+    build_tail(op, st);
+}
+
+// FP32 copies of whatever exists in FP64 and has none yet.
+void ensure_floats(sqd_op_s* op, cudaStream_t st) {
+  ProductLayout& L = op->prod;
+  if (!L.vh32.ptr) {
+    alloc_slabs32(op, st);
+    fill_slabs(op, false, true, st);
+  }
+  if (L.panel_state == 1 && !L.vm32.ptr) {
+    try {
+      L.vm32.alloc(L.vm.count, st);
+      fill_panels(op, false, true, st);
+    } catch (const Error& e) {   // no memory: FP32 tails are read from the pair list
+      if (e.status != SQD_ERR_MEMORY) throw;
+      (void)cudaGetLastError();
+    }
+  }
+  if (L.tail_state == 1 && !L.mval32.ptr) to_float(L.mval, L.mval32, st);
 }
 
 template <typename R, int NCV, int NCA>
-bool launch_tail_smem(sqd_op_s* op, int prec, const R* vin, cudaStream_t st) {
+bool launch_panels(sqd_op_s* op, const R* vin, cudaStream_t st) {
   ProductLayout& L = op->prod;
-  if (!L.tail_slots) return false;
-  const size_t bytes = static_cast<size_t>(L.tail_slots) * L.nl * NCV * sizeof(R);
-  if (bytes > kTailSmemMax) return false;
-  const R* mv;
-  if constexpr (sizeof(R) == 8) mv = L.mval.ptr;
-  else mv = L.mval32.ptr;
-  if (mv == nullptr) return false;
-  const int64_t chunks =
-      std::max<int64_t>(1, std::min<int64_t>(8, (4 * int64_t(num_sms()) + L.nh - 1) / L.nh));
-  dispatch_lpr(op->lanes_per_row[prec], [&](auto lpr_t) {
-    constexpr int LPR = decltype(lpr_t)::value;
-    k_tail_smem<R, NCV, NCA, LPR><<<capped_grid(L.nh * chunks), kTailThreads, bytes, st>>>(
-        L.mptr.ptr, L.msidx.ptr, mv, vin, L.soff.ptr, L.slist.ptr, L.nh, L.nl, chunks, L.t.ptr);
+  if (L.panel_state != 1) return false;
+  const R* vm;
+  if constexpr (sizeof(R) == 8) vm = L.vm.ptr;
+  else vm = L.vm32.ptr;
+  if (vm == nullptr) return false;
+  // Rows staged together: four, or what fits in half of the shared memory (two blocks per SM),
+  // at least one.
+  const size_t row = static_cast<size_t>(panel_row(L.nl, static_cast<int>(sizeof(R)) * NCV));
+  const bool staged = row <= kPanelSmem;
+  const int group = staged ? static_cast<int>(std::max<size_t>(
+                                 1, std::min<size_t>(kPanelGroup, kPanelSmem / 2 / row)))
+                           : kPanelGroup;
+  // Panels per block: one per warp, eight warps, unless the staged row is more than their elements
+  // (short B lists: 48 qubits, 2.3 steps a panel) or there are fewer than six blocks per SM.
+  const double line = 32.0 * sizeof(R) * NCA * double(L.steps) / double(L.panels);
+  const int64_t most = kPanelMaxWarps * kPanelMaxPerWarp;
+  int64_t mine = std::max<int64_t>(8, static_cast<int64_t>(double(row) / std::max(line, 1.0)));
+  mine = std::min(std::min(mine, most), L.panels);
+  while (mine > 4 && L.nh * ((L.panels + mine - 1) / mine) < 6 * int64_t(num_sms())) --mine;
+  const int64_t chunks = (L.panels + mine - 1) / mine;
+  mine = (L.panels + chunks - 1) / chunks;
+  const int64_t per = std::max((mine + kPanelMaxWarps - 1) / kPanelMaxWarps,
+                               std::min<int64_t>(kPanelMaxPerWarp, (mine + 7) / 8));
+  const int64_t warps = (mine + per - 1) / per;
+  SQD_REQUIRE(L.nh * chunks <= INT_MAX, "too many high strings");
+  const unsigned G = static_cast<unsigned>(L.nh * chunks);
+  auto go = [&](auto kern) {
+    const size_t dyn = staged ? group * row : 0;
+    if (dyn > 48 * 1024)
+      SQD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(kPanelSmem)));
+    kern<<<G, static_cast<unsigned>(warps * 32), dyn, st>>>(
+        plan_view(*op->plan), L.panel_at.ptr, L.perm.ptr, L.panel_src.ptr, L.horder.ptr,
+        static_cast<int>(L.panels), static_cast<int>(L.steps), static_cast<int>(chunks), group, vm,
+        vin, L.t.ptr);
     SQD_CHECK_LAUNCH();
-  });
+  };
+  auto pick = [&](auto p) {
+    constexpr int P = decltype(p)::value;
+    if (!staged) go(k_tail_panels<R, NCV, NCA, P, false, false>);
+    else if (L.panel_full) go(k_tail_panels<R, NCV, NCA, P, true, true>);
+    else go(k_tail_panels<R, NCV, NCA, P, true, false>);
+  };
+  switch (per) {
+    case 1: pick(IntTag<1>{}); break;
+    case 2: pick(IntTag<2>{}); break;
+    case 3: pick(IntTag<3>{}); break;
+    default: pick(IntTag<4>{}); break;
+  }
   return true;
 }
 
 }  // namespace
 
-void op_product_build(sqd_op_s* op, cudaStream_t st) {
-  if (op->prod.built) return;
+void op_product_build(sqd_op_s* op, int layout, cudaStream_t st) {
+  if (op->prod.built) {
+    build_mixed(op, layout, st);
+    return;
+  }
   SQD_REQUIRE(op->x_cache == 1 && op->z_cache == 2,
               "the product layout needs cache_strategy (1, 2)");
   SQD_REQUIRE(op->nnz == 0 || op->grps.ptr != nullptr,
@@ -769,11 +917,8 @@ void op_product_build(sqd_op_s* op, cudaStream_t st) {
   L.t.alloc(L.pairs_m > 0 ? static_cast<size_t>(n) * 2 : 1, st);
   op->prod = std::move(L);
   try {
-    const bool f32 = op->values32.ptr && op->layout[1] != SQD_LAYOUT_CSR;
-    if (f32) alloc_slabs32(op, st);
-    fill_slabs(op, true, f32, st);
-    build_tail(op, st);
-    if (f32 && op->prod.mval.ptr) to_float(op->prod.mval, op->prod.mval32, st);
+    fill_slabs(op, true, false, st);
+    build_mixed(op, layout, st);
     SQD_CUDA(cudaStreamSynchronize(st));
   } catch (...) {
     op->prod = ProductLayout();
@@ -795,16 +940,15 @@ void op_product_targets(sqd_op_s* op, ElementOut* out) {
 }
 
 void op_product_refresh(sqd_op_s* op, cudaStream_t st) {
-  if (!op->prod.built) return;
-  refill_tail(op, st);
-  if (op->prod.vh32.ptr && op->prod.mval.ptr) to_float(op->prod.mval, op->prod.mval32, st);
+  ProductLayout& L = op->prod;
+  if (!L.built) return;
+  if (L.panel_state == 1) fill_panels(op, true, L.vm32.ptr != nullptr, st);
+  if (L.tail_state == 1) fill_tail(op, false, st);
+  if (L.mval32.ptr) to_float(L.mval, L.mval32, st);
 }
 
 void op_product_values32(sqd_op_s* op, cudaStream_t st) {
-  if (!op->prod.built || op->prod.vh32.ptr) return;
-  alloc_slabs32(op, st);
-  fill_slabs(op, false, true, st);
-  if (op->prod.mval.ptr) to_float(op->prod.mval, op->prod.mval32, st);
+  if (op->prod.built) ensure_floats(op, st);
 }
 
 void op_product_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st) {
@@ -850,13 +994,17 @@ void op_product_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaSt
     // 4. M part: t3[r]
     if (L.pairs_m > 0) {
       if (op->layout[prec] == SQD_LAYOUT_PRODUCT_CSR ||
-          !launch_tail_smem<R, NCV, NCA>(op, prec, vin, st)) {
+          !launch_panels<R, NCV, NCA>(op, vin, st)) {
         const R* MV = nullptr;  // the short-tail copy's elements, when it exists
-        if (L.compact_tail) {
+        if (L.tail_state == 1) {
           if constexpr (sizeof(R) == 8) MV = L.mval.ptr;
           else MV = L.mval32.ptr;
         }
-        dispatch_lpr(op->lanes_per_row[prec], [&](auto lpr_t) {
+        // lanes from the mean tail length unless the caller chose them (48 qubits, 3072 x 2816
+        // strings: 5.6 pairs a tail, 1.87 ms with the whole row's 32 lanes)
+        const int lanes = op->lanes_chosen[prec] ? op->lanes_per_row[prec]
+                                                 : lanes_for(double(L.pairs_m) / double(n));
+        dispatch_lpr(lanes, [&](auto lpr_t) {
           constexpr int LPR = decltype(lpr_t)::value;
           if (MV != nullptr)
             k_mv_mixed<R, NCV, NCA, LPR, true><<<mixed_grid(n, LPR), 256, 0, st>>>(
@@ -892,7 +1040,7 @@ extern "C" int sqd_op_set_layout(sqd_op_t op, int precision, int layout, void* s
                 "unknown layout");
     if (layout != SQD_LAYOUT_CSR) {
       cudaStream_t st = as_stream(stream);
-      op_product_build(op, st);
+      op_product_build(op, layout, st);
       if (precision == 1) {
         const int prev = op->layout[1];
         op->layout[1] = layout;
