@@ -123,11 +123,52 @@ struct CAcc {
     else
       p[i] = re.value_d();
   }
+  // The result at element i of a vector.
+  __device__ __forceinline__ void store(R* out, int64_t i) const {
+    st_elem<R, NCV>(out, i, cx_make<R>(re.value(), im.value()));
+  }
+};
+
+// Two complex vectors at once: each as it is summed alone.
+template <typename R, int NCA>
+struct CAcc<R, 4, NCA> {
+  CAcc<R, 2, NCA> a, b;
+  __device__ __forceinline__ void add(Cx<R> m, Cx2<R> x) {
+    a.add(m, x.a);
+    b.add(m, x.b);
+  }
+  __device__ __forceinline__ void add4(const Cx<R>* m, const Cx2<R>* x) {
+    static_assert(sizeof(R) == 8, "pairs of vectors: FP64");
+#pragma unroll
+    for (int u = 0; u < 4; ++u) add(m[u], x[u]);
+  }
+  __device__ __forceinline__ void merge(int width) {
+    a.merge(width);
+    b.merge(width);
+  }
+  __device__ __forceinline__ void add_partial(const double* p, int64_t i) {
+    a.add_partial(p, 2 * i);
+    b.add_partial(p, 2 * i + 1);
+  }
+  __device__ __forceinline__ void store_partial(double* p, int64_t i) const {
+    a.store_partial(p, 2 * i);
+    b.store_partial(p, 2 * i + 1);
+  }
+  __device__ __forceinline__ void store(R* out, int64_t i) const {
+    a.store(out, 2 * i);
+    b.store(out, 2 * i + 1);
+  }
 };
 
 // One lane's share of a CSR row: pairs i0, i0 + LPR, ... below e.  Four pairs per step with
 // independent index -> amplitude gathers in flight, then the remainder.
 // CG: read v through L2 (v written earlier in the same launch by other blocks).
+template <typename R, int NCV, bool CG>
+__device__ __forceinline__ Elem<R, NCV> amplitude(const R* __restrict__ v, int64_t i) {
+  if constexpr (CG) return ld_elem_cg<R, NCV>(v, i);
+  else return ld_elem<R, NCV>(v, i);
+}
+
 template <typename R, int NCV, int NCA, int LPR, bool CG = false>
 __device__ __forceinline__ void csr_row_dot(const uint32_t* __restrict__ cols,
                                             const R* __restrict__ vals,
@@ -138,11 +179,12 @@ __device__ __forceinline__ void csr_row_dot(const uint32_t* __restrict__ cols,
     uint32_t c[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) c[u] = __ldg(cols + i + u * LPR);
-    Cx<R> a[4], x[4];
+    Cx<R> a[4];
+    Elem<R, NCV> x[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       a[u] = ld_elem<R, NCA>(vals, i + u * LPR);
-      x[u] = CG ? ld_elem_cg<R, NCV>(v, c[u]) : ld_elem<R, NCV>(v, c[u]);
+      x[u] = amplitude<R, NCV, CG>(v, c[u]);
     }
     acc.add4(a, x);
   }
@@ -160,7 +202,7 @@ __device__ __forceinline__ void csr_row_dot(const uint32_t* __restrict__ cols,
       for (int u = 0; u < 4; ++u) {
         const bool ok = i + u * LPR < e;
         a[u] = ok ? ld_elem<R, NCA>(vals, i + u * LPR) : cx_make<R>(R(0), R(0));
-        x[u] = ok ? (CG ? ld_elem_cg<R, NCV>(v, c[u]) : ld_elem<R, NCV>(v, c[u]))
+        x[u] = ok ? (amplitude<R, NCV, CG>(v, c[u]))
                   : cx_make<R>(R(0), R(0));
       }
       acc.add4(a, x);
@@ -168,7 +210,7 @@ __device__ __forceinline__ void csr_row_dot(const uint32_t* __restrict__ cols,
   } else {
     for (; i < e; i += LPR)
       acc.add(ld_elem<R, NCA>(vals, i),
-              CG ? ld_elem_cg<R, NCV>(v, __ldg(cols + i)) : ld_elem<R, NCV>(v, __ldg(cols + i)));
+              amplitude<R, NCV, CG>(v, __ldg(cols + i)));
   }
 }
 

@@ -141,10 +141,28 @@ __device__ __forceinline__ Cx<R> cx_make(R a, R b) {
   return c;
 }
 
-// Vector element load/store: NC = 1 (real) or 2 (interleaved complex).
+// Two complex vectors side by side (NC = 4: re, im of the first, re, im of the second).
+template <typename R>
+struct Cx2 {
+  Cx<R> a, b;
+};
 template <typename R, int NC>
-__device__ __forceinline__ Cx<R> ld_elem(const R* p, int64_t i) {
-  if constexpr (NC == 2) {
+struct ElemOf {
+  using type = Cx<R>;
+};
+template <typename R>
+struct ElemOf<R, 4> {
+  using type = Cx2<R>;
+};
+template <typename R, int NC>
+using Elem = typename ElemOf<R, NC>::type;
+
+// Vector element load/store: NC = 1 (real), 2 (interleaved complex) or 4 (two complex vectors).
+template <typename R, int NC>
+__device__ __forceinline__ Elem<R, NC> ld_elem(const R* p, int64_t i) {
+  if constexpr (NC == 4) {
+    return Cx2<R>{ld_elem<R, 2>(p, 2 * i), ld_elem<R, 2>(p, 2 * i + 1)};
+  } else if constexpr (NC == 2) {
     if constexpr (sizeof(R) == 8) {
       double2 v = __ldg(reinterpret_cast<const double2*>(p) + i);
       return cx_make<R>(v.x, v.y);
@@ -161,7 +179,8 @@ __device__ __forceinline__ Cx<R> ld_elem(const R* p, int64_t i) {
 // Load through L2 only (ld.global.cg): for data written earlier in the same kernel launch by
 // other thread blocks, which a non-coherent L1 copy could shadow.
 template <typename R, int NC>
-__device__ __forceinline__ Cx<R> ld_elem_cg(const R* p, int64_t i) {
+__device__ __forceinline__ Elem<R, NC> ld_elem_cg(const R* p, int64_t i) {
+  static_assert(NC <= 2, "one vector");
   if constexpr (NC == 2) {
     if constexpr (sizeof(R) == 8) {
       const double2 v = __ldcg(reinterpret_cast<const double2*>(p) + i);
@@ -200,6 +219,23 @@ __device__ __forceinline__ void st_elem(R* p, int64_t i, Cx<R> v) {
     }
   } else {
     p[i] = v.re;
+  }
+}
+
+// Zero, and the element or zero.
+template <typename R, int NC>
+__device__ __forceinline__ Elem<R, NC> zero_elem() {
+  if constexpr (NC == 4) return Cx2<R>{cx_make<R>(R(0), R(0)), cx_make<R>(R(0), R(0))};
+  else return cx_make<R>(R(0), R(0));
+}
+template <typename R, int NC>
+__device__ __forceinline__ Elem<R, NC> elem_unless(bool gone, Elem<R, NC> v) {
+  if constexpr (NC == 4) {
+    return Cx2<R>{elem_unless<R, 2>(gone, v.a), elem_unless<R, 2>(gone, v.b)};
+  } else {
+    v.re = gone ? R(0) : v.re;
+    if constexpr (NC == 2) v.im = gone ? R(0) : v.im;
+    return v;
   }
 }
 

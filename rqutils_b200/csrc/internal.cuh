@@ -297,6 +297,13 @@ __device__ __forceinline__ uint32_t filter_bit(uint64_t key, int log2) {
 // Build helpers implemented in operator.cu and matvec.cu.
 void op_build(sqd_op_s* op, cudaStream_t st);
 void op_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st);
+// Hv of two FP64 vectors (nc = 1: real, 2: complex) in one pass over the cached elements; scratch
+// of op_pair_scratch() doubles, 0 where two matvecs are the better way.
+size_t op_pair_scratch(const sqd_op_s* op, int nc);
+void op_matvec_pair(sqd_op_s* op, const void* v0, void* out0, const void* v1, void* out1, int nc,
+                    double* scratch, cudaStream_t st);
+void op_product_matvec_pair(sqd_op_s* op, const double* v, double* out, double* scratch,
+                            cudaStream_t st);
 void op_ensure_values32(sqd_op_s* op, cudaStream_t st);
 // Product layout (product.cu).
 bool op_product_detect(sqd_op_s* op, cudaStream_t st, int64_t* nh, int64_t* nl);

@@ -1455,6 +1455,34 @@ class Locg {
     if (rc != SQD_OK) throw Error(rc, std::string("matvec callback failed: ") + last_msg());
   }
 
+  // A y and A p of the reference iteration: one pass over an operator's cached elements for both
+  // where that pays (set_pair_op), else two matvecs.
+  void matvec2(const void* in0, void* out0, const void* in1, void* out1) {
+    if constexpr (sizeof(R) == 8) {
+      if (pair_.ptr) {
+        op_matvec_pair(pair_op_, in0, out0, in1, out1, NC, pair_.ptr, cur_);
+        return;
+      }
+    }
+    matvec(in0, out0);
+    matvec(in1, out1);
+  }
+
+  // Scratch for matvec2; without memory for it, or where it does not pay, two matvecs.
+  void set_pair_op(sqd_op_s* op) {
+    pair_op_ = op;
+    const size_t want = op ? op_pair_scratch(op, NC) : 0;
+    if (want == pair_.count) return;
+    pair_.release();
+    if (want == 0) return;
+    try {
+      pair_.alloc(want, st_);
+    } catch (const Error& e) {
+      if (e.status != SQD_ERR_MEMORY) throw;
+      (void)cudaGetLastError();
+    }
+  }
+
   void read_host() {
     SQD_CUDA(cudaMemcpyAsync(host_, dev_.ptr, sizeof(LocgDev), cudaMemcpyDeviceToHost, st_));
     SQD_CUDA(cudaStreamSynchronize(st_));
@@ -1496,9 +1524,9 @@ class Locg {
       SQD_CUDA(cudaMemsetAsync(y_.ptr, 0, sizeof(R) * NC * n_, st_));
       return;
     }
-    // body_iter1 (:293-322)
+    // body_iter1 (:293-322); A x is still body_iter0's unless that was projected
     lc({r_.ptr}, {p_.ptr}, {}, P_NONE);
-    matvec(x, ax_.ptr);
+    if (!orth.empty()) matvec(x, ax_.ptr);
     matvec(p_.ptr, ap_.ptr);
     lc({x, p_.ptr, ax_.ptr, ap_.ptr}, {}, {{0, 2}, {1, 2}, {1, 3}}, P_RR2);
     lc({x, p_.ptr}, {t0_.ptr, ay_.ptr}, {{100, 100}, {101, 101}}, P_TU_NORM);  // t, u
@@ -1521,10 +1549,9 @@ class Locg {
     lc({p, x, y}, {p}, {{1, 100}, {2, 100}}, P_PROJ_IPS, g);
     lc({p, x, y}, {p}, {{100, 100}}, P_PROJ_MASK, g);
     lc({p}, {p}, {}, P_NONE, g | G_KEEP);
-    // Rayleigh-Ritz on {x, y, p}
-    matvec(x, ax_.ptr);
-    matvec(y, ay_.ptr);
-    matvec(p, ap_.ptr);
+    // Rayleigh-Ritz on {x, y, p}.  The reference applies A to x again here; x has not changed
+    // since the residual was formed from A x, which ax still holds.
+    matvec2(y, ay_.ptr, p, ap_.ptr);
     lc({x, y, p, ax_.ptr, ay_.ptr, ap_.ptr}, {}, {{0, 3}, {1, 4}, {2, 5}, {1, 3}, {2, 3}, {2, 4}},
        P_RR3, g);
     // s = k1 y + k2 p (virtual), |s|
@@ -1875,6 +1902,8 @@ class Locg {
   int hist_cap_ = 0;
   int hist_phase_ = 0;
   sqd_op_s* persist_op_ = nullptr;
+  sqd_op_s* pair_op_ = nullptr;
+  DevBuf<double> pair_;       // scratch of matvec2
   unsigned persist_grid_ = 0;
   bool persist_cluster_ = false;
   DevBuf<double> ppart_;
@@ -1998,6 +2027,7 @@ void run_locg(int64_t n, int dtype, sqd_matvec_fn fn, void* ctx, sqd_op_s* cache
       own = std::make_unique<Locg<double, NC>>(n, fn, ctx, st);
       lp = own.get();
     }
+    lp->set_pair_op(cache_op);
     Locg<double, NC>& L = *lp;
     HistRecorder rec{g_hist_request};
     g_hist_request = HistRequest{};

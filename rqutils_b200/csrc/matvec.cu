@@ -39,7 +39,7 @@ k_mv_csr(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ cols,
       csr_row_dot<R, NCV, NCA, LPR>(cols, vals, v, b + sub, e, acc);
     }
     acc.merge(LPR);
-    if (sub == 0 && row < lim) st_elem<R, NCV>(out, row, cx_make<R>(acc.re.value(), acc.im.value()));
+    if (sub == 0 && row < lim) acc.store(out, row);
   };
   if (chunk <= 0) {
     // Interleaved: consecutive warps of the grid take consecutive row groups.
@@ -211,6 +211,32 @@ __global__ void k_fill_tail(const R* v, R* out, int64_t n_unique, int64_t size,
   st_elem<R, NCV>(out, size - 1, o);
 }
 
+// Two vectors into one of interleaved elements (E: a real or complex element), and back.
+template <typename E>
+__global__ void k_interleave(const E* __restrict__ a, const E* __restrict__ b, E* __restrict__ out,
+                             int64_t n) {
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    out[2 * i] = a[i];
+    out[2 * i + 1] = b[i];
+  }
+}
+template <typename E>
+__global__ void k_deinterleave(const E* __restrict__ in, E* __restrict__ a, E* __restrict__ b,
+                               int64_t n) {
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    a[i] = in[2 * i];
+    b[i] = in[2 * i + 1];
+  }
+}
+
+// From where the pair list is read for two vectors at once (op_pair_scratch).  FP64 iteration at
+// 32 qubits, pair / two matvecs: 100 x 98 strings (56 pairs a row) 76.8 / 75.1 us, 180 x 170 (107 a
+// row) 96.2 / 96.4, 448 x 400 (339 a row) 511 / about 640; 200,000 states with one pair a row
+// 142.0 / 138.8.
+constexpr int64_t kPairMinRows = 16384, kPairMinPerRow = 16;
+
 unsigned mv_grid(int64_t rows, int lpr) {
   const int64_t warps = (rows * lpr + 31) / 32;
   const int64_t blocks = (warps + 7) / 8;
@@ -290,6 +316,64 @@ void op_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t s
       }
     }
   });
+}
+
+// Two FP64 vectors share one pass over the elements.  Interleaving them costs four reads and
+// writes of each vector, so it pays where a row has many more pairs than that.  Real vectors
+// become one complex vector over the same (real) elements; every component is summed as it is
+// alone, so the results are bit-identical to two matvecs.
+size_t op_pair_scratch(const sqd_op_s* op, int nc) {
+  if (op->x_cache != 1 || op->z_cache != 2) return 0;
+  const int64_t n = op->s->states_size;
+  // The product layouts' five launches per matvec make the pair the better way at every size
+  // (100 x 98 strings 120 / 136 us an iteration).
+  const bool product = op->prod.built && op->layout[0] != SQD_LAYOUT_CSR;
+  if (!product && (n < kPairMinRows || op->nnz < kPairMinPerRow * n)) return 0;
+  return static_cast<size_t>(n) * nc * 4 + (product && nc == 2 ? static_cast<size_t>(n) * 12 : 0);
+}
+
+void op_matvec_pair(sqd_op_s* op, const void* v0, void* out0, const void* v1, void* out1, int nc,
+                    double* scratch, cudaStream_t st) {
+  const int64_t n = op->s->states_size;
+  double* in = scratch;
+  double* out = scratch + n * nc * 2;
+  double* rest = scratch + n * nc * 4;
+  const unsigned G = grid_for(n, 256, num_sms() * 16);
+  if (nc == 1)
+    k_interleave<double><<<G, 256, 0, st>>>(static_cast<const double*>(v0),
+                                            static_cast<const double*>(v1), in, n);
+  else
+    k_interleave<double2><<<G, 256, 0, st>>>(static_cast<const double2*>(v0),
+                                             static_cast<const double2*>(v1),
+                                             reinterpret_cast<double2*>(in), n);
+  SQD_CHECK_LAUNCH();
+  if (nc == 1) {
+    op_matvec(op, in, out, SQD_C128, st);
+  } else if (op->prod.built && op->layout[0] != SQD_LAYOUT_CSR) {
+    op_product_matvec_pair(op, in, out, rest, st);
+  } else {
+    dispatch_lpr(op->lanes_per_row[0], [&](auto lpr_t) {
+      constexpr int LPR = decltype(lpr_t)::value;
+      const unsigned GM = mv_grid(n, LPR);
+      if (op->value_complex)
+        k_mv_csr<double, 4, 2, LPR><<<GM, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr,
+                                                        op->values.ptr, in, out, n,
+                                                        op->chunk_rows[0]);
+      else
+        k_mv_csr<double, 4, 1, LPR><<<GM, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr,
+                                                        op->values.ptr, in, out, n,
+                                                        op->chunk_rows[0]);
+      SQD_CHECK_LAUNCH();
+    });
+  }
+  if (nc == 1)
+    k_deinterleave<double><<<G, 256, 0, st>>>(out, static_cast<double*>(out0),
+                                              static_cast<double*>(out1), n);
+  else
+    k_deinterleave<double2><<<G, 256, 0, st>>>(reinterpret_cast<const double2*>(out),
+                                               static_cast<double2*>(out0),
+                                               static_cast<double2*>(out1), n);
+  SQD_CHECK_LAUNCH();
 }
 
 }  // namespace sqd

@@ -73,6 +73,25 @@ __global__ void k_to_float32(const double* __restrict__ in, float* __restrict__ 
     out[i] = static_cast<float>(in[i]);
 }
 
+// A vector element as it is copied.
+template <typename R, int NC>
+struct RawOf {
+  using type = std::conditional_t<sizeof(R) == 8, double2, float2>;
+};
+template <typename R>
+struct RawOf<R, 1> {
+  using type = R;
+};
+struct __align__(16) Double4 {
+  double2 a, b;
+};
+template <typename R>
+struct RawOf<R, 4> {
+  using type = Double4;
+};
+template <typename R, int NC>
+using Raw = typename RawOf<R, NC>::type;
+
 // out[c][r] = in[r][c] for an rows x cols matrix of elements E (32 x 32 tiles, 256 threads).
 template <typename E>
 __global__ void __launch_bounds__(256)
@@ -114,7 +133,8 @@ k_slab(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* __
   // 2 KB ahead is prefetched into L2, one 128-byte line per lane, so the element loads wait on
   // L2 rather than on DRAM (measured: C3 FP64 matvec 5.9 -> 5.1 ms, C2 0.370 -> 0.324 ms; 4 KB
   // ahead was slightly slower, 8 KB no better than none).
-  constexpr int kChunkLines = 8 * 32 * NCA * static_cast<int>(sizeof(R)) / 128;
+  constexpr int U = NCV == 4 ? 4 : 8;   // entries per step; four when an amplitude is 32 bytes
+  constexpr int kChunkLines = U * 32 * NCA * static_cast<int>(sizeof(R)) / 128;
   constexpr int pv = kChunkLines >= 16 ? 1 : 16 / kChunkLines;   // steps ahead
   for (int64_t blk = blockIdx.x; blk < panels * a_tiles; blk += gridDim.x) {
     const int64_t p = blk / a_tiles;
@@ -129,24 +149,26 @@ k_slab(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* __
     const int64_t k1 = __ldg(off + a + 1);
     int64_t k = __ldg(off + a);
     const R* vp = V + ((p * total_k + k) * 32 + lane) * NCA;
-    for (; k + 7 < k1; k += 8) {
+    for (; k + U - 1 < k1; k += U) {
       // prefetch: the next step's source offsets (one 32-byte sector) into L1 ahead of use
-      if (prefetch && k + 15 < k1) asm volatile("prefetch.global.L1 [%0];" ::"l"(src + k + 8));
-      if (lane < kChunkLines && k + 8 * pv + 7 < k1)
+      if (prefetch && k + 2 * U - 1 < k1)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(src + k + U));
+      if (lane < kChunkLines && k + U * pv + U - 1 < k1)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(
-            reinterpret_cast<const char*>(vp - lane * NCA + 8 * 32 * NCA * pv) + lane * 128));
-      uint32_t si[8];
+            reinterpret_cast<const char*>(vp - lane * NCA + U * 32 * NCA * pv) + lane * 128));
+      uint32_t si[U];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) si[u] = __ldg(src + k + u);
-      Cx<R> m[8], xv[8];
+      for (int u = 0; u < U; ++u) si[u] = __ldg(src + k + u);
+      Cx<R> m[U];
+      Elem<R, NCV> xv[U];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < U; ++u) {
         m[u] = ld_elem<R, NCA>(vp, 32 * u);
         xv[u] = ld_elem<R, NCV>(x, int64_t(si[u]) + b);
       }
-      acc.add4(m, xv);
-      acc.add4(m + 4, xv + 4);
-      vp += 8 * 32 * NCA;
+#pragma unroll
+      for (int u = 0; u < U; u += 4) acc.add4(m + u, xv + u);
+      vp += U * 32 * NCA;
     }
     // remainder: one entry at a time (a predicated eight-entry step measured 5-11 % slower
     // for FP64 at 32 and 48 qubits)
@@ -154,7 +176,7 @@ k_slab(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* __
       acc.add(ld_elem<R, NCA>(vp, 0), ld_elem<R, NCV>(x, int64_t(__ldg(src + k)) + b));
       vp += 32 * NCA;
     }
-    if constexpr (FINAL) st_elem<R, NCV>(out, a * B + b, cx_make<R>(acc.re.value(), acc.im.value()));
+    if constexpr (FINAL) acc.store(out, a * B + b);
     else acc.store_partial(out_part, a * B + b);
   }
 }
@@ -428,8 +450,10 @@ __device__ __forceinline__ void copy_async(void* smem, const void* global) {
 }
 
 template <typename R, int NC>
-__device__ __forceinline__ Cx<R> sm_elem(const R* p, int64_t i) {
-  if constexpr (NC == 2) {
+__device__ __forceinline__ Elem<R, NC> sm_elem(const R* p, int64_t i) {
+  if constexpr (NC == 4) {
+    return Cx2<R>{sm_elem<R, 2>(p, 2 * i), sm_elem<R, 2>(p, 2 * i + 1)};
+  } else if constexpr (NC == 2) {
     if constexpr (sizeof(R) == 8) {
       const double2 d = reinterpret_cast<const double2*>(p)[i];
       return cx_make<R>(d.x, d.y);
@@ -454,7 +478,8 @@ constexpr int kPanelGroup = 4;
 constexpr int kPanelAhead = 6;
 
 template <typename R, int NCV, int NCA, int P, bool STAGED, bool FULL>
-__global__ void __launch_bounds__(P < kPanelMaxPerWarp ? 256 : 1024, P < kPanelMaxPerWarp ? 6 : 1)
+__global__ void __launch_bounds__(P < kPanelMaxPerWarp ? 256 : 1024,
+                                  P == kPanelMaxPerWarp ? 1 : NCV == 4 ? 4 : 6)
 k_tail_panels(PlanView c, const int32_t* __restrict__ at, const uint32_t* __restrict__ perm,
               const uint16_t* __restrict__ src, const uint32_t* __restrict__ horder, int panels,
               int steps, int chunks, int group, const R* __restrict__ vm, const R* __restrict__ v, double* __restrict__ part) {
@@ -480,8 +505,9 @@ k_tail_panels(PlanView c, const int32_t* __restrict__ at, const uint32_t* __rest
         const char* from = reinterpret_cast<const char*>(v) +
                            int64_t(__ldg(part_h + kb + u)) * c.nl * EB;
         char* to = reinterpret_cast<char*>(rows + u * row);
-        for (int i = threadIdx.x; i < nl; i += blockDim.x)
-          copy_async<EB>(to + i * EB, from + int64_t(i) * EB);
+        constexpr int CB = EB < 16 ? EB : 16;
+        for (int i = threadIdx.x; i < nl * (EB / CB); i += blockDim.x)
+          copy_async<CB>(to + i * CB, from + int64_t(i) * CB);
         if (threadIdx.x < NCV) rows[u * row + nl * NCV + threadIdx.x] = R(0);   // padding's source
       }
       asm volatile("cp.async.commit_group;");
@@ -518,7 +544,8 @@ k_tail_panels(PlanView c, const int32_t* __restrict__ at, const uint32_t* __rest
             asm volatile("prefetch.global.L2 [%0];" ::"l"(ahead + (t + kPanelAhead) * 32 * NCA));
           int s = __ldg(sp + t * 32);
           if constexpr (!STAGED) s = min(s, nl - 1);
-          Cx<R> el[kPanelGroup], xv[kPanelGroup];
+          Cx<R> el[kPanelGroup];
+          Elem<R, NCV> xv[kPanelGroup];
 #pragma unroll
           for (int u = 0; u < KN; ++u) el[u] = ld_elem<R, NCA>(vp + u * stride, t * 32);
 #pragma unroll
@@ -529,11 +556,13 @@ k_tail_panels(PlanView c, const int32_t* __restrict__ at, const uint32_t* __rest
             if constexpr (FULL) break;
             const bool gone = is_absent(el[u].re);
             el[u].re = gone ? R(0) : el[u].re;
-            xv[u].re = gone ? R(0) : xv[u].re;
-            if constexpr (NCV == 2) xv[u].im = gone ? R(0) : xv[u].im;
+            xv[u] = elem_unless<R, NCV>(gone, xv[u]);
           }
 #pragma unroll
-          for (int u = KN; u < kPanelGroup; ++u) el[u] = xv[u] = cx_make<R>(R(0), R(0));
+          for (int u = KN; u < kPanelGroup; ++u) {
+            el[u] = cx_make<R>(R(0), R(0));
+            xv[u] = zero_elem<R, NCV>();
+          }
           acc[i].add4(el, xv);
         }
       };
@@ -703,7 +732,7 @@ void build_panels(sqd_op_s* op, cudaStream_t st) {
   });
   // Rows too long to stage have no zero behind them for the padding.
   L.panel_full = L.pairs_m == q.ta * q.tb &&
-                 panel_row(L.nl, 16) <= static_cast<int64_t>(kPanelSmem);
+                 panel_row(L.nl, 32) <= static_cast<int64_t>(kPanelSmem);
   const int64_t panels = (L.nl + 31) / 32;
   std::vector<int32_t> at(static_cast<size_t>(panels) + 1, 0);
   int64_t steps = 0;
@@ -817,7 +846,7 @@ void ensure_floats(sqd_op_s* op, cudaStream_t st) {
 }
 
 template <typename R, int NCV, int NCA>
-bool launch_panels(sqd_op_s* op, const R* vin, cudaStream_t st) {
+bool launch_panels(sqd_op_s* op, const R* vin, double* part, cudaStream_t st) {
   ProductLayout& L = op->prod;
   if (L.panel_state != 1) return false;
   const R* vm;
@@ -853,7 +882,7 @@ bool launch_panels(sqd_op_s* op, const R* vin, cudaStream_t st) {
     kern<<<G, static_cast<unsigned>(warps * 32), dyn, st>>>(
         plan_view(*op->plan), L.panel_at.ptr, L.perm.ptr, L.panel_src.ptr, L.horder.ptr,
         static_cast<int>(L.panels), static_cast<int>(L.steps), static_cast<int>(chunks), group, vm,
-        vin, L.t.ptr);
+        vin, part);
     SQD_CHECK_LAUNCH();
   };
   auto pick = [&](auto p) {
@@ -951,80 +980,102 @@ void op_product_values32(sqd_op_s* op, cudaStream_t st) {
   if (op->prod.built) ensure_floats(op, st);
 }
 
+namespace {
+
+// Scratch of one product matvec: FP64 values per row and vector component.
+struct ProductScratch {
+  double *vt, *tt, *t;
+};
+
+template <typename R, int NCV, int NCA>
+void product_matvec(sqd_op_s* op, const R* vin, R* vout, const ProductScratch& w,
+                    cudaStream_t st) {
+  ProductLayout& L = op->prod;
+  const int64_t nh = L.nh, nl = L.nl, n = nh * nl;
+  const int prec = sizeof(R) == 8 ? 0 : 1;
+  using E = Raw<R, NCV>;
+  using ED = Raw<double, NCV>;
+  const R* VH;
+  const R* VL;
+  const R* VC;
+  if constexpr (sizeof(R) == 8) {
+    VH = L.vh.ptr;
+    VL = L.vl.ptr;
+    VC = op->values.ptr;
+  } else {
+    VH = L.vh32.ptr;
+    VL = L.vl32.ptr;
+    VC = op->values32.ptr;
+  }
+  R* vt = reinterpret_cast<R*>(w.vt);
+  // FP32 slabs in 64-wide panels (both halves even): paired accesses to the library's own
+  // buffers always, to v and Hv when their addresses allow
+  const bool wide = sizeof(R) == 4 && L.wide32;
+  const uintptr_t pair_bytes = 2 * NCV * sizeof(R);
+  const bool vec_io = reinterpret_cast<uintptr_t>(vin) % pair_bytes == 0 &&
+                      reinterpret_cast<uintptr_t>(vout) % pair_bytes == 0;
+  // 1. vT[l][h] = v[h][l]
+  launch_transpose<E>(vin, vt, nh, nl, st);
+  // 2. L part: t2[l][h]
+  launch_slab<R, NCV, NCA, false, false>(nl, nh, L.tl, L.lo.ptr, L.lsrc.ptr, VL, vt, nullptr,
+                                         nullptr, nullptr, w.tt, st, wide, true);
+  // 3. t2 back in row order, into the vT buffer
+  launch_transpose<ED>(w.tt, w.vt, nl, nh, st);
+  // 4. M part: t3[r]
+  if (L.pairs_m > 0) {
+    if (op->layout[prec] == SQD_LAYOUT_PRODUCT_CSR ||
+        !launch_panels<R, NCV, NCA>(op, vin, w.t, st)) {
+      const R* MV = nullptr;  // the short-tail copy's elements, when it exists
+      if (L.tail_state == 1) {
+        if constexpr (sizeof(R) == 8) MV = L.mval.ptr;
+        else MV = L.mval32.ptr;
+      }
+      // lanes from the mean tail length unless the caller chose them (48 qubits, 3072 x 2816
+      // strings: 5.6 pairs a tail, 1.87 ms with the whole row's 32 lanes)
+      const int lanes = op->lanes_chosen[prec] ? op->lanes_per_row[prec]
+                                               : lanes_for(double(L.pairs_m) / double(n));
+      dispatch_lpr(lanes, [&](auto lpr_t) {
+        constexpr int LPR = decltype(lpr_t)::value;
+        if (MV != nullptr)
+          k_mv_mixed<R, NCV, NCA, LPR, true><<<mixed_grid(n, LPR), 256, 0, st>>>(
+              L.mptr.ptr, L.mcol.ptr, MV, vin, nullptr, nullptr, nl, w.t, n,
+              op->chunk_rows[prec]);
+        else
+          k_mv_mixed<R, NCV, NCA, LPR, false><<<mixed_grid(n, LPR), 256, 0, st>>>(
+              op->row_ptr.ptr, op->cols.ptr, VC, vin, L.ho.ptr, L.lo.ptr, nl, w.t, n,
+              op->chunk_rows[prec]);
+        SQD_CHECK_LAUNCH();
+      });
+    }
+    // 5. H part plus both partials
+    launch_slab<R, NCV, NCA, true, true>(nh, nl, L.th, L.ho.ptr, L.hsrc.ptr, VH, vin, w.vt, w.t,
+                                         vout, nullptr, st, wide, vec_io);
+  } else {
+    launch_slab<R, NCV, NCA, true, false>(nh, nl, L.th, L.ho.ptr, L.hsrc.ptr, VH, vin, w.vt,
+                                          nullptr, vout, nullptr, st, wide, vec_io);
+  }
+}
+
+}  // namespace
+
 void op_product_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st) {
   ProductLayout& L = op->prod;
-  const bool dbl = dtype_is_double(dtype);
-  SQD_REQUIRE(dbl || L.vh32.ptr != nullptr, "FP32 product-layout elements were not prepared");
-  const int64_t nh = L.nh, nl = L.nl, n = nh * nl;
-  const int prec = dbl ? 0 : 1;
+  SQD_REQUIRE(dtype_is_double(dtype) || L.vh32.ptr != nullptr,
+              "FP32 product-layout elements were not prepared");
+  const ProductScratch w{L.vt.ptr, L.tt.ptr, L.t.ptr};
   dispatch_vec(dtype, op->value_complex, [&](auto rt, auto ncv_t, auto nca_t) {
     using R = typename decltype(rt)::type;
-    constexpr int NCV = decltype(ncv_t)::value;
-    constexpr int NCA = decltype(nca_t)::value;
-    using E = std::conditional_t<NCV == 2, std::conditional_t<sizeof(R) == 8, double2, float2>, R>;
-    using ED = std::conditional_t<NCV == 2, double2, double>;
-    const R* vin = static_cast<const R*>(v);
-    R* vout = static_cast<R*>(out);
-    const R* VH;
-    const R* VL;
-    const R* VC;
-    if constexpr (sizeof(R) == 8) {
-      VH = L.vh.ptr;
-      VL = L.vl.ptr;
-      VC = op->values.ptr;
-    } else {
-      VH = L.vh32.ptr;
-      VL = L.vl32.ptr;
-      VC = op->values32.ptr;
-    }
-    R* vt = reinterpret_cast<R*>(L.vt.ptr);
-    // FP32 slabs in 64-wide panels (both halves even): paired accesses to the library's own
-    // buffers always, to v and Hv when their addresses allow
-    const bool wide = sizeof(R) == 4 && L.wide32;
-    const uintptr_t pair_bytes = 2 * NCV * sizeof(R);
-    const bool vec_io = reinterpret_cast<uintptr_t>(vin) % pair_bytes == 0 &&
-                        reinterpret_cast<uintptr_t>(vout) % pair_bytes == 0;
-    // 1. vT[l][h] = v[h][l]
-    launch_transpose<E>(vin, vt, nh, nl, st);
-    // 2. L part: t2[l][h]
-    launch_slab<R, NCV, NCA, false, false>(nl, nh, L.tl, L.lo.ptr, L.lsrc.ptr, VL, vt, nullptr,
-                                           nullptr, nullptr, L.tt.ptr, st, wide, true);
-    // 3. t2 back in row order, into the vT buffer
-    launch_transpose<ED>(L.tt.ptr, L.vt.ptr, nl, nh, st);
-    // 4. M part: t3[r]
-    if (L.pairs_m > 0) {
-      if (op->layout[prec] == SQD_LAYOUT_PRODUCT_CSR ||
-          !launch_panels<R, NCV, NCA>(op, vin, st)) {
-        const R* MV = nullptr;  // the short-tail copy's elements, when it exists
-        if (L.tail_state == 1) {
-          if constexpr (sizeof(R) == 8) MV = L.mval.ptr;
-          else MV = L.mval32.ptr;
-        }
-        // lanes from the mean tail length unless the caller chose them (48 qubits, 3072 x 2816
-        // strings: 5.6 pairs a tail, 1.87 ms with the whole row's 32 lanes)
-        const int lanes = op->lanes_chosen[prec] ? op->lanes_per_row[prec]
-                                                 : lanes_for(double(L.pairs_m) / double(n));
-        dispatch_lpr(lanes, [&](auto lpr_t) {
-          constexpr int LPR = decltype(lpr_t)::value;
-          if (MV != nullptr)
-            k_mv_mixed<R, NCV, NCA, LPR, true><<<mixed_grid(n, LPR), 256, 0, st>>>(
-                L.mptr.ptr, L.mcol.ptr, MV, vin, nullptr, nullptr, nl, L.t.ptr, n,
-                op->chunk_rows[prec]);
-          else
-            k_mv_mixed<R, NCV, NCA, LPR, false><<<mixed_grid(n, LPR), 256, 0, st>>>(
-                op->row_ptr.ptr, op->cols.ptr, VC, vin, L.ho.ptr, L.lo.ptr, nl, L.t.ptr, n,
-                op->chunk_rows[prec]);
-          SQD_CHECK_LAUNCH();
-        });
-      }
-      // 5. H part plus both partials
-      launch_slab<R, NCV, NCA, true, true>(nh, nl, L.th, L.ho.ptr, L.hsrc.ptr, VH, vin, L.vt.ptr,
-                                           L.t.ptr, vout, nullptr, st, wide, vec_io);
-    } else {
-      launch_slab<R, NCV, NCA, true, false>(nh, nl, L.th, L.ho.ptr, L.hsrc.ptr, VH, vin,
-                                            L.vt.ptr, nullptr, vout, nullptr, st, wide, vec_io);
-    }
+    product_matvec<R, decltype(ncv_t)::value, decltype(nca_t)::value>(
+        op, static_cast<const R*>(v), static_cast<R*>(out), w, st);
   });
+}
+
+void op_product_matvec_pair(sqd_op_s* op, const double* v, double* out, double* scratch,
+                            cudaStream_t st) {
+  const int64_t n = op->prod.nh * op->prod.nl;
+  const ProductScratch w{scratch, scratch + 4 * n, scratch + 8 * n};
+  if (op->value_complex) product_matvec<double, 4, 2>(op, v, out, w, st);
+  else product_matvec<double, 4, 1>(op, v, out, w, st);
 }
 
 }  // namespace sqd
