@@ -134,6 +134,10 @@ struct ProductPlan {
   sqd::DevBuf<int32_t> mtable;        // [na * nb] group of (a, b) or -1 (dense form)
   sqd::DevBuf<uint64_t> xa, xb, xm;   // distinct parts; two-half masks, ascending (sparse form)
   sqd::DevBuf<int32_t> gm;            // [nm] groups of xm
+  // The lists' entries by (class, key), for sums per group (grad.cu, on first use): key and
+  // (string, partner); classes H, L, A, B one after the other.
+  sqd::DevBuf<uint32_t> gkey;
+  sqd::DevBuf<uint2> gpair;
 };
 
 // Solver objects an operator keeps between LOCG solves (locg.cu): work vectors and the

@@ -1,5 +1,4 @@
-// The projected operator: connectivity cache, matrix elements, diagonals, vinit, CSR export and
-// the Hellmann-Feynman per-term reduction.
+// The projected operator: connectivity cache, matrix elements, diagonals, vinit and CSR export.
 //
 // Connectivity (cache_strategy x = 1) is the sparse form of the reference's xsources cache
 // (run_sqd, sqd.py:343-351): instead of a dense J x N int32 array with -1 for missing sources,
@@ -224,98 +223,6 @@ __global__ void k_cols_to_i32(const uint32_t* cols, int32_t* out, int64_t n) {
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * blockDim.x)
     out[i] = static_cast<int32_t>(cols[i]);
-}
-
-// ---------------------------------------------------------------------------------------------
-// Hellmann-Feynman per-term reduction  g_t = Re sum_i conj(u_i) ph_t (-1)^{|s_i & z_t|} v_src.
-// ---------------------------------------------------------------------------------------------
-constexpr int GR_TILE = 1024;
-
-// Diagonal group (x = 0, src = i): per block, w_i = conj(u_i) v_i for a tile of rows in shared
-// memory, then one block-wide reduction per term and one atomicAdd per (block, term).
-template <int NCV>
-__global__ void k_grad_diag(const uint64_t* states, int64_t n_unique, const int64_t* gs,
-                            const int32_t* ge, const uint64_t* tz, const double* tc,
-                            const double* u, const double* v, double* g) {
-  __shared__ uint64_t s_st[GR_TILE];
-  __shared__ double s_wr[GR_TILE], s_wi[GR_TILE];
-  __shared__ double red[32];
-  const int64_t r0 = static_cast<int64_t>(blockIdx.x) * GR_TILE;
-  for (int k = threadIdx.x; k < GR_TILE; k += blockDim.x) {
-    const int64_t r = r0 + k;
-    double wr = 0.0, wi = 0.0;
-    uint64_t s = 0;
-    if (r < n_unique) {
-      s = states[r];
-      const Cx<double> a = ld_elem<double, NCV>(u, r), b = ld_elem<double, NCV>(v, r);
-      wr = a.re * b.re + a.im * b.im;
-      wi = a.re * b.im - a.im * b.re;
-    }
-    s_st[k] = s;
-    s_wr[k] = wr;
-    s_wi[k] = wi;
-  }
-  __syncthreads();
-  const int64_t b = gs[0];
-  const int32_t K = ge[0];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  // x = 0: the phase is 1 and Re((-1)^{|s & z|} w) = (-1)^{|s & z|} Re w.
-  for (int32_t t = 0; t < K; ++t) {
-    const uint64_t z = tz[b + t];
-    double ar = 0.0;
-    for (int k = threadIdx.x; k < GR_TILE; k += blockDim.x)
-      ar += parity64(s_st[k] & z) ? -s_wr[k] : s_wr[k];
-    ar = warp_sum(ar);
-    if (lane == 0) red[warp] = ar;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double sr = 0.0;
-      for (int w = 0; w < nwarp; ++w) sr += red[w];
-      atomicAdd(g + b + t, sr);
-    }
-    __syncthreads();
-  }
-}
-
-// Off-diagonal stored pairs: per pair, loop over the group's terms and atomically add.
-template <int NCV>
-__global__ void k_grad_offdiag(const int64_t* row_ptr, const uint32_t* cols,
-                               const uint32_t* grps, const uint64_t* states, int64_t n_unique,
-                               int has_diag, const int64_t* gs, const int32_t* ge,
-                               const uint64_t* gx, const uint64_t* tz, const double* u,
-                               const double* v, double* g) {
-  const int lane = threadIdx.x & 31;
-  const int64_t w0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t r = w0; r < n_unique; r += nw) {
-    const uint64_t s = states[r];
-    const Cx<double> a = ld_elem<double, NCV>(u, r);
-    const int64_t b = row_ptr[r] + has_diag, e = row_ptr[r + 1];
-    for (int64_t i = b + lane; i < e; i += 32) {
-      const int64_t j = grps[i];
-      const Cx<double> x = ld_elem<double, NCV>(v, cols[i]);
-      // w = conj(u_r) v_src
-      const double wr = a.re * x.re + a.im * x.im;
-      const double wi = a.re * x.im - a.im * x.re;
-      const uint64_t xm = gx[j];
-      const int64_t tb = gs[j];
-      const int32_t K = ge[j];
-      for (int32_t t = 0; t < K; ++t) {
-        const uint64_t z = tz[tb + t];
-        const int ph = __popcll(xm & z) & 3;
-        // Re((-i)^ph * w)
-        double val;
-        switch (ph) {
-          case 0: val = wr; break;
-          case 1: val = wi; break;
-          case 2: val = -wr; break;
-          default: val = -wi; break;
-        }
-        if (parity64(s & z)) val = -val;
-        atomicAdd(g + tb + t, val);
-      }
-    }
-  }
 }
 
 }  // namespace
@@ -703,48 +610,6 @@ extern "C" int sqd_op_refresh(sqd_op_t op, void* stream) {
     }
     op_product_refresh(op, st);
     ++op->schedule_version;
-  });
-}
-
-extern "C" int sqd_grad_terms(sqd_op_t op, const void* u, const void* v, int dtype,
-                              double* out_terms, void* stream) {
-  return guarded([&] {
-    SQD_REQUIRE(op != nullptr && u && v && out_terms, "NULL argument");
-    SQD_REQUIRE(op->x_cache == 1, "the coefficient gradient needs cache_strategy x = 1");
-    SQD_REQUIRE(op->nnz == 0 || op->grps.ptr != nullptr,
-                "the operator released its group indices; create a new operator");
-    SQD_REQUIRE(dtype == SQD_F64 || dtype == SQD_C128, "gradient dtype must be F64 or C128");
-    SQD_REQUIRE(dtype == SQD_C128 || !op->value_complex, "complex Hamiltonian needs C128");
-    sqd_paulis_s* p = op->p;
-    sqd_space_s* sp = op->s;
-    cudaStream_t st = as_stream(stream);
-    SQD_CUDA(cudaMemsetAsync(out_terms, 0, p->num_terms * sizeof(double), st));
-    const double* ud = static_cast<const double*>(u);
-    const double* vd = static_cast<const double*>(v);
-    if (op->has_diag_group && sp->n_unique > 0) {
-      const unsigned G = grid_for(sp->n_unique, GR_TILE);
-      if (dtype == SQD_C128)
-        k_grad_diag<2><<<G, 256, 0, st>>>(sp->states.ptr, sp->n_unique, p->group_start.ptr,
-                                          p->group_eff.ptr, p->term_z.ptr, p->term_c.ptr, ud, vd,
-                                          out_terms);
-      else
-        k_grad_diag<1><<<G, 256, 0, st>>>(sp->states.ptr, sp->n_unique, p->group_start.ptr,
-                                          p->group_eff.ptr, p->term_z.ptr, p->term_c.ptr, ud, vd,
-                                          out_terms);
-      SQD_CHECK_LAUNCH();
-    }
-    const unsigned G = grid_for(sp->n_unique * 32, 256, 16384);
-    if (dtype == SQD_C128)
-      k_grad_offdiag<2><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->grps.ptr,
-                                           sp->states.ptr, sp->n_unique, op->has_diag_group,
-                                           p->group_start.ptr, p->group_eff.ptr, p->group_x.ptr,
-                                           p->term_z.ptr, ud, vd, out_terms);
-    else
-      k_grad_offdiag<1><<<G, 256, 0, st>>>(op->row_ptr.ptr, op->cols.ptr, op->grps.ptr,
-                                           sp->states.ptr, sp->n_unique, op->has_diag_group,
-                                           p->group_start.ptr, p->group_eff.ptr, p->group_x.ptr,
-                                           p->term_z.ptr, ud, vd, out_terms);
-    SQD_CHECK_LAUNCH();
   });
 }
 
