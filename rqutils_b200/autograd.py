@@ -30,11 +30,9 @@ def _apply_coeffs(op, coeffs):
 
 
 def _scatter_terms(op, g_terms):
+    # a gather, not a masked assignment, which would wait for the mask's count on the host
     r2t = op.hamiltonian.raw_to_term()
-    out = torch.zeros(r2t.shape[0], dtype=torch.float64, device=g_terms.device)
-    ok = r2t >= 0
-    out[ok] = g_terms[r2t[ok]]
-    return out
+    return torch.where(r2t >= 0, g_terms[r2t.clamp(min=0)], g_terms.new_zeros(()))
 
 
 class _Matvec(torch.autograd.Function):
