@@ -90,6 +90,7 @@ struct ProductLayout {
   sqd::DevBuf<float> vh32, vl32;     // FP32 copies (64-wide panels when wide32)
   int wide32 = 0;                    // both halves even: FP32 slabs read two positions per lane
   sqd::DevBuf<double> vt, tt, t;     // per-matvec scratch: transposed input, L and M partials
+  sqd::DevBuf<double> t2;            // H partial (small grids only)
   // Two-half (M) pairs.  Panel form (SQD_LAYOUT_PRODUCT, product.cu k_tail_panels): the low
   // strings sorted by the length of their B list (perm, 0xffffffff in the padding) in panels of
   // 32, panel p with panel_at[p + 1] - panel_at[p] steps; element of A entry k, step t, lane at

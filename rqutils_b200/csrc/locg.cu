@@ -2126,13 +2126,15 @@ void run_locg(int64_t n, int dtype, sqd_matvec_fn fn, void* ctx, sqd_op_s* cache
   L.set_history(rec.rows[0].ptr, static_cast<int>(rec.req.max_rows), 0);
   l32->set_history(rec.rows[1].ptr, static_cast<int>(rec.req.max_rows), 1);
   // Persistent iterations (one cooperative launch per loop) where the matvec is the cached
-  // CSR kernel and the operator is small enough that launch latency, not bandwidth, bounds the
-  // graph form: up to 4 Mi rows and 64 Mi stored pairs (a large matvec runs better as its own
-  // kernel at full occupancy).  SQD_LOCG_PERSISTENT=0 disables, =1 forces.
+  // CSR kernel and launch latency, not the matvec, bounds the graph form: up to 4 Mi rows with at
+  // most 36 stored pairs each on average (a longer matvec runs better as its own kernel at full
+  // occupancy).  Persistent / graph, us per iteration, 32 and 48 qubits: 3,840 rows of 33 pairs 30.4 /
+  // 37.0, 250,000 of 19 75 / 94, 16,380 of 73 48.8 / 36.9, 1.1 M of 39 346 / 234.
+  // SQD_LOCG_PERSISTENT=0 disables, =1 forces.
   {
     const char* env = std::getenv("SQD_LOCG_PERSISTENT");
     const bool on = env ? std::atoi(env) != 0
-                        : n <= (int64_t(4) << 20) && op->nnz <= (int64_t(64) << 20);
+                        : n <= (int64_t(4) << 20) && op->nnz <= 36 * n;
     auto csr = [&](int prec) {
       return op->x_cache == 1 && op->z_cache == 2 &&
              (!op->prod.built || op->layout[prec] == SQD_LAYOUT_CSR);

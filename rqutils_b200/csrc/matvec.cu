@@ -329,7 +329,7 @@ size_t op_pair_scratch(const sqd_op_s* op, int nc) {
   // (100 x 98 strings 120 / 136 us an iteration).
   const bool product = op->prod.built && op->layout[0] != SQD_LAYOUT_CSR;
   if (!product && (n < kPairMinRows || op->nnz < kPairMinPerRow * n)) return 0;
-  return static_cast<size_t>(n) * nc * 4 + (product && nc == 2 ? static_cast<size_t>(n) * 12 : 0);
+  return static_cast<size_t>(n) * nc * 4 + (product && nc == 2 ? static_cast<size_t>(n) * 16 : 0);
 }
 
 void op_matvec_pair(sqd_op_s* op, const void* v0, void* out0, const void* v1, void* out1, int nc,

@@ -122,13 +122,13 @@ k_transpose(const E* __restrict__ in, E* __restrict__ out, int64_t rows, int64_t
 //                  result at out[a * B + b].
 // Eight entries per step keep eight independent index -> amplitude chains in flight.
 template <typename R, int NCV, int NCA, bool FINAL, bool HAS_M>
-__global__ void __launch_bounds__(256)
-k_slab(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* __restrict__ off,
-       const uint32_t* __restrict__ src, const R* __restrict__ V, const R* __restrict__ x,
-       const double* __restrict__ part_t, const double* __restrict__ part_m, R* __restrict__ out,
-       double* __restrict__ out_part, int prefetch) {
+__device__ __forceinline__ void
+slab_block(int64_t blk, int64_t A, int64_t B, int64_t total_k, int64_t a_tiles,
+           const int64_t* __restrict__ off, const uint32_t* __restrict__ src,
+           const R* __restrict__ V, const R* __restrict__ x, const double* __restrict__ part_t,
+           const double* __restrict__ part_m, R* __restrict__ out, double* __restrict__ out_part,
+           int prefetch) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t panels = (B + 31) >> 5;
   // A step's elements are one contiguous chunk of 8 x 32 entries (2 or 4 KB).  The chunk about
   // 2 KB ahead is prefetched into L2, one 128-byte line per lane, so the element loads wait on
   // L2 rather than on DRAM (measured: C3 FP64 matvec 5.9 -> 5.1 ms, C2 0.370 -> 0.324 ms; 4 KB
@@ -136,11 +136,10 @@ k_slab(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* __
   constexpr int U = NCV == 4 ? 4 : 8;   // entries per step; four when an amplitude is 32 bytes
   constexpr int kChunkLines = U * 32 * NCA * static_cast<int>(sizeof(R)) / 128;
   constexpr int pv = kChunkLines >= 16 ? 1 : 16 / kChunkLines;   // steps ahead
-  for (int64_t blk = blockIdx.x; blk < panels * a_tiles; blk += gridDim.x) {
-    const int64_t p = blk / a_tiles;
-    const int64_t a = (blk - p * a_tiles) * 8 + warp;
-    const int64_t b = p * 32 + lane;
-    if (a >= A || b >= B) continue;
+  const int64_t p = blk / a_tiles;
+  const int64_t a = (blk - p * a_tiles) * 8 + warp;
+  const int64_t b = p * 32 + lane;
+  if (a < A && b < B) {
     CAcc<R, NCV, NCA> acc;
     if constexpr (FINAL) {
       acc.add_partial(part_t, a * B + b);
@@ -181,6 +180,19 @@ k_slab(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* __
   }
 }
 
+// Blocks per SM that the register counts have to leave room for: the passes wait on their loads, and
+// one block less costs about 10 % (3072 x 2816 strings: complex64 final pass 461 -> 515 us at 50
+// instead of 48 registers).
+template <typename R, int NCV, int NCA, bool FINAL, bool HAS_M>
+__global__ void __launch_bounds__(256, NCV == 4 || NCA == 2 ? 4 : 6)
+k_slab(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* __restrict__ off,
+       const uint32_t* __restrict__ src, const R* __restrict__ V, const R* __restrict__ x,
+       const double* __restrict__ part_t, const double* __restrict__ part_m, R* __restrict__ out,
+       double* __restrict__ out_part, int prefetch) {
+  slab_block<R, NCV, NCA, FINAL, HAS_M>(blockIdx.x, A, B, total_k, a_tiles, off, src, V, x, part_t,
+                                        part_m, out, out_part, prefetch);
+}
+
 // FP32 slabs in 64-wide panels: a lane owns two adjacent positions b, b + 1, so one 16-byte
 // (complex64) or 8-byte (float) load reads both amplitudes and one 8- or 16-byte load both
 // elements; four entries per step.  Same sums per position as k_slab (FMA chains of four
@@ -216,25 +228,24 @@ __device__ __forceinline__ void pair_vec(const R* x, int64_t i, Cx<R>& v0, Cx<R>
 }
 
 template <typename R, int NCV, int NCA, bool FINAL, bool HAS_M, bool VEC>
-__global__ void __launch_bounds__(256)
-k_slab2(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* __restrict__ off,
-        const uint32_t* __restrict__ src, const R* __restrict__ V, const R* __restrict__ x,
-        const double* __restrict__ part_t, const double* __restrict__ part_m, R* __restrict__ out,
-        double* __restrict__ out_part) {
+__device__ __forceinline__ void
+slab2_block(int64_t blk, int64_t A, int64_t B, int64_t total_k, int64_t a_tiles,
+            const int64_t* __restrict__ off, const uint32_t* __restrict__ src,
+            const R* __restrict__ V, const R* __restrict__ x, const double* __restrict__ part_t,
+            const double* __restrict__ part_m, R* __restrict__ out,
+            double* __restrict__ out_part) {
   static_assert(sizeof(R) == 4, "two positions per lane: FP32 slabs");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t panels = (B + 63) >> 6;
   // element chunk of a step (4 x 64 entries, 1 or 2 KB) prefetched into L2 about 2 KB ahead,
   // as in k_slab (C3 FP32 matvec 3.32 -> 2.78 ms, C2 0.234 -> 0.210 ms; 1 KB ahead: 2.95 ms);
   // in the first pass only: the final pass, which also reads both FP64 partials, measured
   // slower with it (c3_small 90.5 -> 104.9 us, C3 1171 -> 1295 us)
   constexpr int kChunkLines = FINAL ? 0 : 4 * 64 * NCA * static_cast<int>(sizeof(R)) / 128;
   constexpr int pv = kChunkLines >= 16 ? 1 : kChunkLines > 0 ? 16 / kChunkLines : 1;
-  for (int64_t blk = blockIdx.x; blk < panels * a_tiles; blk += gridDim.x) {
-    const int64_t p = blk / a_tiles;
-    const int64_t a = (blk - p * a_tiles) * 8 + warp;
-    const int64_t b = p * 64 + 2 * lane;  // positions b and b + 1 (B is even)
-    if (a >= A || b >= B) continue;
+  const int64_t p = blk / a_tiles;
+  const int64_t a = (blk - p * a_tiles) * 8 + warp;
+  const int64_t b = p * 64 + 2 * lane;  // positions b and b + 1 (B is even)
+  if (a < A && b < B) {
     CAcc<R, NCV, NCA> acc0, acc1;
     if constexpr (FINAL) {
       acc0.add_partial(part_t, a * B + b);
@@ -298,6 +309,16 @@ k_slab2(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* _
       acc1.store_partial(out_part, a * B + b + 1);
     }
   }
+}
+
+template <typename R, int NCV, int NCA, bool FINAL, bool HAS_M, bool VEC>
+__global__ void __launch_bounds__(256, NCA == 2 ? 4 : NCV == 2 ? 5 : 6)
+k_slab2(int64_t A, int64_t B, int64_t total_k, int64_t a_tiles, const int64_t* __restrict__ off,
+        const uint32_t* __restrict__ src, const R* __restrict__ V, const R* __restrict__ x,
+        const double* __restrict__ part_t, const double* __restrict__ part_m, R* __restrict__ out,
+        double* __restrict__ out_part) {
+  slab2_block<R, NCV, NCA, FINAL, HAS_M, VEC>(blockIdx.x, A, B, total_k, a_tiles, off, src, V, x,
+                                              part_t, part_m, out, out_part);
 }
 
 // M pairs of every row, FP64 partial per row.  Same schedule as the CSR matvec: LPR lanes per
@@ -477,16 +498,27 @@ __device__ __forceinline__ Elem<R, NC> sm_elem(const R* p, int64_t i) {
 constexpr int kPanelGroup = 4;
 constexpr int kPanelAhead = 6;
 
+struct PanelArgs {
+  const int32_t* at;
+  const uint32_t* perm;
+  const uint16_t* src;
+  const uint32_t* horder;
+  int panels, steps, chunks, group;
+};
+
 template <typename R, int NCV, int NCA, int P, bool STAGED, bool FULL>
-__global__ void __launch_bounds__(P < kPanelMaxPerWarp ? 256 : 1024,
-                                  P == kPanelMaxPerWarp ? 1 : NCV == 4 ? 4 : 6)
-k_tail_panels(PlanView c, const int32_t* __restrict__ at, const uint32_t* __restrict__ perm,
-              const uint16_t* __restrict__ src, const uint32_t* __restrict__ horder, int panels,
-              int steps, int chunks, int group, const R* __restrict__ vm, const R* __restrict__ v, double* __restrict__ part) {
+__device__ __forceinline__ void
+panel_block(int blk, const PlanView& c, const PanelArgs& q, const R* __restrict__ vm,
+            const R* __restrict__ v, double* __restrict__ part) {
+  const int32_t* __restrict__ at = q.at;
+  const uint32_t* __restrict__ perm = q.perm;
+  const uint16_t* __restrict__ src = q.src;
+  const uint32_t* __restrict__ horder = q.horder;
+  const int panels = q.panels, steps = q.steps, chunks = q.chunks, group = q.group;
   extern __shared__ __align__(16) unsigned char panel_raw[];
   constexpr int EB = static_cast<int>(sizeof(R)) * NCV;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const int at_h = blockIdx.x / chunks, chunk = blockIdx.x - at_h * chunks;
+  const int at_h = blk / chunks, chunk = blk - at_h * chunks;
   const int h = __ldg(horder + at_h);
   const int nl = static_cast<int>(c.nl);
   const int64_t a_first = __ldg(c.aoff);
@@ -581,6 +613,92 @@ k_tail_panels(PlanView c, const int32_t* __restrict__ at, const uint32_t* __rest
   }
 }
 
+template <typename R, int NCV, int NCA, int P, bool STAGED, bool FULL>
+__global__ void __launch_bounds__(P < kPanelMaxPerWarp ? 256 : 1024,
+                                  P == kPanelMaxPerWarp ? 1 : NCV == 4 ? 4 : 6)
+k_tail_panels(PlanView c, PanelArgs q, const R* __restrict__ vm, const R* __restrict__ v,
+              double* __restrict__ part) {
+  panel_block<R, NCV, NCA, P, STAGED, FULL>(blockIdx.x, c, q, vm, v, part);
+}
+
+// ---- small grids: the three parts in one launch --------------------------------------------
+// The H, L and M parts depend only on v and its transpose.  On subspaces whose slab grids are
+// under two waves each pass waits on its own chains with most of the chip idle, so one launch
+// runs the blocks of all three (M first, whose blocks are the longest) into FP64 partials and
+// k_combine adds them: three launches instead of five.  M parts: eight warps, P panels each.
+template <typename R>
+struct SlabArgs {
+  int64_t A, B, total_k, a_tiles, blocks;
+  const int64_t* off;
+  const uint32_t* src;
+  const R* V;
+  const R* x;
+  double* part;
+  int vec;                   // FP32 pairs of positions: x allows the paired accesses
+};
+
+template <typename R, int NCV, int NCA, int P, bool FULL, bool WIDE>
+__global__ void __launch_bounds__(256, NCV == 4 ? 3 : P > 1 ? 4 : 5)
+k_parts(PlanView c, PanelArgs q, int64_t m_blocks, const R* __restrict__ vm,
+        const R* __restrict__ v, double* __restrict__ part_m, SlabArgs<R> L, SlabArgs<R> H) {
+  int64_t blk = blockIdx.x;
+  if (blk < m_blocks) {
+    panel_block<R, NCV, NCA, P, true, FULL>(static_cast<int>(blk), c, q, vm, v, part_m);
+    return;
+  }
+  blk -= m_blocks;
+  const bool low = blk < L.blocks;
+  const SlabArgs<R>& S = low ? L : H;
+  if (!low) blk -= L.blocks;
+  if constexpr (WIDE) {
+    if (S.vec)
+      slab2_block<R, NCV, NCA, false, false, true>(blk, S.A, S.B, S.total_k, S.a_tiles, S.off,
+                                                   S.src, S.V, S.x, nullptr, nullptr, nullptr,
+                                                   S.part);
+    else
+      slab2_block<R, NCV, NCA, false, false, false>(blk, S.A, S.B, S.total_k, S.a_tiles, S.off,
+                                                    S.src, S.V, S.x, nullptr, nullptr, nullptr,
+                                                    S.part);
+  } else {
+    slab_block<R, NCV, NCA, false, false>(blk, S.A, S.B, S.total_k, S.a_tiles, S.off, S.src, S.V,
+                                          S.x, nullptr, nullptr, nullptr, S.part, 1);
+  }
+}
+
+// out[h][l] = tL[l][h] + tH[h][l] (+ tM[h][l]), rounded once (32 x 32 tiles).
+template <typename R, int NCV, bool HAS_M>
+__global__ void __launch_bounds__(256)
+k_combine(const double* __restrict__ pl, const double* __restrict__ ph,
+          const double* __restrict__ pm, int64_t nh, int64_t nl, R* __restrict__ out) {
+  __shared__ double tile[NCV][32][33];
+  const int64_t th = (nh + 31) / 32, tl = (nl + 31) / 32;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int64_t t = blockIdx.x; t < th * tl; t += gridDim.x) {
+    const int64_t h0 = (t / tl) * 32, l0 = (t % tl) * 32;
+    for (int i = ty; i < 32; i += 8) {
+      const int64_t l = l0 + i, h = h0 + tx;
+      if (l < nl && h < nh) {
+#pragma unroll
+        for (int q = 0; q < NCV; ++q) tile[q][i][tx] = pl[(l * nh + h) * NCV + q];
+      }
+    }
+    __syncthreads();
+    for (int i = ty; i < 32; i += 8) {
+      const int64_t h = h0 + i, l = l0 + tx;
+      if (h < nh && l < nl) {
+        const int64_t r = (h * nl + l) * NCV;
+#pragma unroll
+        for (int q = 0; q < NCV; ++q) {
+          double s = tile[q][tx][i];
+          if constexpr (HAS_M) s += pm[r + q];
+          out[r + q] = static_cast<R>(s + ph[r + q]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
 // ---- short row tails ----------------------------------------------------------------------
 __global__ void k_tail_lengths(const int64_t* __restrict__ row_ptr, const int64_t* __restrict__ ho,
                                const int64_t* __restrict__ lo, int64_t n, int64_t nl,
@@ -608,8 +726,10 @@ __global__ void k_tail_fill(const int64_t* __restrict__ row_ptr, const uint32_t*
   }
 }
 
-unsigned capped_grid(int64_t blocks) {
-  return static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(blocks, INT_MAX)));
+// One block per tile: at most n / 256 + n / 32 of them for n < 2^31 rows.
+unsigned tile_grid(int64_t blocks) {
+  SQD_REQUIRE(blocks <= INT_MAX, "grid too large");
+  return static_cast<unsigned>(std::max<int64_t>(1, blocks));
 }
 
 // wide: FP32 slabs in 64-wide panels (k_slab2); vec: x and out allow its paired accesses.
@@ -622,10 +742,10 @@ void launch_slab(int64_t A, int64_t B, int64_t total_k, const int64_t* off, cons
     if (wide) {
       const int64_t a_tiles = (A + 7) / 8, panels = (B + 63) / 64;
       if (vec)
-        k_slab2<R, NCV, NCA, FINAL, HAS_M, true><<<capped_grid(a_tiles * panels), 256, 0, st>>>(
+        k_slab2<R, NCV, NCA, FINAL, HAS_M, true><<<tile_grid(a_tiles * panels), 256, 0, st>>>(
             A, B, total_k, a_tiles, off, src, V, x, part_t, part_m, out, out_part);
       else
-        k_slab2<R, NCV, NCA, FINAL, HAS_M, false><<<capped_grid(a_tiles * panels), 256, 0, st>>>(
+        k_slab2<R, NCV, NCA, FINAL, HAS_M, false><<<tile_grid(a_tiles * panels), 256, 0, st>>>(
             A, B, total_k, a_tiles, off, src, V, x, part_t, part_m, out, out_part);
       SQD_CHECK_LAUNCH();
       return;
@@ -637,14 +757,14 @@ void launch_slab(int64_t A, int64_t B, int64_t total_k, const int64_t* off, cons
   // 8,192 warps, FP64 matvec 0.348 -> 0.320 ms); on larger grids the other warps hide it and
   // the extra requests cost 2-4 % (C3, 524,288 warps).
   const int prefetch = A * panels <= 2 * 64 * int64_t(num_sms()) ? 1 : 0;
-  k_slab<R, NCV, NCA, FINAL, HAS_M><<<capped_grid(a_tiles * panels), 256, 0, st>>>(
+  k_slab<R, NCV, NCA, FINAL, HAS_M><<<tile_grid(a_tiles * panels), 256, 0, st>>>(
       A, B, total_k, a_tiles, off, src, V, x, part_t, part_m, out, out_part, prefetch);
   SQD_CHECK_LAUNCH();
 }
 
 template <typename E>
 void launch_transpose(const void* in, void* out, int64_t rows, int64_t cols, cudaStream_t st) {
-  const unsigned G = capped_grid(
+  const unsigned G = tile_grid(
       std::min<int64_t>(((rows + 31) / 32) * ((cols + 31) / 32), int64_t(num_sms()) * 32));
   k_transpose<E><<<G, 256, 0, st>>>(static_cast<const E*>(in), static_cast<E*>(out), rows, cols);
   SQD_CHECK_LAUNCH();
@@ -845,58 +965,162 @@ void ensure_floats(sqd_op_s* op, cudaStream_t st) {
   if (L.tail_state == 1 && !L.mval32.ptr) to_float(L.mval, L.mval32, st);
 }
 
-template <typename R, int NCV, int NCA>
-bool launch_panels(sqd_op_s* op, const R* vin, double* part, cudaStream_t st) {
-  ProductLayout& L = op->prod;
-  if (L.panel_state != 1) return false;
-  const R* vm;
-  if constexpr (sizeof(R) == 8) vm = L.vm.ptr;
-  else vm = L.vm32.ptr;
-  if (vm == nullptr) return false;
-  // Rows staged together: four, or what fits in half of the shared memory (two blocks per SM),
-  // at least one.
-  const size_t row = static_cast<size_t>(panel_row(L.nl, static_cast<int>(sizeof(R)) * NCV));
-  const bool staged = row <= kPanelSmem;
-  const int group = staged ? static_cast<int>(std::max<size_t>(
-                                 1, std::min<size_t>(kPanelGroup, kPanelSmem / 2 / row)))
-                           : kPanelGroup;
+// How k_tail_panels runs: rows staged together, panels per block (chunks), per warp.
+struct PanelShape {
+  PanelArgs args;
+  bool staged;
+  size_t dyn;
+  int64_t per, warps, blocks;
+};
+
+// max_dyn: shared memory for the staged rows; max_warps: of a block.
+PanelShape panel_shape(const ProductLayout& L, int element_bytes, double line, size_t max_dyn,
+                       int64_t max_warps) {
+  PanelShape s{};
+  // Rows staged together: four, or what fits, at least one.
+  const size_t row = static_cast<size_t>(panel_row(L.nl, element_bytes));
+  s.staged = row <= kPanelSmem;
+  const int group =
+      s.staged ? static_cast<int>(std::max<size_t>(1, std::min<size_t>(kPanelGroup, max_dyn / row)))
+               : kPanelGroup;
+  s.dyn = s.staged ? group * row : 0;
   // Panels per block: one per warp, eight warps, unless the staged row is more than their elements
   // (short B lists: 48 qubits, 2.3 steps a panel) or there are fewer than six blocks per SM.
-  const double line = 32.0 * sizeof(R) * NCA * double(L.steps) / double(L.panels);
-  const int64_t most = kPanelMaxWarps * kPanelMaxPerWarp;
   int64_t mine = std::max<int64_t>(8, static_cast<int64_t>(double(row) / std::max(line, 1.0)));
-  mine = std::min(std::min(mine, most), L.panels);
+  mine = std::min(std::min(mine, max_warps * kPanelMaxPerWarp), L.panels);
   while (mine > 4 && L.nh * ((L.panels + mine - 1) / mine) < 6 * int64_t(num_sms())) --mine;
   const int64_t chunks = (L.panels + mine - 1) / mine;
   mine = (L.panels + chunks - 1) / chunks;
-  const int64_t per = std::max((mine + kPanelMaxWarps - 1) / kPanelMaxWarps,
-                               std::min<int64_t>(kPanelMaxPerWarp, (mine + 7) / 8));
-  const int64_t warps = (mine + per - 1) / per;
-  SQD_REQUIRE(L.nh * chunks <= INT_MAX, "too many high strings");
-  const unsigned G = static_cast<unsigned>(L.nh * chunks);
+  s.per = std::max((mine + max_warps - 1) / max_warps,
+                   std::min<int64_t>(kPanelMaxPerWarp, (mine + 7) / 8));
+  s.warps = (mine + s.per - 1) / s.per;
+  s.blocks = L.nh * chunks;
+  s.args = PanelArgs{L.panel_at.ptr, L.perm.ptr, L.panel_src.ptr, L.horder.ptr,
+                     static_cast<int>(L.panels), static_cast<int>(L.steps),
+                     static_cast<int>(chunks), group};
+  return s;
+}
+
+template <typename R>
+const R* panel_elements(const ProductLayout& L) {
+  if (L.panel_state != 1) return nullptr;
+  if constexpr (sizeof(R) == 8) return L.vm.ptr;
+  else return L.vm32.ptr;
+}
+// Bytes of a panel's elements per A entry, on average.
+template <typename R, int NCA>
+double panel_line(const ProductLayout& L) {
+  return 32.0 * sizeof(R) * NCA * double(L.steps) / double(L.panels);
+}
+
+void allow_smem(const void* kern, size_t dyn) {
+  if (dyn > 48 * 1024)
+    SQD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(kPanelSmem)));
+}
+
+template <typename R, int NCV, int NCA>
+bool launch_panels(sqd_op_s* op, const R* vin, double* part, cudaStream_t st) {
+  ProductLayout& L = op->prod;
+  const R* vm = panel_elements<R>(L);
+  if (vm == nullptr) return false;
+  // two blocks per SM at least
+  const PanelShape s = panel_shape(L, static_cast<int>(sizeof(R)) * NCV, panel_line<R, NCA>(L),
+                                   kPanelSmem / 2, kPanelMaxWarps);
+  SQD_REQUIRE(s.blocks <= INT_MAX, "too many high strings");
   auto go = [&](auto kern) {
-    const size_t dyn = staged ? group * row : 0;
-    if (dyn > 48 * 1024)
-      SQD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(kPanelSmem)));
-    kern<<<G, static_cast<unsigned>(warps * 32), dyn, st>>>(
-        plan_view(*op->plan), L.panel_at.ptr, L.perm.ptr, L.panel_src.ptr, L.horder.ptr,
-        static_cast<int>(L.panels), static_cast<int>(L.steps), static_cast<int>(chunks), group, vm,
-        vin, part);
+    allow_smem(reinterpret_cast<const void*>(kern), s.dyn);
+    kern<<<static_cast<unsigned>(s.blocks), static_cast<unsigned>(s.warps * 32), s.dyn, st>>>(
+        plan_view(*op->plan), s.args, vm, vin, part);
     SQD_CHECK_LAUNCH();
   };
   auto pick = [&](auto p) {
     constexpr int P = decltype(p)::value;
-    if (!staged) go(k_tail_panels<R, NCV, NCA, P, false, false>);
+    if (!s.staged) go(k_tail_panels<R, NCV, NCA, P, false, false>);
     else if (L.panel_full) go(k_tail_panels<R, NCV, NCA, P, true, true>);
     else go(k_tail_panels<R, NCV, NCA, P, true, false>);
   };
-  switch (per) {
+  switch (s.per) {
     case 1: pick(IntTag<1>{}); break;
     case 2: pick(IntTag<2>{}); break;
     case 3: pick(IntTag<3>{}); break;
     default: pick(IntTag<4>{}); break;
   }
+  return true;
+}
+
+// Slab grids of at most two waves of warps (64 per SM) run the three parts in one launch: 512 x 512
+// strings at 32 qubits (0.9 waves) complex128 273 -> 212 us, complex64 172 -> 146, 130 x 100 36 -> 21.
+// Beyond, one launch and five are within 15 % either way (900 x 800, 2.4 waves: complex128 1082 /
+// 1225 us, float64 1023 / 917; 48 qubits, 1100 x 1000, 3.7 waves: complex64 88 / 104, float64 119 /
+// 117) and the additional partial vector costs memory.
+bool small_grid(const ProductLayout& L) {
+  const int64_t warps = std::max(L.nh * ((L.nl + 31) / 32), L.nl * ((L.nh + 31) / 32));
+  return warps <= 2 * 64 * int64_t(num_sms());
+}
+constexpr size_t kPartsSmem = 40 * 1024;
+
+template <typename R>
+SlabArgs<R> slab_args(int64_t A, int64_t B, int64_t total_k, const int64_t* off,
+                      const uint32_t* src, const R* V, const R* x, double* part, bool wide,
+                      bool vec) {
+  SlabArgs<R> s{};
+  s.A = A;
+  s.B = B;
+  s.total_k = total_k;
+  s.a_tiles = (A + 7) / 8;
+  s.blocks = s.a_tiles * (wide ? (B + 63) / 64 : (B + 31) / 32);
+  s.off = off;
+  s.src = src;
+  s.V = V;
+  s.x = x;
+  s.part = part;
+  s.vec = vec ? 1 : 0;
+  return s;
+}
+
+// Launches k_parts and k_combine; false where the M part does not fit beside the slabs (rows of v
+// over kPartsSmem) or is not in panels.
+template <typename R, int NCV, int NCA>
+bool launch_parts(sqd_op_s* op, const R* vin, R* vout, const SlabArgs<R>& low,
+                  const SlabArgs<R>& high, bool wide, double* part_m, cudaStream_t st) {
+  ProductLayout& L = op->prod;
+  PanelShape s{};
+  const R* vm = nullptr;
+  if (L.pairs_m > 0) {
+    vm = panel_elements<R>(L);
+    if (vm == nullptr) return false;
+    s = panel_shape(L, static_cast<int>(sizeof(R)) * NCV, panel_line<R, NCA>(L), kPartsSmem, 8);
+    if (!s.staged || s.dyn > kPartsSmem) return false;
+  }
+  const int64_t blocks = s.blocks + low.blocks + high.blocks;
+  if (blocks == 0 || blocks > INT_MAX) return false;
+  auto go = [&](auto kern) {
+    kern<<<static_cast<unsigned>(blocks), 256, s.dyn, st>>>(
+        plan_view(*op->plan), s.args, s.blocks, vm, vin, part_m, low, high);
+    SQD_CHECK_LAUNCH();
+  };
+  auto pick = [&](auto p) {
+    constexpr int P = decltype(p)::value;
+    if constexpr (sizeof(R) == 4) {
+      if (wide) {
+        if (L.panel_full) go(k_parts<R, NCV, NCA, P, true, true>);
+        else go(k_parts<R, NCV, NCA, P, false, true>);
+        return;
+      }
+    }
+    if (L.panel_full) go(k_parts<R, NCV, NCA, P, true, false>);
+    else go(k_parts<R, NCV, NCA, P, false, false>);
+  };
+  if (s.per <= 1) pick(IntTag<1>{});
+  else pick(IntTag<4>{});
+  const int64_t tiles = ((L.nh + 31) / 32) * ((L.nl + 31) / 32);
+  const unsigned G = static_cast<unsigned>(std::min<int64_t>(tiles, int64_t(num_sms()) * 16));
+  if (L.pairs_m > 0)
+    k_combine<R, NCV, true><<<G, 256, 0, st>>>(low.part, high.part, part_m, L.nh, L.nl, vout);
+  else
+    k_combine<R, NCV, false><<<G, 256, 0, st>>>(low.part, high.part, nullptr, L.nh, L.nl, vout);
+  SQD_CHECK_LAUNCH();
   return true;
 }
 
@@ -944,6 +1168,7 @@ void op_product_build(sqd_op_s* op, int layout, cudaStream_t st) {
   L.vt.alloc(static_cast<size_t>(n) * 2, st);
   L.tt.alloc(static_cast<size_t>(n) * 2, st);
   L.t.alloc(L.pairs_m > 0 ? static_cast<size_t>(n) * 2 : 1, st);
+  if (small_grid(L)) L.t2.alloc(static_cast<size_t>(n) * 2, st);
   op->prod = std::move(L);
   try {
     fill_slabs(op, true, false, st);
@@ -983,8 +1208,9 @@ void op_product_values32(sqd_op_s* op, cudaStream_t st) {
 namespace {
 
 // Scratch of one product matvec: FP64 values per row and vector component.
+// th: only for small grids (small_grid), else NULL.
 struct ProductScratch {
-  double *vt, *tt, *t;
+  double *vt, *tt, *t, *th;
 };
 
 template <typename R, int NCV, int NCA>
@@ -1016,6 +1242,13 @@ void product_matvec(sqd_op_s* op, const R* vin, R* vout, const ProductScratch& w
                       reinterpret_cast<uintptr_t>(vout) % pair_bytes == 0;
   // 1. vT[l][h] = v[h][l]
   launch_transpose<E>(vin, vt, nh, nl, st);
+  if (small_grid(L) && op->layout[prec] == SQD_LAYOUT_PRODUCT && w.th != nullptr) {
+    const SlabArgs<R> low = slab_args<R>(nl, nh, L.tl, L.lo.ptr, L.lsrc.ptr, VL, vt, w.tt, wide,
+                                         true);
+    const SlabArgs<R> high = slab_args<R>(nh, nl, L.th, L.ho.ptr, L.hsrc.ptr, VH, vin, w.th, wide,
+                                          vec_io);
+    if (launch_parts<R, NCV, NCA>(op, vin, vout, low, high, wide, w.t, st)) return;
+  }
   // 2. L part: t2[l][h]
   launch_slab<R, NCV, NCA, false, false>(nl, nh, L.tl, L.lo.ptr, L.lsrc.ptr, VL, vt, nullptr,
                                          nullptr, nullptr, w.tt, st, wide, true);
@@ -1062,7 +1295,7 @@ void op_product_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaSt
   ProductLayout& L = op->prod;
   SQD_REQUIRE(dtype_is_double(dtype) || L.vh32.ptr != nullptr,
               "FP32 product-layout elements were not prepared");
-  const ProductScratch w{L.vt.ptr, L.tt.ptr, L.t.ptr};
+  const ProductScratch w{L.vt.ptr, L.tt.ptr, L.t.ptr, L.t2.ptr};
   dispatch_vec(dtype, op->value_complex, [&](auto rt, auto ncv_t, auto nca_t) {
     using R = typename decltype(rt)::type;
     product_matvec<R, decltype(ncv_t)::value, decltype(nca_t)::value>(
@@ -1073,7 +1306,7 @@ void op_product_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaSt
 void op_product_matvec_pair(sqd_op_s* op, const double* v, double* out, double* scratch,
                             cudaStream_t st) {
   const int64_t n = op->prod.nh * op->prod.nl;
-  const ProductScratch w{scratch, scratch + 4 * n, scratch + 8 * n};
+  const ProductScratch w{scratch, scratch + 4 * n, scratch + 8 * n, scratch + 12 * n};
   if (op->value_complex) product_matvec<double, 4, 2>(op, v, out, w, st);
   else product_matvec<double, 4, 1>(op, v, out, w, st);
 }

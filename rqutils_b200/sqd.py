@@ -67,9 +67,8 @@ class SQDOptions:
     autotune: bool = False           # pick lanes_per_row by timing
     # With cache_strategy (1, 0) or (1, 1): cache the elements of the stored pairs, i.e. run
     # as (1, 2), when they fit in a quarter of the free device memory, or of the library pool's
-    # unused memory (the same Hv to
-    # rounding, several times faster), with the product-subspace layout where it applies.
-    # False keeps the requested strategy.
+    # unused memory (the same Hv to rounding, several times faster), with the product-subspace
+    # layout where it applies.  False keeps the requested strategy.
     promote_cache: bool = True
 
 
@@ -304,8 +303,9 @@ class SQDOperator:
 
     def promote_cache(self, fraction=0.25):
         """(1, 0)/(1, 1) -> (1, 2) when ``element_bytes()`` fits in ``fraction`` of the free
-        device memory or of what the library's pool holds unused; the product layout is selected when the subspace is a product of
-        high-half and low-half strings.  Returns True when the elements were cached."""
+        device memory or of what the library's pool holds unused; the product layout is
+        selected when the subspace is a product of high-half and low-half strings.  Returns
+        True when the elements were cached."""
         if tuple(self.cache_strategy) == (1, 2):
             return True
         if self.cache_strategy[0] != 1:
