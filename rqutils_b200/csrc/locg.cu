@@ -350,9 +350,10 @@ __device__ void run_post(LocgDev* d, int post, int nsrc, int use_cond,
       const double nv = sqrt(d->red[0][0]);
       set_coef_r(d, 0, 0, nv == 0.0 ? 1.0 : 1.0 / nv);
     } break;
-    case P_SET_R_COEF: {
+    case P_SET_R_COEF: {   // r over (ax, x) or (ax, x, y)
       set_coef_r(d, 0, 0, 1.0);
       set_coef_r(d, 0, 1, -d->theta);
+      set_coef_r(d, 0, 2, 0.0);
     } break;
     case P_THETA_ONLY: d->theta = d->red[0][0]; break;
     case P_RESET: {
@@ -743,6 +744,7 @@ using ShapeList = std::tuple<
     PassShape<3, 2, 100, 100, 101, 101>,
     PassShape<2, 2>,
     PassShape<2, 1, 100, 100, 0, 0>,                         // residual + convergence
+    PassShape<3, 1, 100, 100, 0, 0, 1, 100, 2, 100>,         // residual + convergence + ips
     PassShape<2, 1, 0, 0>,
     PassShape<1, 0, 0, 0>,
     PassShape<2, 0, 1, 0>,
@@ -1536,14 +1538,16 @@ class Locg {
     post_only(P_SET_R_COEF);
     lc({ax_.ptr, x}, {r_.ptr}, {}, P_NONE);
     project_orth(orth, r_.ptr, false, G_NONE);
+    if (orth.empty()) proj_ips();
   }
 
   // One body iteration (:324-383).  All passes are gated on `done`.
   void body(const std::vector<const void*>& orth) {
     R *x = x_.ptr, *y = y_.ptr, *r = r_.ptr, *p = p_.ptr;
     const int g = G_DONE;
-    // p = project_out((x, y), r): 4 rounds, normalising in the first two.
-    lc({r, x, y}, {}, {{1, 0}, {2, 0}}, P_PROJ_IPS, g);
+    // p = project_out((x, y), r): 4 rounds, normalising in the first two.  Without constraints the
+    // pass that formed r has left the first round's coefficients.
+    if (!orth.empty()) lc({r, x, y}, {}, {{1, 0}, {2, 0}}, P_PROJ_IPS, g);
     lc({r, x, y}, {p}, {{100, 100}, {1, 100}, {2, 100}}, P_PROJ_NORM_IPS, g);
     lc({p, x, y}, {p}, {{100, 100}, {1, 100}, {2, 100}}, P_PROJ_NORM_IPS, g);
     lc({p, x, y}, {p}, {{1, 100}, {2, 100}}, P_PROJ_IPS, g);
@@ -1563,7 +1567,7 @@ class Locg {
     matvec(x, ax_.ptr);
     if (!orth.empty()) post_only(P_SET_R_COEF, g);
     if (orth.empty()) {
-      lc({ax_.ptr, x}, {r}, {{100, 100}, {0, 0}}, P_CONV, g);
+      lc({ax_.ptr, x, y}, {r}, {{100, 100}, {0, 0}, {1, 100}, {2, 100}}, P_CONV_PROJ, g);
     } else {
       lc({ax_.ptr, x}, {r}, {{0, 0}}, P_STORE_AX, g);
       project_orth(orth, r, false, g);

@@ -36,6 +36,13 @@ _LOOKUPS = {'hash': _lib.SQD_LOOKUP_HASH, 'bsearch': _lib.SQD_LOOKUP_BSEARCH,
             'auto': _lib.SQD_LOOKUP_AUTO, 'product': _lib.SQD_LOOKUP_PRODUCT}
 
 
+# Stored pairs from which ``run_sqd`` takes the product layout of a product subspace.  A mixed /
+# FP64 iteration at 32 qubits: 66.8 / 148 us on it against 67.7 / 143 on the pair list at 9.7 M
+# pairs, 130 / 301 against 150 / 350 at 41 M, but 47 / 88 against 38 / 70 at 1.2 M, where its three
+# launches are the longer ones.
+_PRODUCT_FROM = 8 << 20
+
+
 @dataclass(frozen=True)
 class SQDOptions:
     """Options of ``sqd`` (sqd.py:183-196) plus B200 extensions (after ``locg_tol``).
@@ -301,11 +308,11 @@ class SQDOperator:
         per = 16 if self.value_complex else 8
         return int(self.nnz * per * 3)
 
-    def promote_cache(self, fraction=0.25):
+    def promote_cache(self, fraction=0.25, product_from=0):
         """(1, 0)/(1, 1) -> (1, 2) when ``element_bytes()`` fits in ``fraction`` of the free
         device memory or of what the library's pool holds unused; the product layout is
-        selected when the subspace is a product of high-half and low-half strings.  Returns
-        True when the elements were cached."""
+        selected when the subspace is a product of high-half and low-half strings and there are
+        at least ``product_from`` stored pairs.  Returns True when the elements were cached."""
         if tuple(self.cache_strategy) == (1, 2):
             return True
         if self.cache_strategy[0] != 1:
@@ -318,7 +325,7 @@ class SQDOperator:
             if self.element_bytes() > fraction * free:
                 return False
         self.cache_values()
-        if self.has_product_layout:
+        if self.nnz >= product_from and self.has_product_layout:
             self.set_layout(0, 'product')
             self.set_layout(1, 'product')
         return True
@@ -405,7 +412,7 @@ def run_sqd(hamiltonian, states, states_size, options=None, log_level=logging.IN
     op = SQDOperator(hamiltonian, space, options.cache_strategy, options.lookup,
                      options.lanes_per_row)
     if options.promote_cache and tuple(options.cache_strategy) in ((1, 0), (1, 1)):
-        op.promote_cache()
+        op.promote_cache(product_from=_PRODUCT_FROM)
     if options.autotune and options.lanes_per_row is None:
         op.autotune()
     if debug:
