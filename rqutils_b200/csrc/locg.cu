@@ -1348,6 +1348,216 @@ __global__ void __launch_bounds__(LC_THREADS, 2) k_locg_persist(PersistArgs pa) 
   }
 }
 
+// ------------------------------------------------------------ persistent reference iteration
+// The FP64 reference iteration (Locg::body without constraints) on a small cached CSR operator as
+// one launch, like k_locg_persist: its twelve launches per iteration become eight phases.  The
+// projection rounds, |s| and the update are persist_pass; A y and A p share one walk over a row's
+// pairs and form the Gram products of their rows on the spot (phase 5); the new x is normalised as
+// it is gathered for A x, whose phase also forms the residual and the products for the convergence
+// test and the next projection (phase 8).  Every vector holds what the graph form's does; only the
+// order of the dots' block sums differs.  Bound by the phases' barriers and scalar steps; persistent /
+// graph, us per iteration: 3,840 rows of 33 pairs 52 / 61, 5,000 of 6 54 / 71, 200,000 of one pair
+// 72 / 135, 250,000 of 19 (48 qubits) 135 / 173.
+struct PersistRefArgs {
+  // 0: first projection over (r, x, y); 1, 2: next rounds over (p, x, y); 3: last round and |p|;
+  // 4: the Gram products' post step; 5: |s|; 6: u, t and norms; 7: the convergence step
+  LCArgs<6, 10, 5> ps[8];
+  const void *x, *y, *p, *r, *ax, *ay, *ap;
+};
+
+template <typename R, int NC, int NCA, int LPR, bool CLU>
+__device__ __forceinline__ bool ref_gram(const PersistArgs& pa, const PersistRefArgs& ra,
+                                         LocgDev& sd, unsigned& gen, double* cpart, int& buf) {
+  // sources x, y, p, A x, A y, A p: <x|Ax>, <y|Ay>, <p|Ap>, <x|Ay>... as Locg::body lists them
+  using S = PassShape<6, 0, 0, 3, 1, 4, 2, 5, 1, 3, 2, 3, 2, 4>;
+  constexpr int ND = S::ND;
+  const R* x = static_cast<const R*>(ra.x);
+  const R* y = static_cast<const R*>(ra.y);
+  R* p = static_cast<R*>(const_cast<void*>(ra.p));
+  const R* ax = static_cast<const R*>(ra.ax);
+  R* ay = static_cast<R*>(const_cast<void*>(ra.ay));
+  R* ap = static_cast<R*>(const_cast<void*>(ra.ap));
+  const R* vals = static_cast<const R*>(pa.vals);
+  double acc[ND][2];
+#pragma unroll
+  for (int d = 0; d < ND; ++d) acc[d][0] = acc[d][1] = 0.0;
+  auto d2 = [](Cx<R> v) { return make_double2(double(v.re), double(v.im)); };
+  constexpr int RPW = 32 / LPR;
+  const int lane = threadIdx.x & 31;
+  const int sub = lane % LPR, slot = lane / LPR;
+  const int64_t w0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t rb = w0 * RPW; rb < pa.n; rb += nw * RPW) {
+    const int64_t row = rb + slot;
+    const bool live = row < pa.n, lead = live && sub == 0;
+    CAcc<R, NC, NCA> my, mp;
+    if (live) {
+      const int64_t e = __ldg(pa.row_ptr + row + 1);
+#pragma unroll 4
+      for (int64_t i = __ldg(pa.row_ptr + row) + sub; i < e; i += LPR) {
+        const uint32_t c = __ldg(pa.cols + i);
+        const Cx<R> el = ld_elem<R, NCA>(vals, i);
+        const Cx<R> vy = ld_elem_cg<R, NC>(y, c), vp = ld_elem_cg<R, NC>(p, c);
+        my.add(el, vy);
+        mp.add(el, vp);
+      }
+    }
+    my.merge(LPR);
+    mp.merge(LPR);
+    if (lead) {
+      const Cx<R> ay_ = cx_make<R>(my.re.value(), my.im.value());
+      const Cx<R> ap_ = cx_make<R>(mp.re.value(), mp.im.value());
+      st_elem<R, NC>(ay, row, ay_);
+      st_elem<R, NC>(ap, row, ap_);
+      const double2 sv[6] = {d2(ld_elem_cg<R, NC>(x, row)),  d2(ld_elem_cg<R, NC>(y, row)),
+                             d2(ld_elem_cg<R, NC>(p, row)),  d2(ld_elem_cg<R, NC>(ax, row)),
+                             d2(ay_),                        d2(ap_)};
+      DotLoop<S, 0, ND>::run(acc, sv, sv);
+    }
+  }
+  if (!persist_finish<ND, CLU>(acc, sd, pa, gen, cpart, buf)) return false;
+  if (threadIdx.x == 0) run_post(&sd, P_RR3, 6, 0, 0);
+  __syncthreads();
+  return true;
+}
+
+// x, y hold u, t; cu = 1 / |u|, ct = 1 / |t|: A x for x = cu u, then x, y, A x and r stored.  u and
+// t are overwritten in place, so the normalised x goes to xn (and the caller swaps the roles).
+template <typename R, int NC, int NCA, int LPR, bool CLU>
+__device__ __forceinline__ bool ref_residual(const PersistArgs& pa, const PersistRefArgs& ra,
+                                             const R* u, R* xn, LocgDev& sd, unsigned& gen,
+                                             double* cpart, int& buf, double cu_d, double ct_d) {
+  // sources ax, x, y; output r: |r|^2, |Ax|^2, <x|r>, <y|r>
+  using S = PassShape<3, 1, 100, 100, 0, 0, 1, 100, 2, 100>;
+  constexpr int ND = S::ND;
+  R* y = static_cast<R*>(const_cast<void*>(ra.y));
+  R* ax = static_cast<R*>(const_cast<void*>(ra.ax));
+  R* r = static_cast<R*>(const_cast<void*>(ra.r));
+  const R* vals = static_cast<const R*>(pa.vals);
+  const R cu = R(cu_d), ct = R(ct_d);
+  const double theta = sd.theta;
+  double acc[ND][2];
+#pragma unroll
+  for (int d = 0; d < ND; ++d) acc[d][0] = acc[d][1] = 0.0;
+  auto d2 = [](Cx<R> v) { return make_double2(double(v.re), double(v.im)); };
+  auto scaled = [](Cx<R> v, R s) { return cx_make<R>(v.re * s, v.im * s); };
+  constexpr int RPW = 32 / LPR;
+  const int lane = threadIdx.x & 31;
+  const int sub = lane % LPR, slot = lane / LPR;
+  const int64_t w0 = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
+  const int64_t nw = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  for (int64_t rb = w0 * RPW; rb < pa.n; rb += nw * RPW) {
+    const int64_t row = rb + slot;
+    const bool live = row < pa.n, lead = live && sub == 0;
+    CAcc<R, NC, NCA> m;
+    if (live) {
+      const int64_t e = __ldg(pa.row_ptr + row + 1);
+#pragma unroll 4
+      for (int64_t i = __ldg(pa.row_ptr + row) + sub; i < e; i += LPR)
+        m.add(ld_elem<R, NCA>(vals, i),
+              scaled(ld_elem_cg<R, NC>(u, __ldg(pa.cols + i)), cu));
+    }
+    m.merge(LPR);
+    if (lead) {
+      const Cx<R> ax_ = cx_make<R>(m.re.value(), m.im.value());
+      const Cx<R> x_ = scaled(ld_elem_cg<R, NC>(u, row), cu);
+      const Cx<R> y_ = scaled(ld_elem_cg<R, NC>(y, row), ct);
+      const Cx<R> r_ = cx_make<R>(R(double(ax_.re) - theta * double(x_.re)),
+                                  NC == 2 ? R(double(ax_.im) - theta * double(x_.im)) : R(0));
+      st_elem<R, NC>(ax, row, ax_);
+      st_elem<R, NC>(xn, row, x_);
+      st_elem<R, NC>(y, row, y_);
+      st_elem<R, NC>(r, row, r_);
+      const double2 sv[3] = {d2(ax_), d2(x_), d2(y_)};
+      const double2 ov[1] = {d2(r_)};
+      DotLoop<S, 0, ND>::run(acc, sv, ov);
+    }
+  }
+  if (!persist_finish<ND, CLU>(acc, sd, pa, gen, cpart, buf)) return false;
+  if (threadIdx.x == 0) run_post(&sd, P_CONV_PROJ, 3, 0, 0);
+  __syncthreads();
+  return true;
+}
+
+// x of iteration k lives in vector k mod 2 of (x, alt): u is written over the old x (phase 7) and
+// the normalised x to the other one.
+template <typename R, int NC, int NCA, int LPR, bool CLU>
+__global__ void __launch_bounds__(LC_THREADS, 2) k_locg_persist_ref(PersistArgs pa,
+                                                                    PersistRefArgs ra, R* alt) {
+  __shared__ LocgDev sd;
+  __shared__ double cpart[2 * 20];
+  __shared__ double ones[6];
+  {
+    const long long* src = reinterpret_cast<const long long*>(pa.dev);
+    long long* dst = reinterpret_cast<long long*>(&sd);
+    for (int i = threadIdx.x; i < int(sizeof(LocgDev) / sizeof(long long)); i += blockDim.x)
+      dst[i] = __ldcg(src + i);
+  }
+  if (threadIdx.x < 6) ones[threadIdx.x] = 1.0;
+  __syncthreads();
+  if (blockIdx.x != 0 && threadIdx.x == 0) sd.hist = nullptr;   // block 0 records
+  __syncthreads();
+  unsigned gen = 0;
+  int buf = 0;
+  R* const home = static_cast<R*>(const_cast<void*>(ra.x));
+  R* x = home;
+  R* other = alt;
+  auto with_x = [&](LCArgs<6, 10, 5> a, int at, int out) {   // the current x as source / output
+    a.src[at] = x;
+    if (out >= 0) a.out[out] = x;
+    return a;
+  };
+  using PProj2 = PassShape<3, 1, 1, 100, 2, 100>;
+  using PNorm = PassShape<3, 1, 100, 100>;
+  using PUpdate = PassShape<3, 2, 100, 100, 101, 101>;
+  for (int it = 0; it < pa.max_iter && !sd.done; ++it) {
+    if (!persist_pass<R, NC, PShape0, CLU>(with_x(ra.ps[0], 1, -1), sd, pa, gen, cpart, buf, ones))
+      return;
+    if (!persist_pass<R, NC, PShape0, CLU>(with_x(ra.ps[1], 1, -1), sd, pa, gen, cpart, buf, ones))
+      return;
+    if (!persist_pass<R, NC, PProj2, CLU>(with_x(ra.ps[2], 1, -1), sd, pa, gen, cpart, buf, ones))
+      return;
+    if (!persist_pass<R, NC, PNorm, CLU>(with_x(ra.ps[3], 1, -1), sd, pa, gen, cpart, buf, ones))
+      return;
+    if (!sd.keep) {   // the search direction vanished: p = 0
+      R* p = static_cast<R*>(const_cast<void*>(ra.p));
+      const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+      for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < pa.n; i += stride) {
+        const Cx<R> v = ld_elem_cg<R, NC>(p, i);   // times 0, as the masking pass computes it
+        st_elem<R, NC>(p, i, cx_make<R>(v.re * R(0), v.im * R(0)));
+      }
+      if (!persist_sync<CLU>(pa, gen)) return;
+    }
+    {
+      PersistRefArgs g = ra;
+      g.x = x;
+      if (!ref_gram<R, NC, NCA, LPR, CLU>(pa, g, sd, gen, cpart, buf)) return;
+    }
+    if (!persist_pass<R, NC, PNorm, CLU>(with_x(ra.ps[5], 0, -1), sd, pa, gen, cpart, buf, ones))
+      return;
+    if (!persist_pass<R, NC, PUpdate, CLU>(with_x(ra.ps[6], 0, 0), sd, pa, gen, cpart, buf, ones))
+      return;
+    // P_XY_NORM left 1 / |u| and 1 / |t| as the coefficients of the scaling pass
+    const double cu = sd.coef[0][0][0], ct = sd.coef[1][1][0];
+    if (!ref_residual<R, NC, NCA, LPR, CLU>(pa, ra, x, other, sd, gen, cpart, buf, cu, ct)) return;
+    R* t = x;
+    x = other;
+    other = t;
+  }
+  if (x != home) {   // the host reads x in its own vector
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < pa.n; i += stride)
+      st_elem<R, NC>(home, i, ld_elem_cg<R, NC>(x, i));
+  }
+  if constexpr (CLU) persist_sync<true>(pa, gen);   // no block leaves while others read its smem
+  if (blockIdx.x == 0) {
+    const long long* src = reinterpret_cast<const long long*>(&sd);
+    long long* dst = reinterpret_cast<long long*>(pa.dev);
+    for (int i = threadIdx.x; i < int(sizeof(LocgDev) / sizeof(long long)); i += blockDim.x)
+      dst[i] = src[i];
+  }
+}
+
 // ----------------------------------------------------------------------------- host driver
 struct Vec {
   void* p = nullptr;
@@ -1655,8 +1865,9 @@ class Locg {
             bool fast = false) {
     read_host();
     if (maxiter <= 0 || host_->done) return;
-    if (fast && use_graph && orth.empty() && persist_op_ != nullptr && persist_aligned()) {
-      loop_persistent(maxiter);
+    if (use_graph && orth.empty() && persist_op_ != nullptr && persist_aligned()) {
+      if (fast) loop_persistent(maxiter);
+      else loop_persistent_ref(maxiter);
       return;
     }
     auto run_body = [&] {
@@ -1784,7 +1995,7 @@ class Locg {
   void set_persistent_op(sqd_op_s* op) { persist_op_ = op; }
   // The persistent passes move 16 bytes of every vector per thread step.
   bool persist_aligned() const {
-    const R* vecs[] = {x_.ptr, y_.ptr, r_.ptr, p_.ptr, ax_.ptr, ay_.ptr, ap_.ptr};
+    const R* vecs[] = {x_.ptr, y_.ptr, r_.ptr, p_.ptr, ax_.ptr, ay_.ptr, ap_.ptr, t0_.ptr};
     for (const R* v : vecs)
       if (reinterpret_cast<uintptr_t>(v) % 16 != 0) return false;
     return true;
@@ -1796,57 +2007,135 @@ class Locg {
   // distributed shared memory.  Larger: a cooperative launch with the bounded grid barrier.
   static constexpr int kClusterMax = 16;
 
-  template <int NCA, int LPR>
-  void launch_persistent(PersistArgs& pa) {
+  // Launches kern_cluster (one thread-block cluster) or kern_grid (cooperative), by size; args:
+  // the kernel's arguments, pa among them.
+  template <typename... A>
+  void launch_persistent(PersistArgs& pa, void (*kern_cluster)(A...), void (*kern_grid)(A...),
+                         unsigned& grid, bool& cluster, void** args) {
     const int64_t want = (n_ + LC_THREADS - 1) / LC_THREADS;
-    if (persist_grid_ == 0) {
+    if (grid == 0) {
       if (want <= kClusterMax) {
-        persist_cluster_ = true;
-        persist_grid_ = static_cast<unsigned>(std::max<int64_t>(1, want));
+        cluster = true;
+        grid = static_cast<unsigned>(std::max<int64_t>(1, want));
       } else {
         int per_sm = 0;
-        SQD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, k_locg_persist<R, NC, NCA, LPR, false>, LC_THREADS, 0));
+        SQD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern_grid, LC_THREADS, 0));
         if (const char* e = std::getenv("SQD_LOCG_PERSIST_BLOCKS"))   // per SM (tuning)
           per_sm = std::min(per_sm, std::max(1, std::atoi(e)));
         const int64_t cap = static_cast<int64_t>(std::max(per_sm, 1)) * num_sms();
-        persist_grid_ = static_cast<unsigned>(std::max<int64_t>(1, std::min(want, cap)));
+        grid = static_cast<unsigned>(std::max<int64_t>(1, std::min(want, cap)));
       }
-      ppart_.alloc(static_cast<size_t>(persist_grid_) * 20 + 20, st_);
-      bar_.alloc(4, st_);
     }
+    const size_t need = static_cast<size_t>(grid) * 20 + 20;
+    if (ppart_.count < need) ppart_.alloc(need, st_);
+    if (!bar_.ptr) bar_.alloc(4, st_);
     pa.partials = ppart_.ptr;
-    pa.red = ppart_.ptr + static_cast<size_t>(persist_grid_) * 20;
+    pa.red = ppart_.ptr + static_cast<size_t>(grid) * 20;
     pa.bar = bar_.ptr;
     SQD_CUDA(cudaMemsetAsync(bar_.ptr, 0, 4 * sizeof(unsigned), st_));
-    if (persist_cluster_) {
-      auto kern = k_locg_persist<R, NC, NCA, LPR, true>;
-      if (persist_grid_ > 8)
+    if (cluster) {
+      const void* kern = reinterpret_cast<const void*>(kern_cluster);
+      if (grid > 8)
         SQD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
       cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(persist_grid_);
+      cfg.gridDim = dim3(grid);
       cfg.blockDim = dim3(LC_THREADS);
       cfg.stream = st_;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = persist_grid_;
+      attr[0].val.clusterDim.x = grid;
       attr[0].val.clusterDim.y = 1;
       attr[0].val.clusterDim.z = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      SQD_CUDA(cudaLaunchKernelEx(&cfg, kern, pa));
+      SQD_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
     } else {
-      auto kern = k_locg_persist<R, NC, NCA, LPR, false>;
-      void* args[] = {&pa};
-      SQD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern), persist_grid_,
+      SQD_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kern_grid), grid,
                                            LC_THREADS, args, 0, st_));
     }
+  }
+
+  void set_persist_operator(PersistArgs& pa, int maxiter) const {
+    const sqd_op_s* op = persist_op_;
+    pa.row_ptr = op->row_ptr.ptr;
+    pa.cols = op->cols.ptr;
+    if constexpr (sizeof(R) == 8) pa.vals = op->values.ptr;
+    else pa.vals = op->values32.ptr;
+    pa.n = n_;
+    pa.dev = dev_.ptr;
+    pa.max_iter = maxiter + 1;
+  }
+
+  // Lanes per row from the mean row length, not the standalone matvec's tuned value: inside
+  // the persistent launch the grid is small and a row's lanes should not exceed its pairs.
+  // f(NCA, LPR).
+  template <typename F>
+  void dispatch_persistent(F&& f) {
+    const sqd_op_s* op = persist_op_;
+    const double avg = n_ > 0 ? static_cast<double>(op->nnz) / static_cast<double>(n_) : 0.0;
+    const int lpr = avg >= 2 ? lanes_for(avg) : 1;
+    dispatch_lpr(lpr, [&](auto lpr_t) {
+      if constexpr (NC == 2) {
+        if (op->value_complex) f(IntTag<2>{}, lpr_t);
+        else f(IntTag<1>{}, lpr_t);
+      } else {
+        f(IntTag<1>{}, lpr_t);
+      }
+    });
+  }
+
+  // State back to the host; a barrier that timed out is an error.
+  void finish_persistent(const char* what, unsigned grid, bool cluster,
+                         std::chrono::steady_clock::time_point t_launch) {
+    read_host();
+    unsigned fault = 0;
+    SQD_CUDA(cudaMemcpyAsync(&fault, bar_.ptr + 2, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                             st_));
+    SQD_CUDA(cudaStreamSynchronize(st_));
+    if (std::getenv("SQD_LOCG_TRACE"))
+      std::fprintf(stderr, "[sqd_locg persistent] %s, %u blocks (%s), %d iterations, %.3f ms\n",
+                   what, grid, cluster ? "cluster" : "cooperative", host_->niter,
+                   std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() -
+                                                             t_launch).count());
+    if (fault)
+      throw Error(SQD_ERR_DEVICE, "persistent LOCG iteration: a grid barrier timed out");
+  }
+
+  // loop (reference iteration) as one launch (k_locg_persist_ref); FP64 only.
+  void loop_persistent_ref(int maxiter) {
+    R *x = x_.ptr, *y = y_.ptr, *r = r_.ptr, *p = p_.ptr;
+    PersistArgs pa{};
+    PersistRefArgs ra{};
+    fill(ra.ps[0], {r, x, y}, {p}, {{100, 100}, {1, 100}, {2, 100}}, P_PROJ_NORM_IPS, G_NONE);
+    fill(ra.ps[1], {p, x, y}, {p}, {{100, 100}, {1, 100}, {2, 100}}, P_PROJ_NORM_IPS, G_NONE);
+    fill(ra.ps[2], {p, x, y}, {p}, {{1, 100}, {2, 100}}, P_PROJ_IPS, G_NONE);
+    fill(ra.ps[3], {p, x, y}, {p}, {{100, 100}}, P_PROJ_MASK, G_NONE);
+    fill(ra.ps[5], {x, y, p}, {nullptr}, {{100, 100}}, P_SNORM, G_NONE);
+    fill(ra.ps[6], {x, y, p}, {x, y}, {{100, 100}, {101, 101}}, P_XY_NORM, G_NONE);
+    ra.x = x;
+    ra.y = y;
+    ra.p = p;
+    ra.r = r;
+    ra.ax = ax_.ptr;
+    ra.ay = ay_.ptr;
+    ra.ap = ap_.ptr;
+    set_persist_operator(pa, maxiter);
+    R* alt = t0_.ptr;
+    void* args[] = {&pa, &ra, &alt};
+    const auto t_launch = std::chrono::steady_clock::now();
+    dispatch_persistent([&](auto nca_t, auto lpr_t) {
+      constexpr int NCA = decltype(nca_t)::value, LPR = decltype(lpr_t)::value;
+      if constexpr (sizeof(R) == 8)
+        launch_persistent(pa, k_locg_persist_ref<R, NC, NCA, LPR, true>,
+                          k_locg_persist_ref<R, NC, NCA, LPR, false>, ref_grid_, ref_cluster_,
+                          args);
+    });
+    finish_persistent("fp64 reference", ref_grid_, ref_cluster_, t_launch);
   }
 
   // loop(fast) as one cooperative launch: the body_fast passes and the CSR matvec, phases
   // separated by grid barriers, until the convergence step sets `done`.
   void loop_persistent(int maxiter) {
-    sqd_op_s* op = persist_op_;
     R *x = x_.ptr, *y = y_.ptr, *r = r_.ptr, *p = p_.ptr;
     R *ax = ax_.ptr, *ay = ay_.ptr, *ap = ap_.ptr;
     PersistArgs pa{};
@@ -1858,43 +2147,18 @@ class Locg {
     fill(pa.ps[3], {x, y, p, ax, ay, ap}, {x, y, ax, ay, r},
          {{100, 100}, {101, 101}, {104, 104}, {102, 102}, {100, 104}, {101, 104}}, P_NONE,
          G_NONE);
-    pa.row_ptr = op->row_ptr.ptr;
-    pa.cols = op->cols.ptr;
-    if constexpr (sizeof(R) == 8) pa.vals = op->values.ptr;
-    else pa.vals = op->values32.ptr;
+    set_persist_operator(pa, maxiter);
     pa.mv_in = p;
     pa.mv_out = ap;
-    pa.n = n_;
-    pa.dev = dev_.ptr;
-    pa.max_iter = maxiter + 1;
-    // Lanes per row from the mean row length, not the standalone matvec's tuned value: inside
-    // the persistent launch the grid is small and a row's lanes should not exceed its pairs.
-    const double avg = n_ > 0 ? static_cast<double>(op->nnz) / static_cast<double>(n_) : 0.0;
-    const int lpr = avg >= 96 ? 32 : avg >= 40 ? 16 : avg >= 16 ? 8 : avg >= 6 ? 4
-                  : avg >= 2 ? 2 : 1;
+    void* args[] = {&pa};
     const auto t_launch = std::chrono::steady_clock::now();
-    dispatch_lpr(lpr, [&](auto lpr_t) {
-      constexpr int LPR = decltype(lpr_t)::value;
-      if constexpr (NC == 2) {
-        if (op->value_complex) launch_persistent<2, LPR>(pa);
-        else launch_persistent<1, LPR>(pa);
-      } else {
-        launch_persistent<1, LPR>(pa);
-      }
+    dispatch_persistent([&](auto nca_t, auto lpr_t) {
+      constexpr int NCA = decltype(nca_t)::value, LPR = decltype(lpr_t)::value;
+      launch_persistent(pa, k_locg_persist<R, NC, NCA, LPR, true>,
+                        k_locg_persist<R, NC, NCA, LPR, false>, persist_grid_, persist_cluster_,
+                        args);
     });
-    read_host();
-    unsigned fault = 0;
-    SQD_CUDA(cudaMemcpyAsync(&fault, bar_.ptr + 2, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                             st_));
-    SQD_CUDA(cudaStreamSynchronize(st_));
-    if (std::getenv("SQD_LOCG_TRACE"))
-      std::fprintf(stderr, "[sqd_locg persistent] %s, %u blocks (%s), %d iterations, %.3f ms\n",
-                   sizeof(R) == 4 ? "fp32" : "fp64", persist_grid_,
-                   persist_cluster_ ? "cluster" : "cooperative", host_->niter,
-                   std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() -
-                                                             t_launch).count());
-    if (fault)
-      throw Error(SQD_ERR_DEVICE, "persistent LOCG iteration: a grid barrier timed out");
+    finish_persistent(sizeof(R) == 4 ? "fp32" : "fp64", persist_grid_, persist_cluster_, t_launch);
   }
 
   int64_t n_;
@@ -1910,6 +2174,8 @@ class Locg {
   DevBuf<double> pair_;       // scratch of matvec2
   unsigned persist_grid_ = 0;
   bool persist_cluster_ = false;
+  unsigned ref_grid_ = 0;
+  bool ref_cluster_ = false;
   DevBuf<double> ppart_;
   DevBuf<unsigned> bar_;
   unsigned blocks_ = 1;
@@ -2009,6 +2275,21 @@ struct HistRecorder {
   }
 };
 
+// Persistent iterations (one cooperative launch per loop) where the matvec is the cached
+// CSR kernel and launch latency, not the matvec, bounds the graph form: up to 4 Mi rows with at
+// most 36 stored pairs each on average (a longer matvec runs better as its own kernel at full
+// occupancy).  Persistent / graph, us per iteration, 32 and 48 qubits: 3,840 rows of 33 pairs 30.4 /
+// 37.0, 250,000 of 19 75 / 94, 16,380 of 73 48.8 / 36.9, 1.1 M of 39 346 / 234.
+// SQD_LOCG_PERSISTENT=0 disables, =1 forces.
+bool persistent_fits(const sqd_op_s* op, int prec) {
+  const int64_t n = op->s->states_size;
+  if (op->x_cache != 1 || op->z_cache != 2 ||
+      (op->prod.built && op->layout[prec] != SQD_LAYOUT_CSR))
+    return false;
+  const char* env = std::getenv("SQD_LOCG_PERSISTENT");
+  return env ? std::atoi(env) != 0 : n <= (int64_t(4) << 20) && op->nnz <= 36 * n;
+}
+
 // cache_op: the sqd operator behind fn (NULL for a caller's own matvec), whose solver cache
 // the FP64 path may use.
 template <int NC>
@@ -2032,6 +2313,7 @@ void run_locg(int64_t n, int dtype, sqd_matvec_fn fn, void* ctx, sqd_op_s* cache
       lp = own.get();
     }
     lp->set_pair_op(cache_op);
+    lp->set_persistent_op(cache_op && persistent_fits(cache_op, 0) ? cache_op : nullptr);
     Locg<double, NC>& L = *lp;
     HistRecorder rec{g_hist_request};
     g_hist_request = HistRequest{};
@@ -2129,23 +2411,8 @@ void run_locg(int64_t n, int dtype, sqd_matvec_fn fn, void* ctx, sqd_op_s* cache
   // always set: a cached solver must not keep a previous solve's (freed) record buffer
   L.set_history(rec.rows[0].ptr, static_cast<int>(rec.req.max_rows), 0);
   l32->set_history(rec.rows[1].ptr, static_cast<int>(rec.req.max_rows), 1);
-  // Persistent iterations (one cooperative launch per loop) where the matvec is the cached
-  // CSR kernel and launch latency, not the matvec, bounds the graph form: up to 4 Mi rows with at
-  // most 36 stored pairs each on average (a longer matvec runs better as its own kernel at full
-  // occupancy).  Persistent / graph, us per iteration, 32 and 48 qubits: 3,840 rows of 33 pairs 30.4 /
-  // 37.0, 250,000 of 19 75 / 94, 16,380 of 73 48.8 / 36.9, 1.1 M of 39 346 / 234.
-  // SQD_LOCG_PERSISTENT=0 disables, =1 forces.
-  {
-    const char* env = std::getenv("SQD_LOCG_PERSISTENT");
-    const bool on = env ? std::atoi(env) != 0
-                        : n <= (int64_t(4) << 20) && op->nnz <= 36 * n;
-    auto csr = [&](int prec) {
-      return op->x_cache == 1 && op->z_cache == 2 &&
-             (!op->prod.built || op->layout[prec] == SQD_LAYOUT_CSR);
-    };
-    l32->set_persistent_op(on && csr(1) ? op : nullptr);
-    L.set_persistent_op(on && csr(0) ? op : nullptr);
-  }
+  l32->set_persistent_op(persistent_fits(op, 1) ? op : nullptr);
+  L.set_persistent_op(persistent_fits(op, 0) ? op : nullptr);
   {
     Locg<float, NC>& L32 = *l32;
     L32.set_stream(st);
