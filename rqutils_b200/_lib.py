@@ -148,9 +148,17 @@ def ptr(t):
     return _vp(t.data_ptr()) if t is not None else _vp(0)
 
 
+DTYPE_CODES = {torch.float64: SQD_F64, torch.complex128: SQD_C128, torch.float32: SQD_F32,
+               torch.complex64: SQD_C64}
+
+
 def dtype_code(dtype):
-    return {torch.float64: SQD_F64, torch.complex128: SQD_C128, torch.float32: SQD_F32,
-            torch.complex64: SQD_C64}[dtype]
+    return DTYPE_CODES[dtype]
+
+
+def raw_stream():
+    """The current device's current stream as an integer (``stream_ptr`` without its objects)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def tensor_from_ptr(address, n, dtype, device):

@@ -269,8 +269,11 @@ class SQDOperator:
             raise ValueError(f'vector length {v.shape[0]} != operator size {self.size}')
         if out is None:
             out = torch.empty_like(v)
-        _lib.call('sqd_matvec', self._handle, _lib.ptr(v), _lib.ptr(out),
-                  _lib.dtype_code(v.dtype), _lib.stream_ptr())
+        # the launch itself: no wrapper objects (at 2,000 rows the call is longer than its kernel)
+        status = _lib.load().sqd_matvec(self._handle, v.data_ptr(), out.data_ptr(),
+                                        _lib.DTYPE_CODES[v.dtype], _lib.raw_stream())
+        if status:
+            _lib.check(status)
         return out
 
     __call__ = matvec
