@@ -377,11 +377,17 @@ def run_ours(args):
     units = n_rows * m_terms
     value, t_max = replica_throughput(units, args.steps, t_local, dist)
     # kernels per matvec: CSR layout 1; product layout: transpose, low-half slabs, transpose,
-    # two-half CSR tails (when there are any), high-half slabs
+    # two-half pairs (when there are any), high-half slabs, or, with at most two waves of warps in
+    # a slab pass (64 per SM), transpose, all three parts, combine
     layout = op.get_layout(prec) if cache == (1, 2) else 'csr'
     per_step = 1
     if layout in ('product', 'product-csr'):
-        per_step = 5 if op.product_info()['pairs_mixed'] > 0 else 4
+        info = op.product_info()
+        nh, nl = info['n_high'], info['n_low']
+        warps = max(nh * ((nl + 31) // 32), nl * ((nh + 31) // 32))
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        small = layout == 'product' and warps <= 2 * 64 * sms
+        per_step = 3 if small else 5 if info['pairs_mixed'] > 0 else 4
     gpu_launches = args.steps * per_step
 
     # end to end: pinned host input -> device -> matvec -> pinned host output, every step.
@@ -572,14 +578,14 @@ def issue_bound(n, m, p, value_complex, sms, sm_mhz, t_matvec_s):
 
 def locg_bytes(n, m, j, p):
     """Algorithmic bytes of one LOCG iteration: matvecs x the matvec formula (W = 1, w_c = 16)
-    plus the vector reads and writes of the fused passes, counted from the iteration bodies:
-    the FP64 reference iteration (ground_locg.py:324-383) makes 4 complex128 matvecs and 42
-    vector reads/writes; an FP32 sweep of the mixed solver 1 complex64 matvec and 33 as a graph
-    of passes, 20 in the persistent launch (operators of at most 4 Mi rows and 64 Mi stored
-    pairs: C1, C5)."""
+    plus the vector reads and writes of the fused passes: the FP64 reference iteration
+    (ground_locg.py:324-383) is 4 complex128 matvecs and 42 vector reads/writes (the solver keeps
+    one product and shares the elements of two, so it moves less); an FP32 sweep of the mixed
+    solver 1 complex64 matvec and 33 as a graph of passes, 20 in the persistent launch (operators
+    of at most 4 Mi rows and 36 stored pairs a row: C1, C5)."""
     def mv(w_v):
         return n * (8 + 2 * w_v) + p * w_v + m * (8 + 16) + j * 8
-    persistent = n <= (4 << 20) and p <= (64 << 20)
+    persistent = n <= (4 << 20) and p <= 36 * n
     return {'fp64': 4 * mv(16) + 42 * n * 16,
             'fp32_sweep': mv(8) + (20 if persistent else 33) * n * 8,
             'fp32_sweep_form': 'persistent launch' if persistent else 'graph of passes',

@@ -129,7 +129,8 @@ void sqd_space_destroy(sqd_space_t s);
 /* The operator H projected on the subspace, with a connectivity cache chosen by
  * cache_strategy (SQDOptions.cache_strategy, sqd.py:187-189, run_sqd sqd.py:343-404):
  *   x_cache = 1: sources cached (sparse: only (row, group) pairs whose source exists);
- *   x_cache = 0: sources searched inside every matvec;
+ *   x_cache = 0: sources searched inside every matvec (product subspaces with SQD_LOOKUP_AUTO or
+ *   SQD_LOOKUP_PRODUCT: enumerated from partner lists per string of each half);
  *   z_cache = 2: matrix elements (composed diagonals) cached per stored pair;
  *   z_cache = 0 or 1: diagonals recomputed from popcounts inside every matvec.
  * lookup = enum sqd_lookup. */
@@ -153,10 +154,11 @@ int sqd_op_set_chunk(sqd_op_t op, int precision, int64_t chunk_rows);
  * that is the product of strings on the high and the low half of the qubits (every high string
  * with every low string, no fill-in slots), the pairs that change one half only are stored as
  * dense slabs whose sources are implied by their position (coalesced loads, no index per
- * pair); the pairs that change both halves gather from their source slabs staged in shared
- * memory when all of a slab's sources fit there, else from their CSR lists.
+ * pair); the pairs that change both halves are stored in panels whose source rows are staged in
+ * shared memory when most combinations of the halves' partners exist, else they gather from their
+ * CSR lists.
  * SQD_LAYOUT_PRODUCT_CSR: the same slabs, with the two-half pairs always on the CSR lists.
- * Lanes and chunk knobs apply to the two-half pairs.  Setting a product layout builds the
+ * Lanes and chunk knobs apply to the two-half pairs' CSR lists.  Setting a product layout builds the
  * slabs on first use (SQD_ERR_UNSUPPORTED when the subspace is not such a product); results
  * equal the CSR layout's up to the order of each row's sum. */
 enum sqd_layout { SQD_LAYOUT_CSR = 0, SQD_LAYOUT_PRODUCT = 1, SQD_LAYOUT_PRODUCT_CSR = 2 };

@@ -7,8 +7,9 @@ GPU through the C ABI of ``libsqd_b200.so``:
 * states are packed to uint64 (bit q = qubit q) and sorted/uniquified by a device radix sort;
   ascending uint64 order is the reference's order of padded big-endian byte rows, so basis
   order and eigenvector indexing match the reference exactly;
-* the b XOR x source lookups run once per operator over all (row, X-group) pairs with sector
-  and bitmap filters and a device hash table (``cache_strategy`` x = 1), or inside every matvec
+* the b XOR x source lookups run once per operator: on product subspaces per string of each half,
+  otherwise over all (row, X-group) pairs with a sector filter, a hashed state filter and a device
+  hash table (``cache_strategy`` x = 1), or inside every matvec
   (x = 0);
 * the matvec composes the diagonals from popcount(s & z) on the fly (z = 0/1) or reads them
   from a cache of the stored pairs (z = 2);
