@@ -237,7 +237,9 @@ enum sqd_locg_mode {
  *  residual_host = final |r| (may be NULL).
  *  With an sqd_op_t and no orth vectors, the solver's work vectors and captured iteration
  *  graphs stay with the operator for its next solve (no rqutils counterpart: XLA caches its
- *  compiled loop per shape): 8 vectors of dtype, plus 8 FP32 ones after a mixed solve, held
+ *  compiled loop per shape): 8 vectors of dtype, the scratch of applying A to two vectors at once
+ *  (4 vectors, 12 with complex vectors on a product layout; without memory for it A is applied
+ *  to one at a time) after an FP64 solve, 8 FP32 vectors after a mixed one, held
  *  until sqd_op_destroy; they are rebuilt when lanes, chunk, layout or coefficients change. */
 int sqd_locg(int64_t n, int dtype, sqd_matvec_fn fn, void* ctx, const void* xinit,
              int64_t xinit_index, const void* const* orth, int n_orth, double tol, int maxiter,

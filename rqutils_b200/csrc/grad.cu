@@ -265,6 +265,7 @@ k_grad_mixed(PlanView c, TermTable T, const GroupPre* __restrict__ groups, int64
 bool plan_groups(sqd_op_s* op, cudaStream_t st) {
   if (!op->plan) return false;
   ProductPlan& q = *op->plan;
+  std::lock_guard<std::mutex> lock(q.gmutex);
   if (q.gkey.ptr) return true;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   SQD_CUDA(cudaStreamIsCapturing(st, &cap));

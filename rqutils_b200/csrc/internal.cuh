@@ -1,6 +1,8 @@
 // Internal handle layouts shared by the library's translation units.
 #pragma once
 
+#include <mutex>
+
 #include "common.cuh"
 
 // Grouped Pauli table (device CSR).  Mirrors PauliSumXZ (paulis/symplectic.py:41-48): groups
@@ -105,6 +107,7 @@ struct ProductLayout {
   sqd::DevBuf<uint16_t> panel_src;   // [steps * 32]
   sqd::DevBuf<uint32_t> horder;      // [nh]
   int panel_full = 0;
+  int panel32_state = 0;             // -1: no memory for the FP32 copy
   sqd::DevBuf<double> vm;            // [ta * steps * 32] (x2 interleaved when complex)
   sqd::DevBuf<float> vm32;
   // Otherwise the CSR kernel runs over the row tails: in place, or over a contiguous copy when
@@ -139,6 +142,7 @@ struct ProductPlan {
   // (string, partner); classes H, L, A, B one after the other.
   sqd::DevBuf<uint32_t> gkey;
   sqd::DevBuf<uint2> gpair;
+  std::mutex gmutex;                  // gradients of one operator from several threads
 };
 
 // Solver objects an operator keeps between LOCG solves (locg.cu): work vectors and the

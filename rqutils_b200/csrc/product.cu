@@ -953,13 +953,14 @@ void ensure_floats(sqd_op_s* op, cudaStream_t st) {
     alloc_slabs32(op, st);
     fill_slabs(op, false, true, st);
   }
-  if (L.panel_state == 1 && !L.vm32.ptr) {
+  if (L.panel_state == 1 && !L.vm32.ptr && L.panel32_state == 0) {
     try {
       L.vm32.alloc(L.vm.count, st);
       fill_panels(op, false, true, st);
     } catch (const Error& e) {   // no memory: FP32 tails are read from the pair list
       if (e.status != SQD_ERR_MEMORY) throw;
       (void)cudaGetLastError();
+      L.panel32_state = -1;
     }
   }
   if (L.tail_state == 1 && !L.mval32.ptr) to_float(L.mval, L.mval32, st);
