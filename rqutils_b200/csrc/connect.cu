@@ -84,14 +84,16 @@ __global__ void k_mtable(const uint64_t* __restrict__ xm, const int32_t* __restr
 // halves' weights conserved (weighed), a mask can only have a partner when it moves as many bits
 // up as down, one popcount instead of a search (48 qubits: 22 % of the masks pass; both passes
 // take 0.47 ms for 1152 x 1000 strings, one warp per string and a search per mask took 1.4 ms).
+// Beyond kListStrings strings they are enough for one warp each, which keeps the counts small.
 constexpr int kListWarps = 8;
+constexpr int64_t kListStrings = 1 << 16;
 struct ListSearch {
   const uint64_t* strs[4];
   int64_t first[5];           // first block of each class; [4] = all blocks
   const uint64_t* xs[4];
   const int32_t* ids[4];      // key of mask k, NULL = k itself
   int64_t nx[4], nstr[4];
-  int weighed;
+  int weighed, warps;
 };
 
 template <bool FILL>
@@ -106,9 +108,9 @@ k_partner_lists(ListSearch q, int64_t* counts, const int64_t* __restrict__ place
   const uint64_t* __restrict__ xs = q.xs[c];
   const int64_t nstr = q.nstr[c], nx = q.nx[c];
   const uint64_t base = __ldg(strs + (int64_t(blockIdx.x) - q.first[c]));
-  const int64_t seg = (nx + kListWarps - 1) / kListWarps;
+  const int64_t seg = (nx + q.warps - 1) / q.warps;
   const int64_t k0 = warp * seg, k1 = min(nx, k0 + seg);
-  const int64_t slot = int64_t(blockIdx.x) * kListWarps + warp;
+  const int64_t slot = int64_t(blockIdx.x) * q.warps + warp;
   int64_t pos = FILL ? place[slot] : 0;
   for (int64_t kb = k0; kb < k1; kb += 32) {
     const int64_t k = kb + lane;
@@ -318,16 +320,17 @@ bool op_plan(sqd_op_s* op, cudaStream_t st) {
   f.ids[0] = gh.ptr;
   f.ids[1] = gl.ptr;
   f.weighed = sp->num_sectors == 2 ? 1 : 0;
+  f.warps = blocks <= kListStrings ? kListWarps : 1;
   SQD_REQUIRE(blocks < (int64_t(1) << 31), "too many half strings");
   DevBuf<int64_t> counts, place;
-  counts.alloc(blocks * kListWarps, st);
-  place.alloc(blocks * kListWarps + 1, st);
-  k_partner_lists<false><<<static_cast<unsigned>(blocks), kListWarps * 32, 0, st>>>(
+  counts.alloc(blocks * f.warps, st);
+  place.alloc(blocks * f.warps + 1, st);
+  k_partner_lists<false><<<static_cast<unsigned>(blocks), static_cast<unsigned>(f.warps * 32), 0, st>>>(
       f, counts.ptr, nullptr, nullptr, nullptr);
   SQD_CHECK_LAUNCH();
-  exclusive_scan_i64(counts.ptr, place.ptr, blocks * kListWarps, true, st);
+  exclusive_scan_i64(counts.ptr, place.ptr, blocks * f.warps, true, st);
   q.offs.alloc(blocks + 1, st);
-  k_every<<<grid_for(blocks + 1, 256, 4096), 256, 0, st>>>(place.ptr, blocks + 1, kListWarps,
+  k_every<<<grid_for(blocks + 1, 256, 4096), 256, 0, st>>>(place.ptr, blocks + 1, f.warps,
                                                            q.offs.ptr);
   SQD_CHECK_LAUNCH();
   int64_t end[4];
@@ -341,7 +344,7 @@ bool op_plan(sqd_op_s* op, cudaStream_t st) {
   q.tb = end[3] - end[2];
   q.key.alloc(std::max<int64_t>(end[3], 1), st);
   q.part.alloc(std::max<int64_t>(end[3], 1), st);
-  k_partner_lists<true><<<static_cast<unsigned>(blocks), kListWarps * 32, 0, st>>>(
+  k_partner_lists<true><<<static_cast<unsigned>(blocks), static_cast<unsigned>(f.warps * 32), 0, st>>>(
       f, nullptr, place.ptr, q.key.ptr, q.part.ptr);
   SQD_CHECK_LAUNCH();
   op->plan = std::move(plan);

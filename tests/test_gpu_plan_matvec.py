@@ -58,3 +58,19 @@ def test_composed_matvec_on_product_subspaces(name):
                 op = rq.SQDOperator(ham, space, cache_strategy=cache, lookup=lookup)
                 got = op.matvec(v).cpu().numpy()
                 assert np.abs(got - ref).max() <= RTOL[dt] * scale, (dt, cache, lookup)
+
+
+@pytest.mark.parametrize('nh, nl', [(1, 70001), (33000, 3)])
+def test_many_strings_in_one_half(nh, nl):
+    """More strings than get eight warps each: the connectivity equals the sweep's."""
+    rng = np.random.default_rng(nh)
+    hi = np.sort(rng.choice(1 << 17, size=nh, replace=False)).astype(np.uint64)
+    lo = np.sort(rng.choice(1 << 17, size=nl, replace=False)).astype(np.uint64)
+    states = ((hi[:, None] << np.uint64(17)) | lo[None, :]).reshape(-1)
+    x, z, c = W.random_pauli_sum(34, 150, rng, wmax=3)
+    ham = rq.PauliSumXZ.from_xz(x, z, c, 34, padded=True)
+    space = rq.Subspace.from_u64(states, 34)
+    a = rq.SQDOperator(ham, space, cache_strategy=(1, 2), lookup='product').csr()
+    b = rq.SQDOperator(ham, space, cache_strategy=(1, 2), lookup='hash').csr()
+    for u, w in zip(a, b):
+        assert torch.equal(u, w)
