@@ -14,6 +14,8 @@ differentiable object there is the matvec w.r.t. ``PauliSumXZ.c``, which is what
 Raw terms whose coefficient was zero when the Pauli sum was created have no slot in the table
 and get zero gradient.  Coefficients are the real raw coefficients (``force_real`` sums).
 """
+import contextlib
+
 import torch
 
 from .ground_locg import ground_locg
@@ -21,12 +23,39 @@ from .ground_locg import ground_locg
 
 def _apply_coeffs(op, coeffs):
     """Load ``coeffs`` into the operator's Pauli sum if they differ from the current ones."""
-    current = getattr(op, '_coeffs', None)
+    ham = op.hamiltonian
     c = coeffs.detach().to(torch.float64)
-    if current is None or current.shape != c.shape or not torch.equal(current, c.to(current.device)):
-        op.hamiltonian.set_coeffs(c)
+    current, imag = ham.raw_coeffs()
+    # coefficients that were set since the operator's last refresh are not in its elements
+    if op.coeffs_version != ham.coeffs_version or imag is not None or \
+            current.shape != c.shape or not torch.equal(current, c.to(current.device)):
+        ham.set_coeffs(c)
         op.refresh()
-        op._coeffs = c.to(op.space.device).clone()
+
+
+def _remember(ctx, op):
+    """The coefficients a forward pass ran with, for its backward pass."""
+    ctx.op = op
+    ctx.coeffs = op.hamiltonian.raw_coeffs()[0]    # a copy that no later call writes to
+    ctx.version = op.hamiltonian.coeffs_version
+
+
+@contextlib.contextmanager
+def _forward_coeffs(ctx):
+    """The operator with the coefficients of the forward pass of ``ctx``; those of a later call
+    come back afterwards.  Nothing to do (and no comparison) when none came in between."""
+    op, ham = ctx.op, ctx.op.hamiltonian
+    if ham.coeffs_version == ctx.version and op.coeffs_version == ctx.version:
+        yield op
+        return
+    (re, im), refreshed = ham.raw_coeffs(), op.coeffs_version == ham.coeffs_version
+    _apply_coeffs(op, ctx.coeffs)
+    try:
+        yield op
+    finally:
+        ham.set_coeffs(re if im is None else torch.complex(re, im))
+        if refreshed:
+            op.refresh()
 
 
 def _scatter_terms(op, g_terms):
@@ -39,19 +68,20 @@ class _Matvec(torch.autograd.Function):
     @staticmethod
     def forward(ctx, coeffs, v, op):
         _apply_coeffs(op, coeffs)
-        ctx.op = op
+        _remember(ctx, op)
         ctx.save_for_backward(v)
         return op.matvec(v.contiguous())
 
     @staticmethod
     def backward(ctx, g):
         (v,) = ctx.saved_tensors
-        op = ctx.op
         g = g.contiguous()
-        gv = op.matvec(g.to(v.dtype)) if ctx.needs_input_grad[1] else None
-        gc = None
-        if ctx.needs_input_grad[0]:
-            gc = _scatter_terms(op, op.grad_terms(g, v))
+        gc = gv = None
+        with _forward_coeffs(ctx) as op:
+            if ctx.needs_input_grad[1]:
+                gv = op.matvec(g.to(v.dtype))
+            if ctx.needs_input_grad[0]:
+                gc = _scatter_terms(op, op.grad_terms(g, v))
         return gc, gv, None
 
 
@@ -61,15 +91,15 @@ class _GroundEnergy(torch.autograd.Function):
         _apply_coeffs(op, coeffs)
         e, vec, _ = ground_locg(op, xinit, **kwargs)
         vec = vec / torch.linalg.vector_norm(vec)
-        ctx.op = op
+        _remember(ctx, op)
         ctx.save_for_backward(vec)
         return torch.tensor(e, dtype=torch.float64, device=vec.device)
 
     @staticmethod
     def backward(ctx, g):
         (vec,) = ctx.saved_tensors
-        op = ctx.op
-        gc = _scatter_terms(op, op.grad_terms(vec, vec)) * g
+        with _forward_coeffs(ctx) as op:
+            gc = _scatter_terms(op, op.grad_terms(vec, vec)) * g
         return gc, None, None, None
 
 

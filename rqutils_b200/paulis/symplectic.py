@@ -29,6 +29,8 @@ class PauliSumXZ:
     from byte-packed arrays ``PauliSumXZ(x, z, c, num_qubits)``.
     """
 
+    coeffs_version = 0      # calls of set_coeffs
+
     def __init__(self, x=None, z=None, c=None, num_qubits=None, *, padded=True, _handle=None,
                  _meta=None):
         self._handle = None
@@ -121,6 +123,7 @@ class PauliSumXZ:
         meta = _info(handle)
         obj = cls(num_qubits=num_qubits, padded=padded, _handle=handle, _meta=meta)
         obj._num_raw = x.shape[0]
+        obj._raw = (re, None if dropped.value else im)
         return obj
 
     def set_coeffs(self, coeffs):
@@ -141,6 +144,13 @@ class PauliSumXZ:
             warnings.warn('Found nonzero imaginary part when force_real=True')
         self._cache.pop('tables', None)
         self._cache.pop('ref', None)
+        self._raw = (re.clone(), None if im is None or dropped.value else im.clone())
+        self.coeffs_version += 1
+
+    def raw_coeffs(self):
+        """(real parts, imaginary parts or None) of the current raw coefficients: CUDA copies,
+        replaced and not written to by :meth:`set_coeffs`."""
+        return self._raw
 
     def raw_to_term(self):
         """int64 CUDA tensor: merged-term index of every raw term (-1 if dropped)."""

@@ -184,6 +184,7 @@ class SQDOperator:
         self.size = size.value
         self.value_complex = bool(cpx.value)
         self.cache_strategy = (x_cache, z_cache)
+        self.coeffs_version = hamiltonian.coeffs_version   # that the elements were made from
         if lanes_per_row is not None:
             self.lanes_per_row = lanes_per_row
 
@@ -304,6 +305,8 @@ class SQDOperator:
     def cache_values(self):
         """Cache the element of every stored pair: cache_strategy (1, 0)/(1, 1) -> (1, 2)."""
         _lib.call('sqd_op_cache_values', self._handle, _lib.stream_ptr())
+        if tuple(self.cache_strategy) != (1, 2):
+            self.coeffs_version = self.hamiltonian.coeffs_version
         self.cache_strategy = (1, 2)
 
     def element_bytes(self):
@@ -337,6 +340,7 @@ class SQDOperator:
     def refresh(self):
         """Recompute the cached matrix elements after ``hamiltonian.set_coeffs``."""
         _lib.call('sqd_op_refresh', self._handle, _lib.stream_ptr())
+        self.coeffs_version = self.hamiltonian.coeffs_version
 
     def grad_terms(self, u, v):
         """Re <u|P_t|v> for every merged term t (FP64 CUDA tensor of num_terms)."""
