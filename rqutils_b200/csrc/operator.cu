@@ -53,19 +53,14 @@ __global__ void k_gpre_fill(const uint64_t* group_x, int64_t J, const int64_t* f
   }
 }
 
-// Fill-in slots: only the last one has an entry (the diagonal group).
-__global__ void k_fill_counts(int64_t n_unique, int64_t size, int chunks, int has_diag,
-                              int64_t* counts) {
-  for (int64_t i = n_unique * chunks + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-       i < size * chunks; i += int64_t(gridDim.x) * blockDim.x)
-    counts[i] = (has_diag && i == (size - 1) * chunks) ? 1 : 0;
-}
-
-__global__ void k_row_starts(const int64_t* __restrict__ place, int64_t size, int chunks,
-                             int64_t* row_ptr) {
+// Row pointers from the real rows' places.  Fill-in slots: only the last one has an entry (the
+// diagonal group).
+__global__ void k_row_starts(const int64_t* __restrict__ place, int64_t n_unique, int64_t size,
+                             int chunks, int has_diag, int64_t* row_ptr) {
   for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r <= size;
        r += int64_t(gridDim.x) * blockDim.x)
-    row_ptr[r] = place[r * chunks];
+    row_ptr[r] = place[min(r, n_unique) * chunks] +
+                 (has_diag && size > n_unique && r == size ? 1 : 0);
 }
 
 // The pairs that the counting sweep kept, to their rows' slots.
@@ -318,7 +313,7 @@ void op_connect_sweep(sqd_op_s* op, cudaStream_t st) {
   const unsigned blocks = static_cast<unsigned>(tiles * chunks);
 
   DevBuf<int64_t> place;
-  place.alloc(size * chunks + 1, st);
+  place.alloc(nu * chunks + 1, st);   // real rows only: most of `size` may be repeats of a few states
   P.counts = place.ptr;
   DevBuf<unsigned long long> n_hits;
   n_hits.alloc(1, st);
@@ -341,15 +336,10 @@ void op_connect_sweep(sqd_op_s* op, cudaStream_t st) {
     kern<<<blocks, kThreads, dyn, st>>>(P);
     SQD_CHECK_LAUNCH();
   }
-  if (size > nu) {
-    k_fill_counts<<<grid_for((size - nu) * chunks, 256, 1024), 256, 0, st>>>(
-        nu, size, P.chunks, op->has_diag_group, place.ptr);
-    SQD_CHECK_LAUNCH();
-  }
-  exclusive_scan_i64(place.ptr, place.ptr, size * chunks, true, st);
+  exclusive_scan_i64(place.ptr, place.ptr, nu * chunks, true, st);
   op->row_ptr.alloc(size + 1, st);
-  k_row_starts<<<grid_for(size + 1, 256, 8192), 256, 0, st>>>(place.ptr, size, P.chunks,
-                                                              op->row_ptr.ptr);
+  k_row_starts<<<grid_for(size + 1, 256, 8192), 256, 0, st>>>(
+      place.ptr, nu, size, P.chunks, op->has_diag_group, op->row_ptr.ptr);
   SQD_CHECK_LAUNCH();
   unsigned long long found = 0;
   SQD_CUDA(cudaMemcpyAsync(&found, n_hits.ptr, sizeof(found), cudaMemcpyDeviceToHost, st));
