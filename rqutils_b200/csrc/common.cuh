@@ -93,6 +93,7 @@ struct DevBuf {
     cudaError_t err =
         cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ptr), n * sizeof(T), library_pool(), s);
     if (err != cudaSuccess) {
+      (void)cudaGetLastError();   // reported here; the next launch's check must not find it
       ptr = nullptr;
       count = 0;
       throw Error(SQD_ERR_MEMORY, std::string("device allocation of ") +

@@ -805,8 +805,11 @@ void alloc_slabs32(sqd_op_s* op, cudaStream_t st) {
   ProductLayout& L = op->prod;
   const int nca = op->value_complex ? 2 : 1;
   const int64_t w = L.wide32 ? 64 : 32;
-  L.vh32.alloc(static_cast<size_t>(std::max<int64_t>((L.nl + w - 1) / w * L.th * w, 1)) * nca, st);
-  L.vl32.alloc(static_cast<size_t>(std::max<int64_t>((L.nh + w - 1) / w * L.tl * w, 1)) * nca, st);
+  DevBuf<float> vh, vl;   // both or none: a failed allocation leaves the layout as it was
+  vh.alloc(static_cast<size_t>(std::max<int64_t>((L.nl + w - 1) / w * L.th * w, 1)) * nca, st);
+  vl.alloc(static_cast<size_t>(std::max<int64_t>((L.nh + w - 1) / w * L.tl * w, 1)) * nca, st);
+  L.vh32 = std::move(vh);
+  L.vl32 = std::move(vl);
 }
 
 // A row tail read in place is a short segment of the row's long pair list (48-qubit subspaces:
@@ -949,7 +952,7 @@ void build_mixed(sqd_op_s* op, int layout, cudaStream_t st) {
 // FP32 copies of whatever exists in FP64 and has none yet.
 void ensure_floats(sqd_op_s* op, cudaStream_t st) {
   ProductLayout& L = op->prod;
-  if (!L.vh32.ptr) {
+  if (!L.vh32.ptr || !L.vl32.ptr) {
     alloc_slabs32(op, st);
     fill_slabs(op, false, true, st);
   }
@@ -1294,7 +1297,7 @@ void product_matvec(sqd_op_s* op, const R* vin, R* vout, const ProductScratch& w
 
 void op_product_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st) {
   ProductLayout& L = op->prod;
-  SQD_REQUIRE(dtype_is_double(dtype) || L.vh32.ptr != nullptr,
+  SQD_REQUIRE(dtype_is_double(dtype) || (L.vh32.ptr != nullptr && L.vl32.ptr != nullptr),
               "FP32 product-layout elements were not prepared");
   const ProductScratch w{L.vt.ptr, L.tt.ptr, L.t.ptr, L.t2.ptr};
   dispatch_vec(dtype, op->value_complex, [&](auto rt, auto ncv_t, auto nca_t) {
