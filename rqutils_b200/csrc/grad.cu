@@ -33,7 +33,7 @@ __device__ __forceinline__ double signed_part(double wr, double wi, int ph, uint
   return __longlong_as_double(__double_as_longlong(v) ^ static_cast<long long>(flip));
 }
 
-// Diagonal group (x = 0, src = i, phase 1).
+// Diagonal group (x = 0, src = i, phase 1); a block takes every gridDim.y-th batch of terms.
 constexpr int GR_TILE = 1024, GR_TERMS = 64;
 
 template <int NCV>
@@ -43,8 +43,7 @@ k_grad_diag(const uint64_t* __restrict__ states, int64_t n_unique, TermTable T,
   __shared__ uint64_t s_st[GR_TILE];
   __shared__ double s_w[GR_TILE];
   const uint2 sp = __ldg(T.span);
-  const unsigned t0 = blockIdx.y * GR_TERMS;
-  if (t0 >= sp.y) return;
+  if (blockIdx.y * GR_TERMS >= sp.y) return;
   const int64_t r0 = static_cast<int64_t>(blockIdx.x) * GR_TILE;
   for (int k = threadIdx.x; k < GR_TILE; k += blockDim.x) {
     const int64_t r = r0 + k;
@@ -54,13 +53,15 @@ k_grad_diag(const uint64_t* __restrict__ states, int64_t n_unique, TermTable T,
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (unsigned t = t0 + warp; t < min(t0 + GR_TERMS, sp.y); t += 8) {
-    const uint64_t z = __ldg(T.rec + sp.x + t).x;
-    double a = 0.0;
+  for (unsigned t0 = blockIdx.y * GR_TERMS; t0 < sp.y; t0 += gridDim.y * GR_TERMS) {
+    for (unsigned t = t0 + warp; t < min(t0 + GR_TERMS, sp.y); t += 8) {
+      const uint64_t z = __ldg(T.rec + sp.x + t).x;
+      double a = 0.0;
 #pragma unroll 4
-    for (int k = lane; k < GR_TILE; k += 32) a += signed_part(s_w[k], 0.0, 0, s_st[k], z);
-    a = warp_sum(a);
-    if (lane == 0) atomicAdd(g + sp.x + t, a);
+      for (int k = lane; k < GR_TILE; k += 32) a += signed_part(s_w[k], 0.0, 0, s_st[k], z);
+      a = warp_sum(a);
+      if (lane == 0) atomicAdd(g + sp.x + t, a);
+    }
   }
 }
 
@@ -304,8 +305,8 @@ void grad_terms(sqd_op_s* op, const double* u, const double* v, double* g, cudaS
   sqd_space_s* sp = op->s;
   const TermTable T = term_table(p);
   if (op->has_diag_group && sp->n_unique > 0) {
-    const unsigned chunks = static_cast<unsigned>((p->max_k + GR_TERMS - 1) / GR_TERMS);
-    SQD_REQUIRE(chunks <= 65535, "diagonal group too large");
+    const unsigned chunks = static_cast<unsigned>(
+        std::min<int64_t>((p->max_k + GR_TERMS - 1) / GR_TERMS, 65535));
     k_grad_diag<NCV><<<dim3(grid_for(sp->n_unique, GR_TILE), chunks), 256, 0, st>>>(
         sp->states.ptr, sp->n_unique, T, u, v, g);
     SQD_CHECK_LAUNCH();
