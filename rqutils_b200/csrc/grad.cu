@@ -2,14 +2,17 @@
 // ph_t = (-i)^{|x & z_t|}, for every merged term t.
 //
 //  * Product subspaces (ProductPlan): a block or warp owns a group, so its terms' sums stay in
-//    registers and are stored once.  An H group x joins the pairs (h, h') of high strings with
+//    registers and are stored once.  Long groups (a few masks on many states, as in lattice
+//    models) have several owners, each adding its sums once.  An H group x joins the pairs (h, h') of high strings with
 //    every low string, an L group the other way round, a two-half group the pairs of its high part
 //    with the pairs of its low part; the pairs per group come from the halves' lists sorted by key.
 //  * Other subspaces: a lane per stored pair and one atomic addition per term.
 //  * The diagonal group: blocks of 1,024 rows by up to 64 terms, a warp per term.
 // Bound by the terms' popcounts and adds.  32 qubits, 256 x 240 strings, complex128: H 0.14, L 0.17,
 // two-half groups 0.07 ms (1.1 ms together with an atomic per pair and term); the diagonal under
-// 0.03 ms (0.29 ms with one block per row tile taking the terms one after the other).
+// 0.03 ms (0.29 ms with one block per row tile taking the terms one after the other).  All states of
+// 20 qubits, float64: an Ising chain 0.54 ms (one owner per group 15.1, an atomic per pair and term
+// 3.8), a Heisenberg chain 0.57 (28.8, 13.4).
 #include "internal.cuh"
 #include "dispatch.cuh"
 
@@ -132,9 +135,36 @@ __device__ __forceinline__ int64_t first_of(const uint32_t* __restrict__ key, in
   return lo;
 }
 
-// One block per H (HIGH) or L group: 256 pairs at a time in shared memory, each warp sums up to
-// eight of 64 terms over them.
-template <int NCV, bool HIGH>
+// The longest run of one key in each class.
+__global__ void k_longest_runs(const uint32_t* __restrict__ key, int64_t th, int64_t tl,
+                               int64_t ta, int64_t tb, unsigned long long* longest) {
+  const int64_t n = th + tl + ta + tb;
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const int cls = i < th ? 0 : i < th + tl ? 1 : i < th + tl + ta ? 2 : 3;
+    const int64_t first = cls == 0 ? 0 : cls == 1 ? th : cls == 2 ? th + tl : th + tl + ta;
+    const int64_t count = cls == 0 ? th : cls == 1 ? tl : cls == 2 ? ta : tb;
+    if (i > first && key[i] == key[i - 1]) continue;
+    atomicMax(longest + cls, static_cast<unsigned long long>(
+                                 first_of(key + first, count, key[i] + 1) - (i - first)));
+  }
+}
+
+// Owners of a group (blocks of k_grad_half, warps of k_grad_mixed): one, unless the longest group
+// has more than `most` pairs or there are too few groups to fill the chip (`room` owners), then
+// shares of at least `least` pairs.  At most kOwners over all groups.
+constexpr int64_t kOwners = 1 << 16;
+constexpr int64_t kHalfLeast = 1024, kHalfMost = 16384, kMixedLeast = 256, kMixedMost = 4096;
+unsigned owners(int64_t longest, int64_t groups, int64_t least, int64_t most, int64_t room) {
+  groups = std::max<int64_t>(groups, 1);
+  const int64_t split = std::min((longest + most - 1) / most, kOwners / groups);
+  const int64_t fill = std::min((longest + least - 1) / least, (room + groups - 1) / groups);
+  return static_cast<unsigned>(std::min<int64_t>(std::max({split, fill, int64_t(1)}), 65535));
+}
+
+// One block per H (HIGH) or L group and share of its pairs: 256 pairs at a time in shared memory,
+// each warp sums up to eight of 64 terms over them.
+template <int NCV, bool HIGH, bool SPLIT>
 __global__ void __launch_bounds__(256)
 k_grad_half(PlanView c, TermTable T, const GroupPre* __restrict__ groups,
             const uint32_t* __restrict__ key, const uint2* __restrict__ pair, int64_t count,
@@ -153,6 +183,14 @@ k_grad_half(PlanView c, TermTable T, const GroupPre* __restrict__ groups,
   if (ni == 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t total = ni * (HIGH ? c.nl : c.nh);
+  int64_t begin = 0, end = total;
+  if constexpr (SPLIT) {
+    const int64_t even = (total + gridDim.y - 1) / gridDim.y;
+    const int64_t share = max(kHalfLeast, (even + 255) / 256 * 256);
+    begin = blockIdx.y * share;
+    end = min(total, begin + share);
+    if (begin >= total) return;
+  }
   for (unsigned t0 = 0; t0 < sp.y; t0 += 64) {
     const unsigned left = sp.y - t0;
     const int mine = left > static_cast<unsigned>(warp) ? min(8u, (left - warp + 7) / 8) : 0;
@@ -165,11 +203,11 @@ k_grad_half(PlanView c, TermTable T, const GroupPre* __restrict__ groups,
       z[m] = m < mine ? __ldg(T.rec + sp.x + t0 + warp + 8 * m).x : 0;
       ph[m] = __popcll(grp.x & z[m]) & 3;
     }
-    for (int64_t q0 = 0; q0 < total; q0 += 256) {
+    for (int64_t q0 = begin; q0 < end; q0 += 256) {
       const int64_t q = q0 + threadIdx.x;
       uint64_t s = 0;
       double2 w = make_double2(0.0, 0.0);
-      if (q < total) {
+      if (q < end) {
         int64_t r, src;
         if constexpr (HIGH) {
           const int64_t i = q / c.nl, l = q - i * c.nl;
@@ -202,14 +240,18 @@ k_grad_half(PlanView c, TermTable T, const GroupPre* __restrict__ groups,
     for (int m = 0; m < 8; ++m) {
       if (m < mine) {
         const double a = warp_sum(acc[m]);
-        if (lane == 0) g[sp.x + t0 + warp + 8 * m] = a;
+        if (lane == 0) {
+          double* at = g + sp.x + t0 + warp + 8 * m;
+          if (SPLIT && end - begin < total) atomicAdd(at, a);
+          else *at = a;
+        }
       }
     }
   }
 }
 
-// One warp per two-half group, eight terms at a time.
-template <int NCV>
+// One warp per two-half group and share of its pairs, eight terms at a time.
+template <int NCV, bool SPLIT>
 __global__ void __launch_bounds__(256)
 k_grad_mixed(PlanView c, TermTable T, const GroupPre* __restrict__ groups, int64_t n_groups,
              uint64_t mlo, uint64_t mhi, int64_t na, const uint32_t* __restrict__ akey,
@@ -228,7 +270,11 @@ k_grad_mixed(PlanView c, TermTable T, const GroupPre* __restrict__ groups, int64
     const unsigned nA = static_cast<unsigned>(first_of(akey, ta, a + 1) - a0);
     const unsigned nB = static_cast<unsigned>(first_of(bkey, tb, b + 1) - b0);
     const unsigned total = nA * nB;       // at most nh * nl
-    if (total == 0) continue;
+    const unsigned share = max(static_cast<unsigned>(kMixedLeast),
+                               (total + gridDim.y - 1) / gridDim.y);
+    const unsigned begin = SPLIT ? min(total, blockIdx.y * share) : 0;   // total < 2^31
+    const unsigned end = SPLIT ? min(total, begin + share) : total;
+    if (begin == end) continue;
     for (unsigned t0 = 0; t0 < sp.y; t0 += 8) {
       const int mine = min(8u, sp.y - t0);
       double acc[8];
@@ -240,7 +286,7 @@ k_grad_mixed(PlanView c, TermTable T, const GroupPre* __restrict__ groups, int64
         z[m] = m < mine ? __ldg(T.rec + sp.x + t0 + m).x : 0;
         ph[m] = __popcll(grp.x & z[m]) & 3;
       }
-      for (unsigned q = lane; q < total; q += 32) {
+      for (unsigned q = begin + lane; q < end; q += 32) {
         const unsigned i = q / nB;
         const uint2 ph_ = __ldg(apair + a0 + i), pl = __ldg(bpair + b0 + (q - i * nB));
         const int64_t r = ph_.x * c.nl + pl.x, src = ph_.y * c.nl + pl.y;
@@ -254,7 +300,11 @@ k_grad_mixed(PlanView c, TermTable T, const GroupPre* __restrict__ groups, int64
       for (int m = 0; m < 8; ++m) {
         if (m < mine) {
           const double s = warp_sum(acc[m]);
-          if (lane == 0) g[sp.x + t0 + m] = s;
+          if constexpr (SPLIT) {
+            if (lane == 0) atomicAdd(g + sp.x + t0 + m, s);
+          } else {
+            if (lane == 0) g[sp.x + t0 + m] = s;
+          }
         }
       }
     }
@@ -275,7 +325,10 @@ bool plan_groups(sqd_op_s* op, cudaStream_t st) {
   DevBuf<uint64_t> keys;
   DevBuf<uint32_t> index, gkey;
   DevBuf<uint2> gpair;
+  DevBuf<unsigned long long> longest;
+  unsigned long long runs[4] = {0, 0, 0, 0};
   try {
+    longest.alloc(4, st);
     keys.alloc(std::max<int64_t>(n, 1), st);
     index.alloc(std::max<int64_t>(n, 1), st);
     gkey.alloc(std::max<int64_t>(n, 1), st);
@@ -287,6 +340,10 @@ bool plan_groups(sqd_op_s* op, cudaStream_t st) {
       radix_sort_u64(keys.ptr, index.ptr, n, 34, st);
       k_entry_pairs<<<G, 256, 0, st>>>(plan_view(q), keys.ptr, index.ptr, n, gkey.ptr, gpair.ptr);
       SQD_CHECK_LAUNCH();
+      SQD_CUDA(cudaMemsetAsync(longest.ptr, 0, longest.bytes(), st));
+      k_longest_runs<<<G, 256, 0, st>>>(gkey.ptr, q.th, q.tl, q.ta, q.tb, longest.ptr);
+      SQD_CHECK_LAUNCH();
+      SQD_CUDA(cudaMemcpyAsync(runs, longest.ptr, longest.bytes(), cudaMemcpyDeviceToHost, st));
     }
   } catch (const Error& e) {   // no memory: a lane per stored pair
     if (e.status != SQD_ERR_MEMORY) throw;
@@ -294,6 +351,7 @@ bool plan_groups(sqd_op_s* op, cudaStream_t st) {
     return false;
   }
   SQD_CUDA(cudaStreamSynchronize(st));   // later calls may come on other streams
+  for (int c = 0; c < 4; ++c) q.longest[c] = static_cast<int64_t>(runs[c]);
   q.gkey = std::move(gkey);
   q.gpair = std::move(gpair);
   return true;
@@ -317,22 +375,27 @@ void grad_terms(sqd_op_s* op, const double* u, const double* v, double* g, cudaS
     const uint32_t* key = q.gkey.ptr;
     const uint2* pair = q.gpair.ptr;
     const int64_t n0 = op->n_gpre_cls[0], n1 = op->n_gpre_cls[1], n2 = op->n_gpre_cls[2];
-    if (q.th > 0) {
-      k_grad_half<NCV, true><<<static_cast<unsigned>(n0), 256, 0, st>>>(
-          c, T, op->gpre.ptr, key, pair, q.th, sp->states.ptr, u, v, g);
+    // SPLIT: G.y owners per group
+    const int64_t room = 8 * num_sms();
+    auto half = [&](auto high, const GroupPre* groups, int64_t n, int64_t first, int64_t count,
+                    int64_t longest) {
+      constexpr bool HIGH = decltype(high)::value != 0;
+      const dim3 G(static_cast<unsigned>(n), owners(longest, n, kHalfLeast, kHalfMost, room));
+      auto kern = G.y > 1 ? k_grad_half<NCV, HIGH, true> : k_grad_half<NCV, HIGH, false>;
+      kern<<<G, 256, 0, st>>>(c, T, groups, key + first, pair + first, count, sp->states.ptr, u,
+                              v, g);
       SQD_CHECK_LAUNCH();
-    }
-    if (q.tl > 0) {
-      k_grad_half<NCV, false><<<static_cast<unsigned>(n1), 256, 0, st>>>(
-          c, T, op->gpre.ptr + n0, key + q.th, pair + q.th, q.tl, sp->states.ptr, u, v, g);
-      SQD_CHECK_LAUNCH();
-    }
+    };
+    if (q.th > 0) half(IntTag<1>{}, op->gpre.ptr, n0, 0, q.th, q.longest[0] * c.nl);
+    if (q.tl > 0) half(IntTag<0>{}, op->gpre.ptr + n0, n1, q.th, q.tl, q.longest[1] * c.nh);
     if (q.ta > 0 && q.tb > 0) {
       const uint64_t mlo = half_mask_low(sp->num_qubits), mhi = sp->fill_state & ~mlo;
       const int64_t oa = q.th + q.tl, ob = oa + q.ta;
-      k_grad_mixed<NCV><<<grid_for(n2 * 32, 256, num_sms() * 64), 256, 0, st>>>(
-          c, T, op->gpre.ptr + n0 + n1, n2, mlo, mhi, q.na, key + oa, pair + oa, q.ta, key + ob,
-          pair + ob, q.tb, sp->states.ptr, u, v, g);
+      const dim3 G(grid_for(n2 * 32, 256, num_sms() * 64),
+                   owners(q.longest[2] * q.longest[3], n2, kMixedLeast, kMixedMost, 8 * room));
+      auto kern = G.y > 1 ? k_grad_mixed<NCV, true> : k_grad_mixed<NCV, false>;
+      kern<<<G, 256, 0, st>>>(c, T, op->gpre.ptr + n0 + n1, n2, mlo, mhi, q.na, key + oa,
+                              pair + oa, q.ta, key + ob, pair + ob, q.tb, sp->states.ptr, u, v, g);
       SQD_CHECK_LAUNCH();
     }
     return;

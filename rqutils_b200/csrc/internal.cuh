@@ -142,6 +142,7 @@ struct ProductPlan {
   // (string, partner); classes H, L, A, B one after the other.
   sqd::DevBuf<uint32_t> gkey;
   sqd::DevBuf<uint2> gpair;
+  int64_t longest[4] = {0, 0, 0, 0};  // entries of one key at most, per class
   std::mutex gmutex;                  // gradients of one operator from several threads
 };
 
