@@ -322,6 +322,7 @@ bool plan_groups(sqd_op_s* op, cudaStream_t st) {
   SQD_CUDA(cudaStreamIsCapturing(st, &cap));
   if (cap != cudaStreamCaptureStatusNone) return false;
   const int64_t n = q.th + q.tl + q.ta + q.tb;
+  if (n >= (int64_t(1) << 31)) return false;   // more than the sort takes: a lane per stored pair
   DevBuf<uint64_t> keys;
   DevBuf<uint32_t> index, gkey;
   DevBuf<uint2> gpair;

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import rqutils_b200 as rq
+from rqutils_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +65,29 @@ def test_groups_of_many_pairs(dt):
         want = ((-1j) ** (bin(xk & zk).count('1') & 3) * (1 - 2 * (b & 1)).double() * w).real.sum()
         # 60,000 products, each rounded by a few ulps, in chains of at most 4096
         assert abs(got[k] - want) <= 4 * 2.0 ** -52 * op.size ** 0.5 * w.abs().sum(), k
+
+
+@pytest.mark.slow
+def test_more_list_entries_than_the_sort_takes():
+    """One high string and 2^26 low ones with 32 masks: 2^31 list entries, summed pair by pair."""
+    bits = 26
+    x = np.concatenate([1 << np.arange(bits, dtype=np.uint64), np.array([3, 5, 9, 17, 33, 65],
+                                                                        dtype=np.uint64)])
+    z = np.zeros_like(x)
+    z[::2] = np.uint64(1 << 12)
+    z &= ~x
+    ham = rq.PauliSumXZ.from_xz(x, z, np.ones(x.shape[0]), 2 * bits, force_real=True, padded=True)
+    states = torch.arange(1 << bits, dtype=torch.int64, device='cuda')
+    op = rq.SQDOperator(ham, rq.Subspace.from_u64(states, 2 * bits), cache_strategy=(1, 0))
+    assert op.nnz == 1 << 31
+    gen = torch.Generator(device='cuda').manual_seed(1)
+    u, v = (torch.randn(op.size, dtype=torch.float64, generator=gen, device='cuda')
+            for _ in range(2))
+    got = op.grad_terms(u, v)[ham.raw_to_term()]
+    for k in range(x.shape[0]):
+        w = u * v[states ^ int(x[k])]
+        want = (w * (1 - 2 * ((states & int(z[k])) != 0).double())).sum()
+        # 2^26 products added one by one: a random walk of rounding errors of the partial sums
+        assert (got[k] - want).abs() <= 2.0 ** -52 * op.size ** 0.5 * w.abs().sum(), k
+    del op
+    _lib.trim_memory()
