@@ -152,6 +152,8 @@ struct LocgCacheBase {
   virtual ~LocgCacheBase() = default;
 };
 
+constexpr uint64_t kUnsettled = ~0ull;   // values_version after a refresh
+
 struct sqd_op_s {
   sqd_paulis_s* p = nullptr;   // borrowed: must outlive the operator
   sqd_space_s* s = nullptr;    // borrowed
@@ -172,7 +174,7 @@ struct sqd_op_s {
   int64_t n_gpre_cls[3] = {0, 0, 0};  // gpre entries per class (H, L, M), in that order
   int product_built = 0;          // connectivity assembled from the two halves' lists
   std::unique_ptr<ProductPlan> plan;  // product subspaces: the halves' lists
-  uint64_t values_version = 0;    // p->version that the cached elements were computed from
+  uint64_t values_version = 0;    // p->version of elements whose computation has been waited for
   sqd::DevBuf<int> status;        // device status word
   int layout[2] = {0, 0};         // SQD_LAYOUT_* per precision
   ProductLayout prod;

@@ -508,7 +508,8 @@ extern "C" int sqd_vinit(sqd_op_t op, int64_t* index_host, void* stream) {
     keys.alloc(nw, st);
     idx.alloc(nw, st);
     res.alloc(1, st);
-    // Elements older than the coefficients (set_coeffs without a refresh) do not count.
+    // Elements older than the coefficients (set_coeffs without a refresh), or of a refresh, do not
+    // count.
     const bool cached = op->z_cache == 2 && op->values.ptr && op->values_version == p->version;
     if (cached)
       k_argmin_partial<true><<<G, 256, 0, st>>>(sp->states.ptr, sp->n_unique, term_table(p),
@@ -592,7 +593,9 @@ extern "C" int sqd_op_refresh(sqd_op_t op, void* stream) {
     out.values = op->values.ptr;
     op_product_targets(op, &out);
     op_pair_elements(op, out, st);
-    op->values_version = p->version;
+    // Nothing has waited for these elements: vinit, which may run on another stream, composes its
+    // diagonal instead of reading them.
+    op->values_version = kUnsettled;
     if (op->values32.ptr) {
       const size_t n = static_cast<size_t>(op->nnz) * (op->value_complex ? 2 : 1);
       k_to_float<<<grid_for(n, 256, 16384), 256, 0, st>>>(op->values.ptr, op->values32.ptr, n);
