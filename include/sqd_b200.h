@@ -130,7 +130,8 @@ void sqd_space_destroy(sqd_space_t s);
  * cache_strategy (SQDOptions.cache_strategy, sqd.py:187-189, run_sqd sqd.py:343-404):
  *   x_cache = 1: sources cached (sparse: only (row, group) pairs whose source exists);
  *   x_cache = 0: sources searched inside every matvec (product subspaces with SQD_LOOKUP_AUTO or
- *   SQD_LOOKUP_PRODUCT: enumerated from partner lists per string of each half);
+ *   SQD_LOOKUP_PRODUCT: enumerated from partner lists per string of each half, where that is the
+ *   faster way);
  *   z_cache = 2: matrix elements (composed diagonals) cached per stored pair;
  *   z_cache = 0 or 1: diagonals recomputed from popcounts inside every matvec.
  * lookup = enum sqd_lookup. */
@@ -142,7 +143,9 @@ int sqd_op_info(sqd_op_t op, int64_t* nnz, int64_t* states_size, int* value_comp
 /* Tuning knob of the cached matvec (no rqutils counterpart; rqutils leaves the schedule to
  * XLA): lanes of a warp that share one output row, 1/2/4/8/16/32, kept separately for FP64
  * (precision 0: SQD_F64/SQD_C128) and FP32 (precision 1: SQD_F32/SQD_C64) vectors.  Chosen
- * from the mean row length at creation; the autotuner overrides it. */
+ * from the mean row length at creation; the autotuner overrides it.  A matvec that does not walk
+ * the pair list has no use for it: the panels of SQD_LAYOUT_PRODUCT, and large product subspaces
+ * with z_cache 0 or 1, whose pairs are enumerated from partner lists. */
 int sqd_op_set_lanes(sqd_op_t op, int precision, int lanes_per_row);
 int sqd_op_get_lanes(sqd_op_t op, int precision, int* lanes_per_row);
 /* Second knob of the cached matvec: 0 = consecutive warps of the grid take consecutive rows;

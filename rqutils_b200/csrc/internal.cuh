@@ -308,6 +308,8 @@ __device__ __forceinline__ uint32_t filter_bit(uint64_t key, int log2) {
 
 // Build helpers implemented in operator.cu and matvec.cu.
 void op_build(sqd_op_s* op, cudaStream_t st);
+// With op->plan: the matvec that composes its elements reads the lists.
+bool op_plan_pays(const sqd_op_s* op);
 void op_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st);
 // Hv of two FP64 vectors (nc = 1: real, 2: complex) in one pass over the cached elements; scratch
 // of op_pair_scratch() doubles, 0 where two matvecs are the better way.

@@ -10,8 +10,9 @@
 //               The diagonal group (x = 0, K_0 terms, the largest group) is split over the LPR
 //               lanes of the row.
 //  * sweep APPLY (cache_strategy (0, *)): sources searched inside the matvec (apply_h).
-//  * k_mv_plan (both of the above on product subspaces, unless a hash or binary search was asked
-//               for): pairs enumerated from the halves' partner lists, elements composed.
+//  * k_mv_plan (both of the above on product subspaces where op_plan_pays, unless a hash or binary
+//               search was asked for): pairs enumerated from the halves' partner lists, elements
+//               composed.
 // FP32 vectors accumulate with error-free transformations (TwoProduct via fma, TwoSum), i.e.
 // the compensated dot product of Ogita, Rump and Oishi (SIAM J. Sci. Comput. 26, 2005), so the
 // FP32 result is as accurate as if accumulated in twice the working precision.
@@ -246,6 +247,41 @@ unsigned mv_grid(int64_t rows, int lpr) {
 
 }  // namespace
 
+// Whether the composing matvec runs over the halves' lists (k_mv_plan) or, without them, over the
+// stored pairs (k_mv_xc) or by searching (k_sweep).  Times at complex128 in us, lists / other.
+//
+// The lists' kernel looks up a group for every combination of A(h) x B(l), about 4.2 ps each on a
+// full chip, found or not.  Without stored pairs the sweep costs 4.6 ps a (row, group) test and
+// about 80 ps a pair; a share f of the tests of two-half groups finds one, f being that of the
+// parts' partners that exist, so the lists are the better way while
+//     combinations <= tests (1 + 19 f),   f = combinations / (rows na nb).
+// All states of 16 qubits, strings of random Paulis on every qubit: 300 of them 8588 / 1722, 1000
+// 14876 / 5632, 3000 15998 / 16468, 10000 19007 / 52520; molecular and local sums are far on the
+// lists' side (320 x 288 strings at 32 qubits 420 / 28600).
+//
+// With stored pairs a pair costs k_mv_xc about 4 ps per term more than it costs the lists' kernel
+// (terms of a group on one lane each against all lanes on the same group), which has to pay for the
+// combinations: 16 qubits, all states, 1000 terms 707 / 416 (7 combinations and 1.1 terms a pair),
+// 8000 2458 / 2770, 20000 3706 / 5933 (5.2 and 8).  And its blocks are few and long: 32 qubits, 64 x
+// 64 strings 104 / 31, 128 x 128 179 / 80, 200 x 200 297 / 223, 220 x 200 (5.9 M pairs) 274 / 250, 230
+// x 220 (7.2 M) 265 / 300, 64 x 800 (12 M) 370 / 531; 48 qubits, 250 x 250 (0.6 M) 119 / 90, 320 x 300
+// (1.2 M) 127 / 129, 500 x 500 266 / 371; Ising chain of 16 qubits 15 / 12, of 18 29 / 43.  Fewer
+// strings than half a tile in one half leave most lanes idle: 16 x 1820 (13 M pairs) 538 / 625, 12 x
+// 1000 (3 M) 326 / 160, 3 x 1800 519 / 113.
+bool op_plan_pays(const sqd_op_s* op) {
+  const ProductPlan& q = *op->plan;
+  const double rows = double(q.nh) * double(q.nl);
+  const double combinations = double(q.ta) * double(q.tb);
+  if (op->x_cache == 0) {
+    const double parts = std::max(double(q.na) * double(q.nb), 1.0);
+    return combinations * (1.0 - 19.0 * double(q.nm) / parts) <= rows * double(op->n_gpre);
+  }
+  const double terms = double(op->p->num_terms) / double(op->p->num_groups);
+  if (combinations > terms * double(op->nnz) || std::min(q.nh, q.nl) < kTileStrings / 2)
+    return false;
+  return rows >= 90 * 1024 || op->nnz >= 6.5 * 1024 * 1024;
+}
+
 void op_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st) {
   sqd_paulis_s* p = op->p;
   sqd_space_s* sp = op->s;
@@ -262,7 +298,7 @@ void op_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t s
     constexpr int NCA = decltype(nca_t)::value;
     const R* vin = static_cast<const R*>(v);
     R* vout = static_cast<R*>(out);
-    if (op->z_cache != 2 && op->plan) {
+    if (op->z_cache != 2 && op->plan && op_plan_pays(op)) {
       const int64_t tiles = ((op->plan->nh + kTileStrings - 1) / kTileStrings) *
                             ((op->plan->nl + kTileStrings - 1) / kTileStrings);
       k_mv_plan<R, NCV, NCA><<<static_cast<unsigned>(tiles), 1024, 0, st>>>(

@@ -268,7 +268,7 @@ void op_build(sqd_op_s* op, cudaStream_t st) {
     // entries per string) let the matvec enumerate its pairs (k_mv_plan).
     if (op->lookup == SQD_LOOKUP_AUTO || op->lookup == SQD_LOOKUP_PRODUCT) {
       try {
-        op_plan(op, st);
+        if (op_plan(op, st) && !op_plan_pays(op)) op->plan.reset();
       } catch (const Error& e) {   // no memory for the lists: every matvec searches
         if (e.status != SQD_ERR_MEMORY) throw;
         (void)cudaGetLastError();
