@@ -255,7 +255,7 @@ bool op_product_detect(sqd_op_s* op, cudaStream_t st, int64_t* nh_out, int64_t* 
   return true;
 }
 
-bool op_plan(sqd_op_s* op, cudaStream_t st) {
+bool op_plan(sqd_op_s* op, cudaStream_t st, int64_t most) {
   if (op->plan) return true;
   auto plan = std::make_unique<ProductPlan>();
   ProductPlan& q = *plan;
@@ -342,6 +342,7 @@ bool op_plan(sqd_op_s* op, cudaStream_t st) {
   q.tl = end[1] - end[0];
   q.ta = end[2] - end[1];
   q.tb = end[3] - end[2];
+  if (end[3] > most) return false;
   q.key.alloc(std::max<int64_t>(end[3], 1), st);
   q.part.alloc(std::max<int64_t>(end[3], 1), st);
   k_partner_lists<true><<<static_cast<unsigned>(blocks), static_cast<unsigned>(f.warps * 32), 0, st>>>(

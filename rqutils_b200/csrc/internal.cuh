@@ -326,8 +326,9 @@ void op_product_refresh(sqd_op_s* op, cudaStream_t st);
 void op_product_values32(sqd_op_s* op, cudaStream_t st);
 void op_product_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t st);
 // Product subspaces (connect.cu): builds op->plan unless it exists (false when the subspace is
-// not such a product), and the connectivity (row_ptr, cols, grps, nnz) from it.
-bool op_plan(sqd_op_s* op, cudaStream_t st);
+// not such a product, or its lists have more than `most` entries), and the connectivity (row_ptr,
+// cols, grps, nnz) from it.
+bool op_plan(sqd_op_s* op, cudaStream_t st, int64_t most = INT64_MAX);
 bool op_connect_product(sqd_op_s* op, cudaStream_t st);
 // Where the elements of the stored pairs go (elements.cu): the pair list (values: NCA doubles per
 // pair, or complex128 with out_complex) and, for the H and L pairs of a product subspace, the

@@ -265,10 +265,12 @@ void op_build(sqd_op_s* op, cudaStream_t st) {
   }
   if (op->x_cache == 0) {
     // Nothing is kept per row; on a product subspace the halves' partner lists (a few hundred
-    // entries per string) let the matvec enumerate its pairs (k_mv_plan).
+    // entries per string) let the matvec enumerate its pairs (k_mv_plan).  Not where they would be
+    // a pair list after all (one string in a half): 64 MB, or the size of the subspace's own arrays.
+    const int64_t most = std::max<int64_t>(int64_t(8) << 20, 4 * sp->n_unique);
     if (op->lookup == SQD_LOOKUP_AUTO || op->lookup == SQD_LOOKUP_PRODUCT) {
       try {
-        if (op_plan(op, st) && !op_plan_pays(op)) op->plan.reset();
+        if (op_plan(op, st, most) && !op_plan_pays(op)) op->plan.reset();
       } catch (const Error& e) {   // no memory for the lists: every matvec searches
         if (e.status != SQD_ERR_MEMORY) throw;
         (void)cudaGetLastError();
