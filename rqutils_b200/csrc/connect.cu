@@ -87,6 +87,7 @@ __global__ void k_mtable(const uint64_t* __restrict__ xm, const int32_t* __restr
 // Beyond kListStrings strings they are enough for one warp each, which keeps the counts small.
 constexpr int kListWarps = 8;
 constexpr int64_t kListStrings = 1 << 16;
+constexpr int64_t kListBlocks = 1 << 20;   // grid; beyond, a block takes several strings
 struct ListSearch {
   const uint64_t* strs[4];
   int64_t first[5];           // first block of each class; [4] = all blocks
@@ -102,33 +103,35 @@ k_partner_lists(ListSearch q, int64_t* counts, const int64_t* __restrict__ place
                 uint32_t* part) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  int c = 0;
-  while (c < 3 && int64_t(blockIdx.x) >= q.first[c + 1]) ++c;
-  const uint64_t* __restrict__ strs = q.strs[c];
-  const uint64_t* __restrict__ xs = q.xs[c];
-  const int64_t nstr = q.nstr[c], nx = q.nx[c];
-  const uint64_t base = __ldg(strs + (int64_t(blockIdx.x) - q.first[c]));
-  const int64_t seg = (nx + q.warps - 1) / q.warps;
-  const int64_t k0 = warp * seg, k1 = min(nx, k0 + seg);
-  const int64_t slot = int64_t(blockIdx.x) * q.warps + warp;
-  int64_t pos = FILL ? place[slot] : 0;
-  for (int64_t kb = k0; kb < k1; kb += 32) {
-    const int64_t k = kb + lane;
-    int64_t found = -1;
-    if (k < k1) {
-      const uint64_t x = __ldg(xs + k);
-      if (!q.weighed || 2 * __popcll(base & x) == __popcll(x))
-        found = sorted_find(strs, nstr, base ^ x);
+  for (int64_t blk = blockIdx.x; blk < q.first[4]; blk += gridDim.x) {
+    int c = 0;
+    while (c < 3 && blk >= q.first[c + 1]) ++c;
+    const uint64_t* __restrict__ strs = q.strs[c];
+    const uint64_t* __restrict__ xs = q.xs[c];
+    const int64_t nstr = q.nstr[c], nx = q.nx[c];
+    const uint64_t base = __ldg(strs + (blk - q.first[c]));
+    const int64_t seg = (nx + q.warps - 1) / q.warps;
+    const int64_t k0 = warp * seg, k1 = min(nx, k0 + seg);
+    const int64_t slot = blk * q.warps + warp;
+    int64_t pos = FILL ? place[slot] : 0;
+    for (int64_t kb = k0; kb < k1; kb += 32) {
+      const int64_t k = kb + lane;
+      int64_t found = -1;
+      if (k < k1) {
+        const uint64_t x = __ldg(xs + k);
+        if (!q.weighed || 2 * __popcll(base & x) == __popcll(x))
+          found = sorted_find(strs, nstr, base ^ x);
+      }
+      const unsigned b = __ballot_sync(kFullMask, found >= 0);
+      if (FILL && found >= 0) {
+        const int64_t i = pos + __popc(b & lt);
+        key[i] = q.ids[c] ? static_cast<uint32_t>(__ldg(q.ids[c] + k)) : static_cast<uint32_t>(k);
+        part[i] = static_cast<uint32_t>(found);
+      }
+      pos += __popc(b);
     }
-    const unsigned b = __ballot_sync(kFullMask, found >= 0);
-    if (FILL && found >= 0) {
-      const int64_t i = pos + __popc(b & lt);
-      key[i] = q.ids[c] ? static_cast<uint32_t>(__ldg(q.ids[c] + k)) : static_cast<uint32_t>(k);
-      part[i] = static_cast<uint32_t>(found);
-    }
-    pos += __popc(b);
+    if (!FILL && lane == 0) counts[slot] = pos;
   }
-  if (!FILL && lane == 0) counts[slot] = pos;
 }
 
 __global__ void k_every(const int64_t* __restrict__ in, int64_t n, int stride, int64_t* out) {
@@ -321,11 +324,11 @@ bool op_plan(sqd_op_s* op, cudaStream_t st, int64_t most) {
   f.ids[1] = gl.ptr;
   f.weighed = sp->num_sectors == 2 ? 1 : 0;
   f.warps = blocks <= kListStrings ? kListWarps : 1;
-  SQD_REQUIRE(blocks < (int64_t(1) << 31), "too many half strings");
+  const unsigned G = static_cast<unsigned>(std::min(blocks, kListBlocks));
   DevBuf<int64_t> counts, place;
   counts.alloc(blocks * f.warps, st);
   place.alloc(blocks * f.warps + 1, st);
-  k_partner_lists<false><<<static_cast<unsigned>(blocks), static_cast<unsigned>(f.warps * 32), 0, st>>>(
+  k_partner_lists<false><<<G, static_cast<unsigned>(f.warps * 32), 0, st>>>(
       f, counts.ptr, nullptr, nullptr, nullptr);
   SQD_CHECK_LAUNCH();
   exclusive_scan_i64(counts.ptr, place.ptr, blocks * f.warps, true, st);
@@ -345,7 +348,7 @@ bool op_plan(sqd_op_s* op, cudaStream_t st, int64_t most) {
   if (end[3] > most) return false;
   q.key.alloc(std::max<int64_t>(end[3], 1), st);
   q.part.alloc(std::max<int64_t>(end[3], 1), st);
-  k_partner_lists<true><<<static_cast<unsigned>(blocks), static_cast<unsigned>(f.warps * 32), 0, st>>>(
+  k_partner_lists<true><<<G, static_cast<unsigned>(f.warps * 32), 0, st>>>(
       f, nullptr, place.ptr, q.key.ptr, q.part.ptr);
   SQD_CHECK_LAUNCH();
   op->plan = std::move(plan);
@@ -366,7 +369,7 @@ bool op_connect_product(sqd_op_s* op, cudaStream_t st) {
   counts.release();
   op->cols.alloc(op->nnz > 0 ? op->nnz : 1, st);
   op->grps.alloc(op->nnz > 0 ? op->nnz : 1, st);
-  k_row_pairs<<<grid_for(n * 32, 256, 148 * 64), 256, 0, st>>>(c, op->row_ptr.ptr, op->cols.ptr,
+  k_row_pairs<<<grid_for(n * 32, 256, num_sms() * 64), 256, 0, st>>>(c, op->row_ptr.ptr, op->cols.ptr,
                                                                op->grps.ptr);
   SQD_CHECK_LAUNCH();
   op->product_built = 1;
