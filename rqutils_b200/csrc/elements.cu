@@ -7,8 +7,8 @@
 // waits for its longest group) and the diagonal, whose hundreds of terms are one pair of a row
 // (one lane of the warp that serves the row).  So:
 //  * the diagonal is a kernel of its own, a thread per row, every lane on the same term;
-//  * in a product subspace (ProductPlan) the H pairs are computed with a warp on 32 rows of one
-//    slab and the L pairs with a warp on 32 rows of one low string: the lanes share the group;
+//  * in a large product subspace (ProductPlan) the H pairs are computed with a warp on 32 rows of
+//    one slab and the L pairs with a warp on 32 rows of one low string: the lanes share the group;
 //  * the other pairs take a lane each; groups of more than kLongGroup terms wait in a queue in
 //    shared memory until 32 of them run together.
 // 48 qubits, 1152 x 1000 strings, 46 M pairs: 1.55 ms (L with the 1,129-term diagonals 1.04, H 0.34,
@@ -205,12 +205,22 @@ void half_elements(sqd_op_s* op, const ElementOut& o, cudaStream_t st) {
   }
 }
 
+// Whether the halves' kernels compute the elements of a product subspace.  A warp of theirs sums a
+// string's whole list, the diagonal's hundreds of terms with it, so they need strings enough to
+// fill the chip and both halves wide enough to fill the lanes.  Refresh in us, halves / rows: 32
+// qubits, 64 x 64 strings 104 / 45, 128 x 128 157 / 83, 180 x 170 204 / 135, 256 x 240 315 / 300, 400 x
+// 360 712 / 1030, 32 x 1800 627 / 700, 64 x 800 353 / 348, 12 x 1000 318 / 121, 1 x 1820 486 / 68; 48
+// qubits, 100 x 100 94 / 78, 300 x 300 131 / 153.
+bool halves_pay(const ProductPlan& q) {
+  return q.nh * q.nl >= 56 * 1024 && std::min(q.nh, q.nl) >= 32;
+}
+
 template <int NCA>
 void pair_elements(sqd_op_s* op, const ElementOut& o, cudaStream_t st) {
   sqd_space_s* sp = op->s;
   const TermTable T = term_table(op->p);
   const int64_t size = sp->states_size, nu = sp->n_unique;
-  if (op->plan) {
+  if (op->plan && halves_pay(*op->plan)) {
     half_elements<NCA, false>(op, o, st);
     if (op->plan->ta > 0 && op->plan->tb > 0) {
       k_pair_elements<NCA, true><<<grid_for(nu * 32, 256, num_sms() * 64), 256, 0, st>>>(
@@ -229,6 +239,7 @@ void pair_elements(sqd_op_s* op, const ElementOut& o, cudaStream_t st) {
       T, op->row_ptr.ptr, op->grps.ptr, sp->states.ptr, nu, op->has_diag_group, PlanView{},
       o.values, o.out_complex);
   SQD_CHECK_LAUNCH();
+  if (o.vh || o.vh32) half_elements<NCA, true>(op, o, st);
 }
 
 }  // namespace
