@@ -581,11 +581,12 @@ def locg_bytes(n, m, j, p):
     plus the vector reads and writes of the fused passes: the FP64 reference iteration
     (ground_locg.py:324-383) is 4 complex128 matvecs and 42 vector reads/writes (the solver keeps
     one product and shares the elements of two, so it moves less); an FP32 sweep of the mixed
-    solver 1 complex64 matvec and 33 as a graph of passes, 20 in the persistent launch (operators
-    of at most 4 Mi rows and 36 stored pairs a row: C1, C5)."""
+    solver 1 complex64 matvec and 33 as a graph of passes, 20 in the persistent launch (short rows:
+    C1, C5)."""
     def mv(w_v):
         return n * (8 + 2 * w_v) + p * w_v + m * (8 + 16) + j * 8
-    persistent = n <= (4 << 20) and p <= 36 * n
+    persistent = (p <= 36 * n if n <= 1 << 18 else p < 16 * n if n <= 1 << 19
+                  else n <= 1 << 21 and p < 6 * n)
     return {'fp64': 4 * mv(16) + 42 * n * 16,
             'fp32_sweep': mv(8) + (20 if persistent else 33) * n * 8,
             'fp32_sweep_form': 'persistent launch' if persistent else 'graph of passes',

@@ -2276,18 +2276,28 @@ struct HistRecorder {
 };
 
 // Persistent iterations (one cooperative launch per loop) where the matvec is the cached
-// CSR kernel and launch latency, not the matvec, bounds the graph form: up to 4 Mi rows with at
-// most 36 stored pairs each on average (a longer matvec runs better as its own kernel at full
-// occupancy).  Persistent / graph, us per iteration, 32 and 48 qubits: 3,840 rows of 33 pairs 30.4 /
-// 37.0, 250,000 of 19 75 / 94, 16,380 of 73 48.8 / 36.9, 1.1 M of 39 346 / 234.
+// CSR kernel and launch latency, not the matvec, bounds the graph form.  The launch runs 16 warps per
+// SM, so the more pairs there are, the sooner the graph's full occupancy wins.  Persistent / graph in
+// us per iteration, complex128, FP64 and mixed:
+//   rows      2 a row          9                17               25               36
+//   131,072   60/92   32/59    72/106  38/62    97/125  59/68    114/145 62/71    133/161 55/69
+//   262,144   73/138  41/87    96/162  51/92    189/218 95/109   233/256 113/120  227/266 103/123
+//   524,288   99/167  56/106   192/218 81/116   330/294 166/147  382/337 191/160  389/364 177/155
+//   1,048,576 210/240 105/145  370/322 180/174  658/462 327/213  785/562 368/239  765/617 336/228
+//   2,097,152 441/396 215/227  783/552 344/266  1415/824 678/349
+// float64 alike; 5 a row at 1 Mi rows 234/261 116/153, at 2 Mi 486/427 222/232; 15.6 a row at 500,000
+// 269/324 110/139; 250,000 rows of 52 397/359 207/157, 16,380 of 73 (mixed) 49/37.
 // SQD_LOCG_PERSISTENT=0 disables, =1 forces.
 bool persistent_fits(const sqd_op_s* op, int prec) {
-  const int64_t n = op->s->states_size;
+  const int64_t n = op->s->states_size, nnz = op->nnz;
   if (op->x_cache != 1 || op->z_cache != 2 ||
       (op->prod.built && op->layout[prec] != SQD_LAYOUT_CSR))
     return false;
   const char* env = std::getenv("SQD_LOCG_PERSISTENT");
-  return env ? std::atoi(env) != 0 : n <= (int64_t(4) << 20) && op->nnz <= 36 * n;
+  if (env) return std::atoi(env) != 0;
+  if (n <= (1 << 18)) return nnz <= 36 * n;
+  if (n <= (1 << 19)) return nnz < 16 * n;
+  return n <= (prec == 0 ? 1 << 20 : 1 << 21) && nnz < 6 * n;
 }
 
 // cache_op: the sqd operator behind fn (NULL for a caller's own matvec), whose solver cache
