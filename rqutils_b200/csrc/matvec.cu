@@ -232,11 +232,19 @@ __global__ void k_deinterleave(const E* __restrict__ in, E* __restrict__ a, E* _
   }
 }
 
-// From where the pair list is read for two vectors at once (op_pair_scratch).  FP64 iteration at
-// 32 qubits, pair / two matvecs: 100 x 98 strings (56 pairs a row) 76.8 / 75.1 us, 180 x 170 (107 a
-// row) 96.2 / 96.4, 448 x 400 (339 a row) 511 / about 640; 200,000 states with one pair a row
-// 142.0 / 138.8.
-constexpr int64_t kPairMinRows = 16384, kPairMinPerRow = 16;
+// From where the pair list is read for two vectors at once (op_pair_scratch).  FP64 iteration in us,
+// pair / two matvecs, float64 and complex128 with real elements:
+//   rows      16 a row          24               33               64
+//   16,384                                                        65/65   71/71
+//   32,768    64/63   69/68     68/67   74/73    68/68   76/76    78/81   87/87
+//   65,536    78/77   86/85     83/85   93/93    86/87   95/98    100/107 118/120
+//   131,072   105/106 120/118   113/117 132/132  119/122 142/141
+//   262,144   164/164 203/193   188/194 231/234  204/210 252/259
+//   1,048,576 326/348 464/460   402/440 563/592
+// 16,384 rows of 129: 71/75 81/79, 30,600 of 108: 83/87 100/99; complex elements at 262,144 rows of
+// 24: 256/284.
+constexpr int64_t kPairMinRows[2] = {16384, 32768};   // real, complex vectors
+constexpr int64_t kPairMinPerRow = 24, kPairMinPairs = int64_t(3) << 19;
 
 unsigned mv_grid(int64_t rows, int lpr) {
   const int64_t warps = (rows * lpr + 31) / 32;
@@ -356,15 +364,19 @@ void op_matvec(sqd_op_s* op, const void* v, void* out, int dtype, cudaStream_t s
 
 // Two FP64 vectors share one pass over the elements.  Interleaving them costs four reads and
 // writes of each vector, so it pays where a row has many more pairs than that.  Real vectors
-// become one complex vector over the same (real) elements; every component is summed as it is
-// alone, so the results are bit-identical to two matvecs.
+// become one complex vector over the same (real) elements.  On the pair list every component is
+// summed as it is alone, bit for bit; on the product layouts the twice as long elements may take
+// another number of high-string partners at a time, or leave the one-launch form, which adds the
+// same products in another order.
 size_t op_pair_scratch(const sqd_op_s* op, int nc) {
   if (op->x_cache != 1 || op->z_cache != 2) return 0;
   const int64_t n = op->s->states_size;
   // The product layouts' five launches per matvec make the pair the better way at every size
   // (100 x 98 strings 120 / 136 us an iteration).
   const bool product = op->prod.built && op->layout[0] != SQD_LAYOUT_CSR;
-  if (!product && (n < kPairMinRows || op->nnz < kPairMinPerRow * n)) return 0;
+  if (!product && (n < kPairMinRows[nc - 1] || op->nnz < kPairMinPairs ||
+                   op->nnz < kPairMinPerRow * n))
+    return 0;
   return static_cast<size_t>(n) * nc * 4 + (product && nc == 2 ? static_cast<size_t>(n) * 16 : 0);
 }
 
