@@ -2,10 +2,11 @@
 // ph_t = (-i)^{|x & z_t|}, for every merged term t.
 //
 //  * Product subspaces (ProductPlan): a block or warp owns a group, so its terms' sums stay in
-//    registers and are stored once.  Long groups (a few masks on many states, as in lattice
-//    models) have several owners, each adding its sums once.  An H group x joins the pairs (h, h') of high strings with
-//    every low string, an L group the other way round, a two-half group the pairs of its high part
-//    with the pairs of its low part; the pairs per group come from the halves' lists sorted by key.
+//    registers and are stored once.  Long groups (a few masks on many states, as in lattice models)
+//    have several owners, each adding its sums once.  An H group x joins the pairs (h, h') of high
+//    strings with every low string, an L group the other way round, a two-half group the pairs of
+//    its high part with the pairs of its low part; the pairs per group come from the halves' lists
+//    sorted by key.
 //  * Other subspaces: a lane per stored pair and one atomic addition per term.
 //  * The diagonal group: blocks of 1,024 rows by up to 64 terms, a warp per term.
 // Bound by the terms' popcounts and adds.  32 qubits, 256 x 240 strings, complex128: H 0.14, L 0.17,

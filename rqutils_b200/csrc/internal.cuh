@@ -127,7 +127,7 @@ struct ProductLayout {
 //   B: distinct low parts of the two-half masks,  key = index b, partner l'.
 // A two-half group connects (h, l) for every (a in A(h), b in B(l)) whose group exists.  The
 // lists take a few hundred entries per string, so an operator without cached sources keeps
-// them too.
+// them too, unless they are long or its matvec has no use for them (op_plan_pays).
 struct ProductPlan {
   int64_t nh = 0, nl = 0;
   int d = 0;                          // the diagonal group exists
@@ -175,7 +175,6 @@ struct sqd_op_s {
   int product_built = 0;          // connectivity assembled from the two halves' lists
   std::unique_ptr<ProductPlan> plan;  // product subspaces: the halves' lists
   uint64_t values_version = 0;    // p->version of elements whose computation has been waited for
-  sqd::DevBuf<int> status;        // device status word
   int layout[2] = {0, 0};         // SQD_LAYOUT_* per precision
   ProductLayout prod;
   // Bumped whenever the kernels or buffers a matvec launches may change (lanes, chunk,

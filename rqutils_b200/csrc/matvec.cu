@@ -114,7 +114,8 @@ k_mv_xc(const int64_t* __restrict__ row_ptr, const uint32_t* __restrict__ cols,
 // several streams are independent.
 // Bound by the L1 accesses of the two-half pairs' table entries, then by the terms' popcounts.
 // 32 qubits, complex128: 320 x 288 strings 0.42 ms (28.6 ms when every (row, group) was tested
-// against the subspace), 509 x 512 strings 1.44 ms (5.24 ms with stored sources and a lane per pair).
+// against the subspace), 509 x 512 strings 1.44 ms (3.45 ms with stored sources and a lane per pair);
+// L1TEX 88-90 % busy in the SMs that work.
 constexpr int kTileStrings = 32;
 
 template <typename R, int NCV, int NCA>

@@ -234,8 +234,6 @@ void op_build(sqd_op_s* op, cudaStream_t st) {
   copy_to_host(&x0, p->group_x.ptr, 1, st);
   op->has_diag_group = (x0 == 0) ? 1 : 0;
   op->value_complex = p->is_complex;
-  op->status.alloc(1, st);
-  SQD_CUDA(cudaMemsetAsync(op->status.ptr, 0, sizeof(int), st));
 
   // Groups that can connect.
   {
@@ -315,7 +313,7 @@ void op_connect_sweep(sqd_op_s* op, cudaStream_t st) {
   const unsigned blocks = static_cast<unsigned>(tiles * chunks);
 
   DevBuf<int64_t> place;
-  place.alloc(nu * chunks + 1, st);   // real rows only: most of `size` may be repeats of a few states
+  place.alloc(nu * chunks + 1, st);   // real rows only: `size` may be mostly fill-in slots
   P.counts = place.ptr;
   DevBuf<unsigned long long> n_hits;
   n_hits.alloc(1, st);

@@ -2,7 +2,8 @@
 //
 // SQD subspaces are usually the Cartesian product of strings on the high half of the qubits
 // (beta) and strings on the low half (alpha).  Sorted, row r = h * nl + l holds H[h] | L[l].
-// The stored pairs of a row come in three classes (k_gpre_flags, operator.cu; lists of the halves' partners: connect.cu):
+// The stored pairs of a row come in three classes (k_gpre_flags, operator.cu;
+// lists of the halves' partners: connect.cu):
 //   H: x on the high half only, source (h', l) with H[h'] = H[h] ^ x.  Every row of slab h has
 //      the same H sources in the same order;
 //   L: the diagonal group and x on the low half only, source (h, l') with L[l'] = L[l] ^ x.
@@ -832,8 +833,12 @@ void fill_panels(sqd_op_s* op, bool f64, bool f32, cudaStream_t st) {
 }
 
 // Panel form of the M pairs.  It applies when most of A(h) x B(l) exists (the panels hold every
-// combination; up to 1.6 elements per stored pair, where the stream still costs less than
-// sources and scattered gathers) and 16 bits reach a row of v.
+// combination; up to 1.6 elements per stored pair) and 16 bits reach a row of v.  Matvec in us,
+// panels / pair-list tails, complex128 and complex64, by elements per pair: 32 qubits, 512 x 512
+// strings with a share of the two-half groups left out, 1.0 223/327 144/255, 1.5 213/290 137/229,
+// 2.1 211/249 136/177, 2.6 212/233 137/169; 300 x 300 1.6 62/81 50/83; 48 qubits, 2000 x 1800, 1.3
+// 516/575 355/375, 2.6 515/559 355/369.  Sums whose parts hardly ever meet (random Paulis): 5.8 64/27
+// 59/25, 10 492/95 412/85, 25 183/45 156/35.  The limit stays on the safe side of the two.
 void build_panels(sqd_op_s* op, cudaStream_t st) {
   ProductLayout& L = op->prod;
   const ProductPlan& q = *op->plan;

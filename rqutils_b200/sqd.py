@@ -230,7 +230,8 @@ class SQDOperator:
         return getattr(self, '_chunk', [0, 0])[precision]
 
     def set_lanes(self, precision, lanes):
-        """precision 0: FP64 vectors (float64/complex128), 1: FP32 vectors."""
+        """precision 0: FP64 vectors (float64/complex128), 1: FP32 vectors.  No effect on pairs
+        that are not on a pair list: panels, and elements composed from partner lists."""
         _lib.call('sqd_op_set_lanes', self._handle, int(precision), int(lanes))
 
     LAYOUTS = {'csr': 0, 'product': 1, 'product-csr': 2}
@@ -238,8 +239,9 @@ class SQDOperator:
     def set_layout(self, precision, layout):
         """Element layout of the cached matvec for one precision: 'csr' (one pair list per
         row), 'product' (dense slabs for the pairs that change one half of the qubits; the
-        other pairs gather from shared memory when their source slabs fit there) or
-        'product-csr' (the same slabs, the other pairs always on CSR lists).  The product
+        other pairs in panels whose source rows are staged in shared memory, when most
+        combinations of the halves' partners exist) or 'product-csr' (the same slabs, the other
+        pairs always on CSR lists).  The product
         layouts need a product subspace and are built on first use."""
         _lib.call('sqd_op_set_layout', self._handle, int(precision), self.LAYOUTS[layout],
                   _lib.stream_ptr())
